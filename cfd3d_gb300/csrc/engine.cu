@@ -6,7 +6,7 @@
 //
 //   k_timestep            local time step + global minimum   (timestep_module.f90:127-212)
 //   k_ghost x3            boundary program: faces+halos, edges, corners (bc_module.f90:1235-1396)
-//   k_face_flux x3        inviscid + viscous face fluxes per direction (rhs_module.f90:282-538)
+//   face kernels          inviscid + viscous face fluxes (flux.cu, flux_mixed.cu; rhs_module.f90:282-538)
 //   k_rhs                 flux differences + cavitation / SST / dual-time sources (:540-642)
 //   k_sweep (fwd) x S     forward LU-SGS sweep, one launch per hyperplane i+j+k = s
 //   k_sweep (bwd) x S     backward sweep                          (update_module.f90:486-670)
@@ -53,6 +53,10 @@ __device__ __forceinline__ void store_cell(const DevPtr& d, const Par& c, long l
 }
 
 // ------------------------------------------------------------------ pointwise EOS
+// TERMS: the Gibbs sums term by term (deteos_t, the adjoint's), for the free-stream constants:
+// the mixed form's stored flux deviations are taken from them, so they keep the bits that
+// checkpoints and earlier runs had
+template <bool TERMS>
 __global__ void k_eos_points(int fluid, int with_prop, long long n, const double* __restrict__ p,
                              const double* __restrict__ t, const double* __restrict__ y1,
                              const double* __restrict__ y2, double* __restrict__ dv, double* __restrict__ tv,
@@ -60,7 +64,8 @@ __global__ void k_eos_points(int fluid, int with_prop, long long n, const double
   long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n) return;
   double d[NDV], tt[2] = {0.0, 0.0};
-  deteos(fluid, with_prop, p[q], t[q], y1[q], y2[q], d, tt, fb);
+  if constexpr (TERMS) deteos_t<double>(fluid, with_prop, p[q], t[q], y1[q], y2[q], d, tt);
+  else deteos(fluid, with_prop, p[q], t[q], y1[q], y2[q], d, tt, fb);
   for (int v = 0; v < NDV; ++v) dv[NDV * q + v] = d[v];
   if (tv) { tv[2 * q] = tt[0]; tv[2 * q + 1] = tt[1]; }
 }
@@ -90,7 +95,7 @@ __global__ void k_take_pv(const double* __restrict__ a, BlockGeom B, DevPtr d, P
   if (i < 2 || j < 2 || k < 2 || i > B.imax || j > B.jmax || k > B.kmax) return;
   double dv[NDV], tv[3] = {0.0, 0.0, 0.0};
   if (MX) deteos_split(c.fluid, c.with_prop, pv[0] + c.pref, pv[4], pv[5], pv[6], dv, tv, &d.sc->snd2_fallbacks);
-  else deteos<false>(c.fluid, c.with_prop, pv[0] + c.pref, pv[4], pv[5], pv[6], dv, tv, &d.sc->snd2_fallbacks);
+  else deteos(c.fluid, c.with_prop, pv[0] + c.pref, pv[4], pv[5], pv[6], dv, tv, &d.sc->snd2_fallbacks);
   for (int v = 0; v < NDV; ++v) d.dv[v * n + g] = dv[v];
   for (int v = 0; v < c.ntv && v < 2; ++v) d.tv[v * n + g] = tv[v];
 }
@@ -108,7 +113,7 @@ __global__ void k_init(DevPtr d, Par c, int b, int fresh) {
   double pv[NPVM], dv[NDV], tv[3] = {0.0, 0.0, 0.0};
   for (int v = 0; v < c.npv; ++v) pv[v] = d.pv[v * n + g];
   if (MX) deteos_split(c.fluid, c.with_prop, pv[0] + c.pref, pv[4], pv[5], pv[6], dv, tv, &d.sc->snd2_fallbacks);
-  else deteos<false>(c.fluid, c.with_prop, pv[0] + c.pref, pv[4], pv[5], pv[6], dv, tv, &d.sc->snd2_fallbacks);
+  else deteos(c.fluid, c.with_prop, pv[0] + c.pref, pv[4], pv[5], pv[6], dv, tv, &d.sc->snd2_fallbacks);
   for (int v = 0; v < NDV; ++v) d.dv[v * n + g] = dv[v];
   if (!fresh) {
     for (int v = 0; v < c.ntv && v < 2; ++v) d.tv[v * n + g] = tv[v];
@@ -244,7 +249,7 @@ __global__ void k_timestep(DevPtr d, Par c) {
 struct TpProblem { double pt, tt, ht, y1, y2, uu, gam; int fluid; };
 __device__ void tp_funcv(const TpProblem& P, const double* x, double* f) {
   double dv[NDV];
-  deteos_simple<false>(P.fluid, x[0], x[1], P.y1, P.y2, dv, nullptr);
+  deteos_simple(P.fluid, x[0], x[1], P.y1, P.y2, dv, nullptr);
   f[0] = P.pt - x[0] * pow(P.tt / x[1], P.gam / (P.gam - 1.0));
   f[1] = P.ht - (dv[1] + 0.5 * P.uu);
 }
@@ -1642,7 +1647,7 @@ __global__ void __launch_bounds__(128, 3) k_update(DevPtr d, Par c, int stage) {
     for (int v = 0; v < 3; ++v)
       if (v < c.ntv) tv[v] = d.tv[v * n + g];
     if (MX) deteos_split(c.fluid, c.with_prop, pe, te, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
-    else deteos<false>(c.fluid, c.with_prop, pe, te, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
+    else deteos(c.fluid, c.with_prop, pe, te, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
     for (int v = 0; v < NDV; ++v) {
       d.dv[v * n + g] = dv[v];
       if (!finite_bits(dv[v])) bad = 1;
@@ -1945,12 +1950,12 @@ void launch_face_rhs(const Engine& E, cudaStream_t s, bool rec, bool store_res) 
   cudaStreamWaitEvent(s, E.pipe_ev[Engine::MAX_PIPE + 1], 0);
 }
 
-// launches of the face fluxes and the residual: the FP64 form's three face kernels, or the
+// launches of the face fluxes and the residual: the FP64 form's face kernels, or the
 // mixed form's shadow, its reconstruction and flux kernels of each direction (with the j and
 // k faces' column reconstruction under MUSCL), and k_rhs
 int face_rhs_launches(const Engine& E) {
   const Par& c = E.par;
-  if (!c.mixed) return 4;
+  if (!c.mixed) return face_flux_launches(E) + 1;
   const int nb = (int)E.blk.size();
   const int ng = std::min(std::max(E.pipe_groups, 1), std::min(nb, Engine::MAX_PIPE));
   return ng * (8 + (c.nmuscl > 0 ? 2 : 0) + (c.iturb != -3 ? 3 : 0));
@@ -2206,12 +2211,10 @@ float time_calls(Engine& E, int reps, F fn) {
 }
 }  // namespace
 
-extern "C" {
-
-const char* cfd3d_last_error(const cfd3d_handle* h) { return h ? h->E.err.c_str() : "null handle"; }
-
-int cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
-                   const double* y2, double* dv, double* tv) {
+namespace {
+template <bool TERMS>
+int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
+               const double* y2, double* dv, double* tv) {
   if (n <= 0 || !p || !t || !y1 || !y2 || !dv || (fluid != 1 && fluid != 2) || ngas != 1) return CFD3D_ERR_ARG;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return CFD3D_ERR_NODEVICE;
@@ -2228,12 +2231,22 @@ int cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double* 
     cudaMemcpy(dy1, y1, b, cudaMemcpyHostToDevice);
     cudaMemcpy(dy2, y2, b, cudaMemcpyHostToDevice);
     cudaMemset(fb, 0, 8);
-    k_eos_points<<<(unsigned)((n + 127) / 128), 128>>>(fluid, with_prop, n, dp, dt, dy1, dy2, ddv, dtv, fb);
+    k_eos_points<TERMS><<<(unsigned)((n + 127) / 128), 128>>>(fluid, with_prop, n, dp, dt, dy1, dy2, ddv, dtv, fb);
     if (cudaMemcpy(dv, ddv, b * NDV, cudaMemcpyDeviceToHost) != cudaSuccess) rc = CFD3D_ERR_CUDA;
     if (tv && with_prop && cudaMemcpy(tv, dtv, b * 2, cudaMemcpyDeviceToHost) != cudaSuccess) rc = CFD3D_ERR_CUDA;
   }
   cudaFree(dp); cudaFree(dt); cudaFree(dy1); cudaFree(dy2); cudaFree(ddv); cudaFree(dtv); cudaFree(fb);
   return rc;
+}
+}  // namespace
+
+extern "C" {
+
+const char* cfd3d_last_error(const cfd3d_handle* h) { return h ? h->E.err.c_str() : "null handle"; }
+
+int cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
+                   const double* y2, double* dv, double* tv) {
+  return eos_points<false>(fluid, ngas, with_prop, n, p, t, y1, y2, dv, tv);
 }
 
 // ---- pointwise EOS through a static device buffer (no allocation)
@@ -2307,7 +2320,7 @@ int cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const 
       cudaMemcpy(S->y2, y2, b, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(&S->fallbacks, 0, sizeof(unsigned long long)) != cudaSuccess)
     return CFD3D_ERR_CUDA;
-  k_eos_points<<<(unsigned)((n + 127) / 128), 128>>>(fluid, with_prop, n, S->p, S->t, S->y1, S->y2, S->dv, S->tv,
+  k_eos_points<false><<<(unsigned)((n + 127) / 128), 128>>>(fluid, with_prop, n, S->p, S->t, S->y1, S->y2, S->dv, S->tv,
                                                       &S->fallbacks);
   if (cudaGetLastError() != cudaSuccess) return CFD3D_ERR_CUDA;
   if (cudaMemcpy(dv, S->dv, b * NDV, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
@@ -2343,7 +2356,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { E.err = "no CUDA device"; return CFD3D_ERR_NODEVICE; }
   // block layout
-  long long off = 0, ioff = 0, foff[3] = {0, 0, 0}, coff[3] = {0, 0, 0};
+  long long off = 0, ioff = 0, foff[3] = {0, 0, 0}, coff[3] = {0, 0, 0}, poff[3] = {0, 0, 0};
   for (int b = 0; b < nblocks; ++b) {
     const cfd3d_block_desc& d = blocks[b];
     if (d.imax < 4 || d.jmax < 4 || d.kmax < 4 || !d.xyz) { E.err = "block too small or no coordinates"; return CFD3D_ERR_DESCRIPTOR; }
@@ -2351,7 +2364,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
     G.imax = d.imax; G.jmax = d.jmax; G.kmax = d.kmax;
     G.ni = d.imax + 5; G.nj = d.jmax + 5; G.nk = d.kmax + 5;
     G.off = off; G.int_off = ioff;
-    for (int q = 0; q < 3; ++q) { G.face_off[q] = foff[q]; G.col_off[q] = coff[q]; }
+    for (int q = 0; q < 3; ++q) { G.face_off[q] = foff[q]; G.col_off[q] = coff[q]; G.plane_off[q] = poff[q]; }
     coff[1] += (long long)(d.imax - 1) * (d.kmax - 1);
     coff[2] += (long long)(d.imax - 1) * (d.jmax - 1);
     off += (long long)G.ni * G.nj * G.nk;
@@ -2359,11 +2372,14 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
     foff[0] += (long long)d.imax * (d.jmax - 1) * (d.kmax - 1);
     foff[1] += (long long)(d.imax - 1) * d.jmax * (d.kmax - 1);
     foff[2] += (long long)(d.imax - 1) * (d.jmax - 1) * d.kmax;
+    poff[0] += (long long)(d.imax + 3) * (d.jmax - 1) * (d.kmax - 1);
+    poff[1] += (long long)(d.imax - 1) * (d.jmax + 3) * (d.kmax - 1);
+    poff[2] += (long long)(d.imax - 1) * (d.jmax - 1) * (d.kmax + 3);
     E.blk.push_back(G);
   }
   if (off >= (1ll << 31)) { E.err = "case too large for 32-bit cell indices"; return CFD3D_ERR_ARG; }
   E.ncell = off; E.nint = ioff;
-  for (int q = 0; q < 3; ++q) { E.nface[q] = foff[q]; E.ncol[q] = coff[q]; }
+  for (int q = 0; q < 3; ++q) { E.nface[q] = foff[q]; E.ncol[q] = coff[q]; E.nplane[q] = poff[q]; }
   CFD_CUDA(cudaStreamCreateWithFlags(&E.st, cudaStreamNonBlocking));
   CFD_CUDA(cudaStreamCreateWithFlags(&E.st2, cudaStreamNonBlocking));
   for (auto& e : E.pipe_ev) CFD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -2388,8 +2404,14 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   if (c.mixed)
     ok = ok && allocf(E.d.pvf, c.npv) && allocf(E.d.fi32, 3 * c.npv) && allocf(E.d.fv32, (c.iturb == -3) ? 1 : 3 * c.npv) &&
          allocf(E.d.frec, 2 * 12) && allocf(E.d.lqf, NLQ);
-  else
-    ok = ok && alloc(E.d.fi, 3 * c.npv) && alloc(E.d.fv, (c.iturb == -3) ? 1 : 3 * c.npv);
+  else {
+    // the face reconstruction's scratch: all three directions at once up to 256 MB of it (larger
+    // cases fill the GPU one direction at a time)
+    E.d.nfs = (c.nmuscl == 2) ? 5 : (c.nmuscl > 0 ? 1 : 0);
+    E.d.fslots = (3.0 * E.d.nfs * c.npv * 8.0 * (double)n <= 2.56e8) ? 3 : 1;
+    ok = ok && alloc(E.d.fi, 3 * c.npv) && alloc(E.d.fv, (c.iturb == -3) ? 1 : 3 * c.npv) &&
+         alloc(E.d.fsc, (long long)E.d.fslots * E.d.nfs * c.npv);
+  }
   if (c.csf) ok = ok && alloc(E.d.vf, 1) && alloc(E.d.vfg, 3) && alloc(E.d.csf, 3);
   if (!ok) { E.err = "device allocation failed"; return CFD3D_ERR_NOMEM; }
   E.d.ncell = n;
@@ -2440,7 +2462,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   {
     double hp[4] = {cfg->pref, cfg->tref, cfg->y1ref, cfg->y2ref};
     double dvr[NDV], tvr[2] = {0.0, 0.0};
-    int rc = cfd3d_eos_eval(cfg->fluid, cfg->ngas, c.with_prop, 1, &hp[0], &hp[1], &hp[2], &hp[3], dvr, tvr);
+    int rc = eos_points<true>(cfg->fluid, cfg->ngas, c.with_prop, 1, &hp[0], &hp[1], &hp[2], &hp[3], dvr, tvr);
     if (rc != CFD3D_OK) { E.err = "reference-state EOS failed"; return rc; }
     E.par.rhoref = dvr[0];
     if (c.iturb == 0) {
@@ -2464,7 +2486,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
       E.par.tp_tt = 300.0003719;
       double hp2[4] = {E.par.tp_pt, E.par.tp_tt, cfg->y1ref, cfg->y2ref};
       double dvt[NDV], tvt[2] = {0.0, 0.0};
-      rc = cfd3d_eos_eval(cfg->fluid, cfg->ngas, c.with_prop, 1, &hp2[0], &hp2[1], &hp2[2], &hp2[3], dvt, tvt);
+      rc = eos_points<true>(cfg->fluid, cfg->ngas, c.with_prop, 1, &hp2[0], &hp2[1], &hp2[2], &hp2[3], dvt, tvt);
       if (rc != CFD3D_OK) { E.err = "total-pressure EOS failed"; return rc; }
       E.par.tp_ht = dvt[1];
     }
@@ -2542,7 +2564,7 @@ void cfd3d_destroy(cfd3d_handle* h) {
   Engine& E = h->E;
   if (E.graph) cudaGraphExecDestroy(E.graph);
   double* bufs[] = {E.d.pv, E.d.dv, E.d.tv, E.d.gm, E.d.res, E.d.icav, E.d.itt, E.d.ocut, E.d.dt, E.d.rcav,
-                    E.d.qq, E.d.dqs, E.d.dcv, E.d.fi, E.d.fv, E.d.partial, h->staging, E.d.clo,
+                    E.d.qq, E.d.dqs, E.d.dcv, E.d.fi, E.d.fv, E.d.fsc, E.d.partial, h->staging, E.d.clo,
                     E.d.vf, E.d.vfg, E.d.csf};
   for (double* p : bufs) cudaFree(p);
   float* fbufs[] = {E.d.pvf, E.d.fi32, E.d.fv32, E.d.frec, E.d.gmf, E.d.gmlo, E.d.lqf};

@@ -25,6 +25,7 @@ struct BlockGeom {
   long long int_off;        // first interior cell in the flat interior numbering
   long long face_off[3];    // first face of each direction in the flat face numbering
   long long col_off[3];     // first column of cells along direction 1 (i, k) / 2 (i, j)
+  long long plane_off[3];   // first cell of each direction's reconstruction planes (flux.cu)
 };
 
 // gm planes: face vectors and cell geometry
@@ -128,6 +129,10 @@ __host__ __device__ __forceinline__ long long tq_at(long long s, int v) {
 
 struct DevPtr {
   double *pv, *dv, *tv, *gm, *res, *icav, *itt, *ocut, *dt, *rcav, *qq, *dqs, *dcv, *qold, *fi, *fv;
+  // FP64 form: scratch planes of the face reconstruction (flux.cu), nfs per variable and
+  // direction slot; fslots directions at a time (3: all in one launch)
+  double* fsc;
+  int nfs, fslots;
   const BlockGeom* blk;
   int nblk;
   long long ncell;
@@ -206,7 +211,7 @@ struct Engine {
   cfd3d_config cfg;
   Par par;
   std::vector<BlockGeom> blk;
-  long long ncell = 0, nint = 0, nface[3] = {0, 0, 0}, ncol[3] = {0, 0, 0};
+  long long ncell = 0, nint = 0, nface[3] = {0, 0, 0}, ncol[3] = {0, 0, 0}, nplane[3] = {0, 0, 0};
   DevPtr d{};
   // ghost program: phase 0 faces + halos, 1 edges, 2 corners
   GhostOp* d_ops[3] = {nullptr, nullptr, nullptr};
@@ -341,6 +346,7 @@ constexpr int SW_CH = 32;
 
 // face-flux launchers (flux.cu: FP64 form; flux_mixed.cu: mixed form)
 void launch_face_flux(const Engine& E, cudaStream_t s);
+int face_flux_launches(const Engine& E);
 void launch_face_flux_mixed(const Engine& E, cudaStream_t s, int b0, int b1);
 // discrete adjoint (adjoint.cu): buffers (allocated once, zeroed per call), the reverse
 // pass, and release

@@ -17,6 +17,7 @@
 // The reference multiplies by four literals written without a kind suffix, i.e.
 // single-precision constants (src/eos_module.f90:1367,1370,1371,1457); they are kept.
 #pragma once
+#include <type_traits>
 #include <utility>
 
 namespace cfd {
@@ -265,7 +266,11 @@ __device__ __forceinline__ void stiffened(T p, T t, Phase<T>& e) {
 
 template <class T>
 __device__ __forceinline__ T ideal_vis(T t) {
-  return T(1.716e-5) * pow(t / T(273.11), T(1.5)) * T(383.67) / (t + T(110.56));
+  if constexpr (std::is_same<T, double>::value) {
+    const double r = t * (1.0 / 273.11);
+    return 1.716e-5 * (r * ::sqrt(r)) * 383.67 / (t + 110.56);
+  } else
+    return T(1.716e-5) * pow(t / T(273.11), T(1.5)) * T(383.67) / (t + T(110.56));
 }
 template <class T>
 __device__ __forceinline__ T stiffened_vis(T t) {

@@ -17,6 +17,7 @@
 #pragma once
 #include <type_traits>
 #include "iapws.cuh"
+#include "eos64.cuh"
 #include "df64.cuh"
 
 namespace cfd {
@@ -152,24 +153,6 @@ __device__ __forceinline__ df64 dadd(df64 a, df64 b) {
   return fast_two_sum(s.hi, __fadd_rn(__fadd_rn(s.lo, a.lo), b.lo));
 }
 
-template <const IJN* TAB, size_t N>
-struct IGroups {
-  static constexpr bool head(size_t k) { return k == 0 || TAB[k].i != TAB[k - 1].i; }
-  static constexpr int count() {
-    int c = 0;
-    for (size_t k = 0; k < N; ++k) c += head(k) ? 1 : 0;
-    return c;
-  }
-  static constexpr size_t start(int g) {
-    int c = -1;
-    for (size_t k = 0; k < N; ++k) {
-      if (head(k)) ++c;
-      if (c == g) return k;
-    }
-    return N;
-  }
-};
-
 // one term of a group: n I y^J into px, n J y^(J-1) into py (the first contribution of
 // each is assigned, later ones added; `hx`, `hy` say whether one was made)
 template <const IJN* TAB, size_t K>
@@ -250,47 +233,6 @@ __device__ __forceinline__ void if97_r2_rh(df64 P, df64 T, bool meta, df64& gp, 
   gt = dadd(iy, ry);
 }
 
-// IF97 liquid and vapour phases with the Gibbs sums in df64 on the FP32 pipes; one
-// out-of-line copy per FULL flag keeps the expanded sums out of every caller
-template <bool FULL>
-__device__ __noinline__ void iapws_pair_df64(double p, double t, bool meta, Phase<double>& l, Phase<double>& v) {
-  const df64 P(p), T(t);
-  if constexpr (FULL) {
-    Phase<df64> lx, vx;
-    iapws_l<df64, FULL>(P, T, lx);
-    iapws_v_meta<df64, FULL>(P, T, meta, vx);
-    l.rho = (double)lx.rho; l.h = (double)lx.h;
-    v.rho = (double)vx.rho; v.h = (double)vx.h;
-    l.drdp = (double)lx.drdp; l.drdt = (double)lx.drdt; l.dhdp = (double)lx.dhdp; l.dhdt = (double)lx.dhdt;
-    v.drdp = (double)vx.drdp; v.drdt = (double)vx.drdt; v.dhdp = (double)vx.dhdp; v.dhdt = (double)vx.dhdt;
-  } else {
-    // rho = c tau / gamma_pi, h = c' gamma_tau (the constants of iapws_l / iapws_v_meta)
-    df64 gp, gt, tau;
-    if97_r1_rh(P, T, gp, gt, tau);
-    l.rho = (double)(df64((double)25.841246054191803727f) * tau / gp);
-    l.h = (double)(df64(639675.036) * gt);
-    if97_r2_rh(P, T, meta, gp, gt, tau);
-    v.rho = (double)(df64(4.01245401527075799) * tau / gp);
-    v.h = (double)(df64(249224.04) * gt);
-  }
-}
-
-// the liquid phase alone (df64 sums): the face EOS of a face state without vapour
-template <bool FULL>
-__device__ __noinline__ void iapws_liq_df64(double p, double t, Phase<double>& l) {
-  if constexpr (FULL) {
-    Phase<df64> lx;
-    iapws_l<df64, FULL>(df64(p), df64(t), lx);
-    l.rho = (double)lx.rho; l.h = (double)lx.h;
-    l.drdp = (double)lx.drdp; l.drdt = (double)lx.drdt; l.dhdp = (double)lx.dhdp; l.dhdt = (double)lx.dhdt;
-  } else {
-    df64 gp, gt, tau;
-    if97_r1_rh(df64(p), df64(t), gp, gt, tau);
-    l.rho = (double)(df64((double)25.841246054191803727f) * tau / gp);
-    l.h = (double)(df64(639675.036) * gt);
-  }
-}
-
 // The mixed form's face-state EOS: 1/rho and h of the liquid (and of the vapour when VAP)
 // from the df64 sums, the reciprocal also taken in df64 (on the FP32 pipes: an FP64
 // division costs a GB300 far more), and the gas's 1/rho = t / (p r1) from the same df64
@@ -312,44 +254,48 @@ __device__ __noinline__ void iapws_inv_df64(double p, double t, bool meta, doubl
   }
 }
 
-// Phase properties of liquid and vapour.  MX evaluates the IF97 Gibbs sums in df64 (the
-// mixed form); FULL = false evaluates only rho and h.  The metastable branch test
-// p > p_sat(T) is taken in FP64 in both forms so that they select the same term set.
+// Phase properties of liquid, vapour and gas in FP64, with their reciprocal densities ir[3].
+// FULL = false evaluates only ir and h.  The metastable branch test p > p_sat(T) is taken as
+// the FP64 comparison in both forms so that they select the same term set.
 // vap = false (a state without vapour, y1 = 0, whose caller needs only the mixture's rho,
 // h or c2): every vapour term of the mixture carries the factor y1 = 0, so the vapour sums
 // (the larger half of the work) are skipped and a neutral vapour phase returned; the
 // mixture's rho, h and c2 come out the same.
-template <bool MX, bool FULL>
+template <bool FULL>
 __device__ __forceinline__ void phases(int fluid, double p, double t, Phase<double>& l, Phase<double>& v,
-                                       bool vap = true) {
+                                       Phase<double>& g, double* ir, bool vap = true) {
   if (fluid == 1) {
     stiffened(p, t, l);
     ideal_gas(p, t, v);
+    ideal_gas(p, t, g);
+    ir[0] = 1.0 / l.rho; ir[1] = 1.0 / v.rho; ir[2] = ir[1];
     return;
   }
+  const double it = 1.0 / t, pi1 = 1.0e6 / p;
+  if97_liquid<FULL>(p, t, it, l, ir[0]);
+  // the gas: rho = p r1 / t
+  const double r1 = 0.00348383500557;
+  ir[2] = t * pi1 * (1.0e-6 / r1);
+  g.h = 1004.64 * t;
+  g.rho = p * r1 * it;
+  g.drdp = r1 * it;
+  g.drdt = -(g.rho * it);
+  g.dhdp = 0.0;
+  g.dhdt = 1004.64;
   if (!vap) {
-    if constexpr (MX) iapws_liq_df64<FULL>(p, t, l);
-    else iapws_l<double, FULL>(p, t, l);
     v.rho = 1.0; v.h = 0.0; v.drdp = 0.0; v.drdt = 0.0; v.dhdp = 0.0; v.dhdt = 1.0;
+    ir[1] = 1.0;
     return;
   }
-  const bool meta = above_psat(p, t);
-  if constexpr (MX) {
-    iapws_pair_df64<FULL>(p, t, meta, l, v);
-  } else {
-    iapws_l<double, FULL>(p, t, l);
-    iapws_v_meta<double, FULL>(p, t, meta, v);
-  }
+  if97_vapour<FULL>(p, t, pi1, it, above_psat(p, t), v, ir[1]);
 }
 
 template <class T>
 __device__ __forceinline__ void mixture(const Phase<T>& l, const Phase<T>& v, const Phase<T>& g, T y1, T y2, T* dv,
-                                        unsigned long long* fallbacks, T* irh = nullptr) {
-  // irh (optional): the phase reciprocals 1/rho_l, 1/rho_v, 1/rho_g, which the transport
-  // properties reuse (three FP64 divisions fewer)
+                                        unsigned long long* fallbacks, const T* ir) {
+  // ir: the phase reciprocals 1/rho_l, 1/rho_v, 1/rho_g
   dv[2] = l.rho; dv[3] = v.rho; dv[4] = g.rho;
-  T irhol = 1.0 / dv[2], irhov = 1.0 / dv[3], irhog = 1.0 / dv[4];
-  if (irh) { irh[0] = irhol; irh[1] = irhov; irh[2] = irhog; }
+  const T irhol = ir[0], irhov = ir[1], irhog = ir[2];
   T yl = 1.0 - y1 - y2;
   T irho = yl * irhol + y1 * irhov + y2 * irhog;
   dv[0] = 1.0 / irho;
@@ -436,7 +382,7 @@ __device__ __forceinline__ void deteos_t(int fluid, int with_prop, T p, T t, T y
   Phase<T> l, v, g;
   phases_t<T>(fluid, p, t, l, v);
   ideal_gas<T>(p, t, g);
-  T irh[3];
+  const T irh[3] = {1.0 / l.rho, 1.0 / v.rho, 1.0 / g.rho};
   mixture<T>(l, v, g, y1, y2, dv, nullptr, irh);
   if (with_prop) {
     T lv, lc, vv, vc;
@@ -457,13 +403,12 @@ __device__ __forceinline__ void deteos_t(int fluid, int with_prop, T p, T t, T y
 
 // eos%deteos_simple
 // (vap = false: the caller reads only dv(1), dv(2), dv(6) of a state with y1 = 0; see phases)
-template <bool MX = false>
 __device__ __forceinline__ void deteos_simple(int fluid, double p, double t, double y1, double y2, double* dv,
                                               unsigned long long* fb, bool vap = true) {
   Phase<double> l, v, g;
-  phases<MX, true>(fluid, p, t, l, v, vap);
-  ideal_gas(p, t, g);
-  mixture(l, v, g, y1, y2, dv, fb);
+  double ir[3];
+  phases<true>(fluid, p, t, l, v, g, ir, vap);
+  mixture<double>(l, v, g, y1, y2, dv, fb, ir);
 }
 
 // mixture density and static enthalpy only: all that the Roe and AUSM+-up fluxes read of
@@ -490,24 +435,20 @@ __device__ __forceinline__ void eos_rho_h(int fluid, double p, double t, double 
     }
   }
   Phase<double> l, v, g;
-  phases<MX, false>(fluid, p, t, l, v, y1 != 0.0);
-  ideal_gas(p, t, g);
-  double irhol = 1.0 / l.rho, irhov = 1.0 / v.rho, irhog = 1.0 / g.rho;
+  double ir[3];
+  phases<false>(fluid, p, t, l, v, g, ir, y1 != 0.0);
   double yl = 1.0 - y1 - y2;
-  double irho = yl * irhol + y1 * irhov + y2 * irhog;
-  rho = 1.0 / irho;
+  rho = 1.0 / (yl * ir[0] + y1 * ir[1] + y2 * ir[2]);
   h = yl * l.h + y1 * v.h + y2 * g.h;
 }
 
 // eos%deteos: with transport properties when with_prop (tv(1:2) written), else simple
-template <bool MX = false>
 __device__ __forceinline__ void deteos(int fluid, int with_prop, double p, double t, double y1, double y2,
                                        double* dv, double* tv, unsigned long long* fb) {
   Phase<double> l, v, g;
-  phases<MX, true>(fluid, p, t, l, v);
-  ideal_gas(p, t, g);
   double irh[3];
-  mixture(l, v, g, y1, y2, dv, fb, irh);
+  phases<true>(fluid, p, t, l, v, g, irh);
+  mixture<double>(l, v, g, y1, y2, dv, fb, irh);
   if (with_prop) {
     double lv, lc, vv, vc;
     if (fluid == 1) {
@@ -793,13 +734,17 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
     for (int k = 0; k < npv; ++k) fx[k] = T(0.0);
     return;
   }
-  double nx = n[0] / dl, ny = n[1] / dl, nz = n[2] / dl;
+  // (quotients by a common divisor go through its reciprocal: an FP64 division takes about
+  // nine slots of the FP64 pipe, a product one)
+  const double idl = 1.0 / dl;
+  double nx = n[0] * idl, ny = n[1] * idl, nz = n[2] * idl;
   const T* pl = L.pv;
   const T* pr = Rs.pv;
-  T rrho = sqrt(L.rho * Rs.rho);
   const double pref = c.pref;
   const T srl = sqrt(L.rho), srr = sqrt(Rs.rho);
+  const T rrho = srl * srr;
   const T ravg_d = 1.0 / (srl + srr);
+  const T irc2 = 1.0 / rc2;
   const T hl = L.h + 0.5 * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]);
   const T hr = Rs.h + 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]);
   const T uull = nx * pl[1] + ny * pl[2] + nz * pl[3];
@@ -810,12 +755,12 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
     T uuu = nx * ravg[1] + ny * ravg[2] + nz * ravg[3];
     if (c.nscheme == 1) {
       T sndp2 = sndp2_u<T>(c, rc2, u2, uref2);
-      T q = sndp2 / rc2;
+      T q = sndp2 * irc2;
       T uup = 0.5 * (1.0 + q) * uuu;
       T ddd = 0.5 * sqrt((1.0 - q) * (1.0 - q) * uuu * uuu + 4.0 * sndp2);
       T c_star = 0.5 * (fabs(uup + ddd) + fabs(uup - ddd));
       T m_star = 0.5 * (fabs(uup + ddd) - fabs(uup - ddd)) / ddd;
-      T du = m_star * (uurr - uull) + (c_star - q * fabs(uuu) - 0.5 * (1.0 - q) * uuu * m_star) * (pr[0] - pl[0]) / rrho / sndp2;
+      T du = m_star * (uurr - uull) + (c_star - q * fabs(uuu) - 0.5 * (1.0 - q) * uuu * m_star) * (pr[0] - pl[0]) / (rrho * sndp2);
       T dp = m_star * (pr[0] - pl[0]) + (c_star - fabs(uuu) + 0.5 * (1.0 - q) * uuu * m_star) * rrho * (uurr - uull);
       T au = fabs(uuu);
       T df0 = au * (Rs.rho - L.rho) + du * rrho;
@@ -835,10 +780,10 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
       return;
     }
     // Roe-M
-    T am2rmid_du = sndp2_du_u<T>(c, rc2, u2, uref2) / rc2;
-    T am2rmid = sndp2_u<T>(c, rc2, u2, uref2) / rc2;
-    T fmid = sqrt(am2rmid) * (2.0 - sqrt(am2rmid));
-    T fmid_du = sqrt(am2rmid_du) * (2.0 - sqrt(am2rmid_du));
+    const T sq_du = sqrt(sndp2_du_u<T>(c, rc2, u2, uref2) * irc2);
+    const T sq_m = sqrt(sndp2_u<T>(c, rc2, u2, uref2) * irc2);
+    T fmid = sq_m * (2.0 - sq_m);
+    T fmid_du = sq_du * (2.0 - sq_du);
     T amid = sqrt(rc2);
     T b1 = fmax(fmax(0.0, uuu + amid), uurr + amid);
     T b2 = fmin(fmin(0.0, uuu - amid), uull - amid);
@@ -867,42 +812,44 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
     }
     fl[4] = L.rho * uull * hl; fr[4] = Rs.rho * uurr * hr;
     for (int k = 5; k < npv; ++k) { fl[k] = L.rho * uull * pl[k]; fr[k] = Rs.rho * uurr * pr[k]; }
-    bdq[0] = dq[0] - ff * (pr[0] - pl[0]) / rc2 / fmid;
+    bdq[0] = dq[0] - ff * (pr[0] - pl[0]) * irc2 / fmid;
     for (int k = 1; k <= 3; ++k) bdq[k] = bdq[0] * ravg[k] + rrho * (pr[k] - pl[k]);
     bdq[4] = bdq[0] * ravg_ht + rrho * (hr - hl);
     for (int k = 5; k < npv; ++k) bdq[k] = bdq[0] * ravg[k] + rrho * (pr[k] - pl[k]);
-    for (int k = 0; k < npv; ++k) fx[k] = (b1 * fl[k] - b2 * fr[k] + b1 * b2 * (dq[k] - gg * bdq[k] / add)) / (b1 - b2) * dl;
-    for (int q3 = 0; q3 < 3; ++q3)
-      fx[1 + q3] = fx[1 + q3] + gg * b1_du * b2_du * rrho * (uurr - uull) * nn[q3] / aaa / (b1_du - b2_du) * dl;
+    const T b12 = b1 * b2, fdl = dl / (b1 - b2), gadd = gg / add;
+    const T fdu = gg * b1_du * b2_du * rrho * (uurr - uull) * dl / (aaa * (b1_du - b2_du));
+    for (int k = 0; k < npv; ++k) fx[k] = (b1 * fl[k] - b2 * fr[k] + b12 * (dq[k] - gadd * bdq[k])) * fdl;
+    for (int q3 = 0; q3 < 3; ++q3) fx[1 + q3] = fx[1 + q3] + fdu * nn[q3];
     return;
   }
   // AUSM family
   T amid = sqrt(rc2);
-  T zmr = uurr / amid, zml = uull / amid;
+  const T iamid = amid * irc2;
+  T zmr = uurr * iamid, zml = uull * iamid;
   T fmid, fmid1, am2mid;
   if (c.nscheme == 3) {
     am2mid = ravg[1] * ravg[1] + ravg[2] * ravg[2] + ravg[3] * ravg[3];
-    T a1 = sndp2_du_u<T>(c, rc2, am2mid, uref2) / rc2;
-    T a0 = sndp2_u<T>(c, rc2, am2mid, uref2) / rc2;
-    fmid = sqrt(a0) * (2.0 - sqrt(a0));
-    fmid1 = sqrt(a1) * (2.0 - sqrt(a1));
+    const T s1 = sqrt(sndp2_du_u<T>(c, rc2, am2mid, uref2) * irc2);
+    const T s0 = sqrt(sndp2_u<T>(c, rc2, am2mid, uref2) * irc2);
+    fmid = s0 * (2.0 - s0);
+    fmid1 = s1 * (2.0 - s1);
   } else {
     T un = nx * ravg[1] + ny * ravg[2] + nz * ravg[3];
     am2mid = un * un;
-    T a0 = sndp2_u<T>(c, rc2, am2mid, uref2) / rc2;
-    fmid = sqrt(a0) * (2.0 - sqrt(a0));
+    const T s0 = sqrt(sndp2_u<T>(c, rc2, am2mid, uref2) * irc2);
+    fmid = s0 * (2.0 - s0);
     fmid1 = fmid;
   }
   T alpha = 3.0 / 16.0 * (-4.0 + 5.0 * fmid1 * fmid1);
   alpha = fmax(fmin(alpha, 3.0 / 16.0), -3.0 / 4.0);
   const double beta = 0.125;
   T zmmr, pmr, zmpl, ppl;
-  if (fabs(zmr) >= 1.0) { zmmr = 0.5 * (zmr - fabs(zmr)); pmr = 0.5 * (1.0 - zmr / fabs(zmr)); }
+  if (fabs(zmr) >= 1.0) { zmmr = 0.5 * (zmr - fabs(zmr)); pmr = 0.5 * (1.0 - copysign(1.0, zmr)); }
   else {
     zmmr = -(0.25 * (zmr - 1.0) * (zmr - 1.0)) - beta * sq(zmr * zmr - 1.0);
     pmr = 0.25 * (zmr - 1.0) * (zmr - 1.0) * (2.0 + zmr) - alpha * zmr * sq(zmr * zmr - 1.0);
   }
-  if (fabs(zml) >= 1.0) { zmpl = 0.5 * (zml + fabs(zml)); ppl = 0.5 * (1.0 + zml / fabs(zml)); }
+  if (fabs(zml) >= 1.0) { zmpl = 0.5 * (zml + fabs(zml)); ppl = 0.5 * (1.0 + copysign(1.0, zml)); }
   else {
     zmpl = 0.25 * (zml + 1.0) * (zml + 1.0) + beta * sq(zml * zml - 1.0);
     ppl = 0.25 * (zml + 1.0) * (zml + 1.0) * (2.0 - zml) + alpha * zml * sq(zml * zml - 1.0);
@@ -920,8 +867,9 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
     T ww2 = 1.0 - m2 * m2;
     T ww = fmax(ww1, ww2);
     T pmt = rrho * rc2;
-    T pwl = ((pl[0] + pref + rrho * rc2) / pmt - 1.0) * (1.0 - ww) / fmid;
-    T pwr = ((pr[0] + pref + rrho * rc2) / pmt - 1.0) * (1.0 - ww) / fmid;
+    const T ipmt = 1.0 / pmt, wf = (1.0 - ww) / fmid;
+    T pwl = ((pl[0] + pref + pmt) * ipmt - 1.0) * wf;
+    T pwr = ((pr[0] + pref + pmt) * ipmt - 1.0) * wf;
     if (zmid >= 0.0) {
       pwl = pwl * rrho / L.rho;
       pwr = pwr * rrho / L.rho;  // both weights scaled by the left density, as the reference does
@@ -935,7 +883,7 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
     }
   } else {
     const double kp = 0.25;
-    T zmid = zmpl + zmmr - kp * fmax(1.0 - am2mid / rc2, 0.0) * (pr[0] - pl[0]) / rrho / rc2 / fmid;
+    T zmid = zmpl + zmmr - kp * fmax(1.0 - am2mid * irc2, 0.0) * (pr[0] - pl[0]) * irc2 / (rrho * fmid);
     pmid = ppl * (pl[0] + pref) + pmr * (pr[0] + pref) - 2.0 * ppl * pmr * rrho * fmid * amid * (uurr - uull);
     if (zmid > 0.0) { zmpl1 = zmid; zmmr1 = 0.0; } else { zmmr1 = zmid; zmpl1 = 0.0; }
   }
@@ -948,24 +896,6 @@ __device__ inline void inviscid_flux_core(const Par& c, const double* n, const F
   for (int k = 5; k < npv; ++k) fx[k] = (ml * pl[k] + mr * pr[k]) * dl;
 }
 
-
-// FP64 face flux: the Roe-average EOS (only its sound speed is used,
-// src/flux_module.f90:237,319,461,588), then the flux
-template <bool MX = false>
-__device__ inline void inviscid_flux(const Par& c, const double* n, const FaceState& L, const FaceState& Rs,
-                                     const double* sdst_in, double* fx, unsigned long long* fb) {
-  const int npv = c.npv;
-  double dl = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-  if (dl == 0.0) {
-    for (int k = 0; k < npv; ++k) fx[k] = 0.0;
-    return;
-  }
-  double ravg[NPVM];
-  roe_state<double>(npv, L, Rs, ravg);
-  double rdv[NDV];
-  deteos_simple<MX>(c.fluid, ravg[0] + c.pref, ravg[4], ravg[5], ravg[6], rdv, fb, ravg[5] != 0.0);
-  inviscid_flux_core<double>(c, n, L, Rs, sdst_in, ravg, rdv[5], c.uref * c.uref, fx);
-}
 
 // ------------------------------------------------------------------ SST source
 // k-omega SST production, destruction and cross diffusion of one cell (kwsst + calbigf +
@@ -1063,7 +993,8 @@ __device__ __forceinline__ SstOut<T> sst_source(const T (*gr)[3], T kk, T oo, T 
     if constexpr (std::is_same<T, double>::value) tl = sst_length_d(ides, kk, oo, o.bigf, o.strain, vort, hmax, y5, mu, mut);
     else tl = sst_length<T>(ides, kk, oo, o.bigf, o.strain, vort, hmax, y5, mu, mut);
   }
-  o.dest = rho * pow(kk, 1.5) / tl;
+  if constexpr (std::is_same<T, double>::value) o.dest = rho * (kk * sqrt(kk)) / tl;
+  else o.dest = rho * pow(kk, 1.5) / tl;
   o.r7 = (o.prod - o.dest) * vol;
   o.r8 = (o.talpha * rho * (1.0 / mut) * o.prod - o.tbeta * rho * oo * oo + 1.712 * (1.0 - o.bigf) * rho * (1.0 / oo) * o.pkw) * vol;
   return o;
