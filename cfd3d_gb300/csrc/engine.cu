@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(256, MX ? 4 : 1) k_rhs(DevPtr d, Par c, long l
     for (int q = 0; q < NREC; ++q) o[q] = 0.0;
     for (int q = 0; q < 7; ++q) o[REC_PV + q] = (pvi[q] < npv) ? pv2[pvi[q]] : 0.0;
     for (int q = 0; q < 10; ++q) o[REC_DV + q] = dv[dvi[q]];
-    diag_to_array(D, o + REC_DIAG);
+    diag_solution(D, pv2, dv, o + REC_SOL);
     for (int q = 0; q < 6; ++q) o[REC_SPEC + q] = face_spectral<double>(c, fc + 3 * q, pv2, dv);
     // beta = 1/sndp2 - 1/c2 + drho/dp = D.rr - (D.b1 - 1) drho/dp
     o[REC_BETA] = D.rr - (D.b1 - 1.0) * dv[6];
@@ -1151,67 +1151,124 @@ __global__ void __launch_bounds__(256, MX ? 4 : 1) k_rhs(DevPtr d, Par c, long l
 
 // ------------------------------------------------------------------ LU-SGS sweeps
 // FP64 form: the sweeps work in the plane-major numbering t (setup_planes).  k_rhs writes
-// what they read of each cell -- as itself (diagonal block, residual) and as a neighbour
-// (state, split-Jacobian coefficients, + face vectors) -- as the cell's sweep record at t;
-// each hyperplane launch then reads its own records and those of the previous (next) plane
-// with coalesced loads.  dcv and dqs live at t as well; k_update reads dqs through pos[g].
-// The mixed form sweeps by tiles (k_sweep_tile, below).
+// what they read of each cell -- as itself (the coefficients of D^-1, the residual) and as a
+// neighbour (state, split-Jacobian coefficients, + face vectors) -- as the cell's sweep record
+// at t, so that loads of a plane and of its neighbours coalesce.  dcv and dqs live at t as
+// well; k_update reads dqs through pos[g].  The mixed form sweeps by tiles (k_sweep_tile,
+// below).
 
-// a cell's pv / dv as the Jacobian and diagonal routines index them, from its record
-template <class T>
-__device__ __forceinline__ void rec_state(const T* R, long long nint, long long t, T* pv, T* dv) {
-  pv[0] = T(0); pv[4] = T(0);
-  pv[1] = R[(REC_PV + 0) * nint + t]; pv[2] = R[(REC_PV + 1) * nint + t]; pv[3] = R[(REC_PV + 2) * nint + t];
-  pv[5] = R[(REC_PV + 3) * nint + t]; pv[6] = R[(REC_PV + 4) * nint + t];
-  pv[7] = R[(REC_PV + 5) * nint + t]; pv[8] = R[(REC_PV + 6) * nint + t];
-  dv[0] = R[(REC_DV + 0) * nint + t]; dv[1] = R[(REC_DV + 1) * nint + t];
-  dv[2] = dv[3] = dv[4] = dv[5] = T(0);
+// The coefficients of one neighbour's product s A dq (jac_apply_pre's algebra), everything in
+// it that does not depend on dq: the product is then 32 multiply-adds.
+struct NbCoef {
+  double a[7];    // row 1 over dq 0..6
+  double n[3];    // s times the face vector
+  double pv[7];   // pv 1, 2, 3, 5, 6, 7, 8
+  double c[7];    // the enthalpy row over dq 0..6
+  double h, ru;
+};
+
+// q: direction; the forward sweep takes the lower neighbour nb through its + face, the
+// backward sweep the upper one through the + face of t
+template <bool FWD>
+__device__ __forceinline__ void nb_coef(const double* R, long long nint, long long t, long long nb, int q, NbCoef& o) {
+  const long long fr = FWD ? nb : t;
+  const double sg = FWD ? 1.0 : -1.0, s = 0.5 * sg;
+  double nx[3], dv[10];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) dv[6 + q] = R[(REC_DV + 2 + q) * nint + t];
+  for (int e = 0; e < 3; ++e) nx[e] = R[(REC_FACE + 3 * q + e) * nint + fr];
+#pragma unroll
+  for (int e = 0; e < 7; ++e) o.pv[e] = R[(REC_PV + e) * nint + nb];
+#pragma unroll
+  for (int e = 0; e < 10; ++e) dv[e] = R[(REC_DV + e) * nint + nb];   // dv 0, 1, 6 .. 13
+  const double lam = sg * R[(REC_SPEC + 2 * q + (FWD ? 1 : 0)) * nint + nb];
+  const double ds = fma(nx[0], nx[0], fma(nx[1], nx[1], nx[2] * nx[2]));
+  const double vis = sg * R[REC_EVV * nint + nb] * ds;
+  const double u = fma(nx[0], o.pv[0], fma(nx[1], o.pv[1], nx[2] * o.pv[2]));
+  const double lv = lam + vis, su = s * (u + lv), sr = s * dv[0];
+  o.a[0] = s * fma(lam, R[REC_BETA * nint + nb], (u + vis) * dv[2]);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) { o.n[e] = s * nx[e]; o.a[1 + e] = sr * nx[e]; }
+  o.a[4] = su * dv[3]; o.a[5] = su * dv[4]; o.a[6] = su * dv[5];
+  o.ru = dv[0] * su;
+  o.h = fma(0.5, fma(o.pv[0], o.pv[0], fma(o.pv[1], o.pv[1], o.pv[2] * o.pv[2])), dv[1]);
+  o.c[0] = fma(o.ru, dv[6], -s * lv);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) o.c[1 + e] = o.ru * o.pv[e];
+  o.c[4] = o.ru * dv[7]; o.c[5] = o.ru * dv[8]; o.c[6] = o.ru * dv[9];
 }
 
-// the three lower (forward) or upper (backward) neighbours' products, added to acc
-template <bool FWD, bool CG = false>
-__device__ __forceinline__ void sweep_neighbours(const DevPtr& d, int npv, long long t, double* acc) {
-  const long long nint = d.nint;
-  const double* R = d.rec;
+// y = s A dq
+__device__ __forceinline__ void nb_product(const NbCoef& o, const double* dq, double* y) {
+  double r = o.a[0] * dq[0];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    // forward: lower neighbour through its + face; backward: upper neighbour through this
-    // cell's + face.  Neighbours outside the block carry dq = 0.
-    const int nb = FWD ? d.nbf[q * nint + t] : d.nbb[q * nint + t];
-    if (nb < 0) continue;
-    const long long fr = FWD ? nb : t;
-    double nx[3], pv[NPVM], dv[14], dq[NPVM];
-    for (int e = 0; e < 3; ++e) nx[e] = R[(REC_FACE + 3 * q + e) * nint + fr];
-    rec_state<double>(R, nint, nb, pv, dv);
-    // the dataflow sweep reads dq written during this launch by other CTAs: from L2 (CG)
-    for (int v = 0; v < NPVM; ++v) dq[v] = (v < npv) ? (CG ? __ldcg(d.dqs + v * nint + nb) : d.dqs[v * nint + nb]) : 0.0;
-    const double spec = R[(REC_SPEC + 2 * q + (FWD ? 1 : 0)) * nint + nb];
-    const double beta = R[REC_BETA * nint + nb];
-    const double evv = R[REC_EVV * nint + nb];
-    jac_apply_pre<double>(npv, nx, pv, dv, spec, beta, evv, FWD ? 1.0 : -1.0, dq, acc);
-  }
+  for (int e = 1; e < 7; ++e) r = fma(o.a[e], dq[e], r);
+  double g = o.h * r;
+#pragma unroll
+  for (int e = 0; e < 7; ++e) g = fma(o.c[e], dq[e], g);
+  y[0] = r;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) y[1 + e] = fma(o.pv[e], r, fma(o.n[e], dq[0], o.ru * dq[1 + e]));
+  y[4] = g;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) y[5 + e] = fma(o.pv[3 + e], r, o.ru * dq[5 + e]);
 }
 
-// one cell of a sweep: its three neighbours' products, the closed-form D^-1, dq
-template <bool FWD, bool CG>
+// x = D^-1 acc from the REC_SOL coefficients S (diag_solution): p, T and y1 over acc 0, the
+// energy combination w = u.acc(1..3) - acc 4 + (h - u^2 / 2) acc 0 and the advective parts
+// r5, r6 (r_v = acc v - pv v acc 0, where most of the cancellation is), the rest by rows
+__device__ __forceinline__ double sol_w(double hst, const double* pv3, const double* acc) {
+  return fma(hst, acc[0], fma(acc[3], pv3[2], fma(acc[2], pv3[1], acc[1] * pv3[0])) - acc[4]);
+}
+__device__ __forceinline__ double sol_r(const double* acc, int v, double pv) { return fma(-acc[0], pv, acc[v]); }
+__device__ __forceinline__ double sol_dense(const double* S, double a0, double w, double r5, double r6) {
+  return fma(S[2], r5, fma(S[1], w, fma(S[0], a0, S[3] * r6)));
+}
+
+// one cell of the hyperplane form
+template <bool FWD>
 __device__ __forceinline__ void sweep_cell(const DevPtr& d, const Par& c, long long t) {
   const long long nint = d.nint;
   const double* R = d.rec;
   const int npv = c.npv;
-  double pv[NPVM], dv[14], o[PREP_DIAG], acc[NPVM], x[NPVM];
-  rec_state<double>(R, nint, t, pv, dv);
-  for (int q = 0; q < PREP_DIAG; ++q) o[q] = R[(REC_DIAG + q) * nint + t];
-  for (int v = 0; v < NPVM; ++v) { acc[v] = 0.0; x[v] = 0.0; }
-  if (FWD) for (int v = 0; v < npv; ++v) acc[v] = R[(REC_RES + v) * nint + t];
-  else for (int v = 0; v < npv; ++v) acc[v] = d.dcv[v * nint + t];
-  sweep_neighbours<FWD, CG>(d, npv, t, acc);
-  if (FWD) for (int v = 0; v < npv; ++v) d.dcv[v * nint + t] = acc[v];
-  Diag D;
-  diag_from_array(o, D);
-  diag_solve(c, D, pv, dv, acc, x);
-  for (int v = 0; v < npv; ++v) d.dqs[v * nint + t] = x[v];
+  double acc[NPVM], x[NPVM], S[NSOL], pv[7];
+#pragma unroll
+  for (int v = 0; v < NPVM; ++v) {
+    acc[v] = x[v] = 0.0;
+    if (v < npv) acc[v] = FWD ? R[(REC_RES + v) * nint + t] : d.dcv[v * nint + t];
+  }
+  for (int q = 0; q < 3; ++q) {
+    // neighbours outside the block carry dq = 0
+    const int nb = FWD ? d.nbf[q * nint + t] : d.nbb[q * nint + t];
+    if (nb < 0) continue;
+    NbCoef o;
+    nb_coef<FWD>(R, nint, t, nb, q, o);
+    double dq[NPVM], y[NPVM];
+#pragma unroll
+    for (int v = 0; v < NPVM; ++v) dq[v] = (v < npv) ? d.dqs[v * nint + nb] : 0.0;
+    nb_product(o, dq, y);
+#pragma unroll
+    for (int v = 0; v < NPVM; ++v) acc[v] += y[v];
+  }
+#pragma unroll
+  for (int q = 0; q < NSOL; ++q) S[q] = R[(REC_SOL + q) * nint + t];
+#pragma unroll
+  for (int e = 0; e < 7; ++e) pv[e] = R[(REC_PV + e) * nint + t];
+  const double w = sol_w(S[SOL_H], pv, acc), r5 = sol_r(acc, 5, pv[3]), r6 = sol_r(acc, 6, pv[4]);
+  x[0] = sol_dense(S + SOL_P, acc[0], w, r5, r6);
+  x[4] = sol_dense(S + SOL_T, acc[0], w, r5, r6);
+  x[5] = sol_dense(S + SOL_Y, acc[0], w, r5, r6);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) x[1 + e] = sol_r(acc, 1 + e, pv[e]) * S[SOL_IA];
+  x[6] = r6 * S[SOL_IA];
+  const double r7 = sol_r(acc, 7, pv[5]), r8 = sol_r(acc, 8, pv[6]);
+  x[7] = fma(S[SOL_KW], r7, S[SOL_KW + 1] * r8);
+  x[8] = fma(S[SOL_KW + 2], r7, S[SOL_KW + 3] * r8);
+#pragma unroll
+  for (int v = 0; v < NPVM; ++v) {
+    if (v >= npv) continue;
+    if (FWD) d.dcv[v * nint + t] = acc[v];
+    d.dqs[v * nint + t] = x[v];
+  }
 }
 
 // one launch per hyperplane
@@ -1219,10 +1276,10 @@ template <bool FWD>
 __global__ void __launch_bounds__(64) k_sweep(DevPtr d, Par c, long long p0, long long p1) {
   const long long t = p0 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= p1) return;
-  sweep_cell<FWD, false>(d, c, t);
+  sweep_cell<FWD>(d, c, t);
 }
 
-// the dataflow sweeps' done flags: a release store by one thread after a barrier publishes
+// the tile sweeps' done flags: a release store by one thread after a barrier publishes
 // what the barrier ordered before it (release is cumulative), an acquire load followed by a
 // barrier makes it visible to the threads that passed the barrier
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -1246,105 +1303,141 @@ __device__ __forceinline__ void wait_flag(const DevPtr& d, const int* flag, long
   }
 }
 
-// what a dataflow sweep cell reads of one neighbour before its dq is known
-struct SweepNb {
-  int nb;
-  double nx[3], pv[NPVM], dv[14], spec, beta, evv;
-};
-
-template <bool FWD>
-__device__ __forceinline__ void sweep_nb_load(const DevPtr& d, long long t, int q, SweepNb& s) {
-  const long long nint = d.nint;
-  const double* R = d.rec;
-  s.nb = FWD ? d.nbf[q * nint + t] : d.nbb[q * nint + t];
-  if (s.nb < 0) return;
-  const long long fr = FWD ? s.nb : t;
-  for (int e = 0; e < 3; ++e) s.nx[e] = R[(REC_FACE + 3 * q + e) * nint + fr];
-  rec_state<double>(R, nint, s.nb, s.pv, s.dv);
-  s.spec = R[(REC_SPEC + 2 * q + (FWD ? 1 : 0)) * nint + s.nb];
-  s.beta = R[REC_BETA * nint + s.nb];
-  s.evv = R[REC_EVV * nint + s.nb];
-}
-
-template <bool FWD>
-__device__ __forceinline__ void sweep_nb_apply(const DevPtr& d, int npv, const SweepNb& s, double* acc) {
-  if (s.nb < 0) return;
-  const long long nint = d.nint;
-  double dq[NPVM];
-  for (int v = 0; v < NPVM; ++v) dq[v] = (v < npv) ? __ldcg(d.dqs + v * nint + s.nb) : 0.0;
-  jac_apply_pre<double>(npv, s.nx, s.pv, s.dv, s.spec, s.beta, s.evv, FWD ? 1.0 : -1.0, dq, acc);
-}
-
 // Dataflow sweep of the FP64 form: one persistent launch per sweep.  CTAs take chunks
 // (runs of at most SW_CH cells of one plane) in plane order -- reversed for the backward
-// sweep -- from a ticket counter.  A chunk's cells need the dq of their lower (upper)
-// neighbours, which lie in a few chunks of the previous (next) plane.  Each cell first
-// loads everything that does not depend on those dq (its own record, the neighbours'
-// records); then the CTA waits for the needed chunks' done flags (one polling thread per
-// flag), runs the hyperplane kernel's arithmetic and raises its own chunk's flag.  The
-// needed chunks always hold earlier tickets, so the earliest unfinished chunk never waits
-// and its CTA is running: the waits end.  Each wait is still bounded by `spin` polls; a
+// sweep -- from a ticket counter.  What bounds it is the chain over the ni + nj + nk planes:
+// a plane waits for the dq of the previous one, forms its products and solves its diagonal
+// blocks, and one warp issues an FP64 instruction every 64 clocks whatever it does (four
+// warps one every 19 together).  So
+//  - all that does not depend on the neighbours' dq is done before the wait (the products'
+//    coefficients here, those of D^-1 in k_rhs), which leaves 32 instructions per product
+//    and 32 for the solve of 290 together;
+//  - a chunk's cells are worked on by four warps: warps 0 to 2 form the products of the
+//    three neighbours, the sums of the nine components and then the solution's components
+//    are dealt over all four;
+//  - dq itself is the signal: dqs starts as all ones (a NaN pattern that no result keeps),
+//    and a lane polls its neighbour's values until none of them is.  A flag would cost the
+//    writer a fence after its stores and the reader a second round trip to L2.
+// With one warp per chunk and flags a plane took 11.4 us (128x64x64 cells, 254 planes).
+// The needed chunks always hold earlier tickets, so the earliest unfinished chunk never
+// waits and its CTA is running: the waits end.  Each wait is still bounded by `spin` polls; a
 // wait that runs out records sweep_stall, which also ends every other wait, so the launch
 // completes and the host reports CFD3D_ERR_TIMEOUT.  `withhold` >= 0 names a chunk whose
-// flag is never raised (the stall test).
+// dq is never written (the stall test).
+constexpr unsigned long long DQ_UNSET = ~0ull;
+
+__device__ __forceinline__ unsigned long long ld_relaxed(const double* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_dq(double* p, double x) {
+  unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  if (b == DQ_UNSET) b = 0x7ff8000000000000ull;   // (a NaN all the same)
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" : : "l"(p), "l"(b) : "memory");
+}
+
 template <bool FWD>
-__global__ void __launch_bounds__(SW_CH) k_sweep_df(DevPtr d, Par c, long long spin, int withhold) {
-  __shared__ int s_q, s_lo[SW_CH / 32], s_hi[SW_CH / 32];
+__global__ void __launch_bounds__(4 * SW_CH) k_sweep_df(DevPtr d, Par c, long long spin, int withhold) {
+  __shared__ int s_q;
+  __shared__ double s_part[3][NPVM][SW_CH], s_acc[NPVM][SW_CH];
   const long long nint = d.nint;
   const int npv = c.npv;
+  const double* R = d.rec;
   unsigned* ticket = d.tickets + (FWD ? 0 : 1);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // the components whose sum and, below, whose solution this warp forms
+  const int v0 = (w == 0) ? 0 : 2 * w + 1, v1 = min(npv, 2 * w + 3);
   for (;;) {
     if (threadIdx.x == 0) s_q = (int)atomicAdd(ticket, 1u);
     __syncthreads();
     const int q = s_q;
     if (q >= d.nchunk) return;
     const int ch = FWD ? q : d.nchunk - 1 - q;
-    const long long t = d.chunk_t0[ch] + threadIdx.x;
+    const long long t = d.chunk_t0[ch] + lane;
     const bool live = t < d.chunk_t0[ch + 1];
-    // ---- work that does not wait: own record, neighbour records, the needed chunks
-    SweepNb nbs[3];
-    double acc[NPVM], pv[NPVM], dv[14], o[PREP_DIAG];
-    int lo = 0x7fffffff, hi = -1;
+    // ---- before the wait: this warp's coefficients
+    int nb = -1;
+    NbCoef o;
+    double base[3] = {0.0, 0.0, 0.0}, S[9], pv[7], hst = 0.0;
     if (live) {
-      const double* R = d.rec;
-      rec_state<double>(R, nint, t, pv, dv);
-      for (int k = 0; k < PREP_DIAG; ++k) o[k] = R[(REC_DIAG + k) * nint + t];
-      for (int v = 0; v < NPVM; ++v) acc[v] = 0.0;
-      if (FWD) for (int v = 0; v < npv; ++v) acc[v] = R[(REC_RES + v) * nint + t];
-      else for (int v = 0; v < npv; ++v) acc[v] = d.dcv[v * nint + t];
-      for (int k = 0; k < 3; ++k) {
-        sweep_nb_load<FWD>(d, t, k, nbs[k]);
-        if (nbs[k].nb >= 0) {
-          const int cn = d.chunk_of[nbs[k].nb];
-          lo = min(lo, cn);
-          hi = max(hi, cn);
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+        if (v0 + m < v1) base[m] = FWD ? R[(REC_RES + v0 + m) * nint + t] : d.dcv[(v0 + m) * nint + t];
+#pragma unroll
+      for (int e = 0; e < 7; ++e) pv[e] = R[(REC_PV + e) * nint + t];
+      const int s0 = (w == 0) ? SOL_P : (w == 1) ? SOL_T : (w == 2) ? SOL_Y : SOL_IA;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[e] = R[(REC_SOL + s0 + e) * nint + t];
+      S[4] = R[(REC_SOL + SOL_IA) * nint + t];
+      hst = R[(REC_SOL + SOL_H) * nint + t];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[5 + e] = R[(REC_SOL + SOL_KW + e) * nint + t];
+      if (w < 3) nb = FWD ? d.nbf[w * nint + t] : d.nbb[w * nint + t];
+      if (nb >= 0) nb_coef<FWD>(R, nint, t, nb, w, o);
+    }
+    // ---- the wait and the products
+    if (w < 3) {
+      double y[NPVM];
+#pragma unroll
+      for (int v = 0; v < NPVM; ++v) y[v] = 0.0;
+      unsigned long long b[NPVM];
+      long long it = 0;
+      for (;;) {
+        bool set = true;
+        if (nb >= 0) {
+#pragma unroll
+          for (int v = 0; v < NPVM; ++v) b[v] = (v < npv) ? ld_relaxed(d.dqs + v * nint + nb) : 0ull;
+#pragma unroll
+          for (int v = 0; v < NPVM; ++v) set = set && b[v] != DQ_UNSET;
+        }
+        if (__all_sync(0xffffffffu, set)) break;
+        ++it;
+        if ((it & 63) == 0 && *(volatile int*)&d.sc->sweep_stall) break;
+        if (it > spin) { atomicExch(&d.sc->sweep_stall, 1); break; }
+        if (it > 2) __nanosleep(it > 64 ? 200 : 20);
+      }
+      if (nb >= 0) {
+        double dq[NPVM];
+#pragma unroll
+        for (int v = 0; v < NPVM; ++v) dq[v] = __longlong_as_double((long long)b[v]);
+        nb_product(o, dq, y);
+      }
+#pragma unroll
+      for (int v = 0; v < NPVM; ++v) s_part[w][v][lane] = y[v];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const int v = v0 + m;
+      if (v >= v1) continue;
+      const double a = ((base[m] + s_part[0][v][lane]) + s_part[1][v][lane]) + s_part[2][v][lane];
+      s_acc[v][lane] = a;
+      if (FWD && live) d.dcv[v * nint + t] = a;
+    }
+    __syncthreads();
+    if (live && ch != withhold) {
+      double acc[NPVM];
+#pragma unroll
+      for (int v = 0; v < NPVM; ++v) acc[v] = (v < npv) ? s_acc[v][lane] : 0.0;
+      double* X = d.dqs + t;
+      if (w < 3) {
+        const double r5 = sol_r(acc, 5, pv[3]), r6 = sol_r(acc, 6, pv[4]);
+        st_dq(X + (w == 0 ? 0 : 3 + w) * nint, sol_dense(S, acc[0], sol_w(hst, pv, acc), r5, r6));
+        if (w == 0) st_dq(X + 6 * nint, r6 * S[4]);
+        if (w == 2 && npv > 7) {
+          const double r7 = sol_r(acc, 7, pv[5]), r8 = sol_r(acc, 8, pv[6]);
+          st_dq(X + 8 * nint, fma(S[7], r7, S[8] * r8));
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 3; ++e) st_dq(X + (1 + e) * nint, sol_r(acc, 1 + e, pv[e]) * S[4]);
+        if (npv > 7) {
+          const double r7 = sol_r(acc, 7, pv[5]), r8 = sol_r(acc, 8, pv[6]);
+          st_dq(X + 7 * nint, fma(S[5], r7, S[6] * r8));
         }
       }
     }
-    for (int k = 16; k > 0; k >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, k));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, k));
-    }
-    if (lane == 0) { s_lo[wid] = lo; s_hi[wid] = hi; }
-    __syncthreads();
-    for (int w = 0; w < SW_CH / 32; ++w) { lo = min(lo, s_lo[w]); hi = max(hi, s_hi[w]); }
-    // ---- wait: thread k polls chunks lo + k, lo + k + SW_CH, ... (none when no cell of
-    // the chunk has a neighbour: then hi = -1 and lo is not a chunk index)
-    for (int cn = (hi >= 0) ? lo + (int)threadIdx.x : 0; hi >= 0 && cn <= hi; cn += SW_CH) wait_flag(d, d.done + cn, spin);
-    __syncthreads();
-    if (live) {
-      double x[NPVM];
-      for (int k = 0; k < 3; ++k) sweep_nb_apply<FWD>(d, npv, nbs[k], acc);
-      if (FWD) for (int v = 0; v < npv; ++v) d.dcv[v * nint + t] = acc[v];
-      Diag D;
-      diag_from_array(o, D);
-      for (int v = 0; v < NPVM; ++v) x[v] = 0.0;
-      diag_solve(c, D, pv, dv, acc, x);
-      for (int v = 0; v < npv; ++v) d.dqs[v * nint + t] = x[v];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && ch != withhold) st_release(d.done + ch, 1);
   }
 }
 
@@ -1891,8 +1984,9 @@ int ensure_copy_stream(cfd3d_handle* h) {
   return CFD3D_OK;
 }
 
-// polls of a neighbour's done flag before a dataflow sweep gives up (about 0.1-0.5 s)
-constexpr long long SWEEP_SPIN = 1ll << 22;
+// polls of a tile's done flag, and of a neighbour's dq in the FP64 form, before a sweep gives
+// up (some tenths of a second)
+constexpr long long SWEEP_SPIN = 1ll << 22, SWEEP_SPIN_DQ = 1ll << 19;
 
 // k_rhs in the instantiation of the form (mixed / FP64), the time integrator (sweep records
 // for LU-SGS) and the extended sources (DES length scale, gravity)
@@ -1980,6 +2074,11 @@ int launch_boundary(const Engine& E, cudaStream_t s) {
   return n;
 }
 
+// dqs as the FP64 form's dataflow sweeps expect it at their start
+void unset_dq(const Engine& E, cudaStream_t s) {
+  cudaMemsetAsync(E.d.dqs, 0xff, (size_t)E.par.npv * E.nint * sizeof(double), s);
+}
+
 // the launch sequence of one iteration (captured into the graph); `mark` (optional)
 // records an event after each stage for the stage profile
 void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
@@ -2049,13 +2148,13 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
     k_sweep_tile<false><<<E.sweep_grid, 32, TILE_SMEM, s>>>(d, c, SWEEP_SPIN, -1);
     n += 2;
   } else if (!E.sweep_planes) {
-    // dataflow sweeps: flags and tickets cleared, one persistent launch per sweep
+    // dataflow sweeps: tickets cleared and dq unset, one persistent launch per sweep
     cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), s);
-    cudaMemsetAsync(d.done, 0, (size_t)d.nchunk * sizeof(int), s);
-    k_sweep_df<true><<<E.sweep_grid, SW_CH, 0, s>>>(d, c, SWEEP_SPIN, -1);
+    unset_dq(E, s);
+    k_sweep_df<true><<<E.sweep_grid, 4 * SW_CH, 0, s>>>(d, c, SWEEP_SPIN_DQ, -1);
     stage(5);
-    cudaMemsetAsync(d.done, 0, (size_t)d.nchunk * sizeof(int), s);
-    k_sweep_df<false><<<E.sweep_grid, SW_CH, 0, s>>>(d, c, SWEEP_SPIN, -1);
+    unset_dq(E, s);
+    k_sweep_df<false><<<E.sweep_grid, 4 * SW_CH, 0, s>>>(d, c, SWEEP_SPIN_DQ, -1);
     n += 2;
   } else {
     const int np = (int)E.plane_off.size() - 1;
@@ -2405,10 +2504,11 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
     ok = ok && allocf(E.d.pvf, c.npv) && allocf(E.d.fi32, 3 * c.npv) && allocf(E.d.fv32, (c.iturb == -3) ? 1 : 3 * c.npv) &&
          allocf(E.d.frec, 2 * 12) && allocf(E.d.lqf, NLQ);
   else {
-    // the face reconstruction's scratch: all three directions at once up to 256 MB of it (larger
-    // cases fill the GPU one direction at a time)
+    // the face reconstruction's scratch: all three directions at once up to 128 MB of it.  A
+    // launch per direction leaves three partial last waves (the face stage of 128x64x64 cells
+    // 7.5 ms against 7.4), which is less than a larger allocation costs a short run.
     E.d.nfs = (c.nmuscl == 2) ? 5 : (c.nmuscl > 0 ? 1 : 0);
-    E.d.fslots = (3.0 * E.d.nfs * c.npv * 8.0 * (double)n <= 2.56e8) ? 3 : 1;
+    E.d.fslots = (3.0 * E.d.nfs * c.npv * 8.0 * (double)n <= 1.28e8) ? 3 : 1;
     ok = ok && alloc(E.d.fi, 3 * c.npv) && alloc(E.d.fv, (c.iturb == -3) ? 1 : 3 * c.npv) &&
          alloc(E.d.fsc, (long long)E.d.fslots * E.d.nfs * c.npv);
   }
@@ -2541,9 +2641,8 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   E.d.cells = E.d_planes; E.d.pos = E.d_pos; E.d.nbf = E.d_nbf; E.d.nbb = E.d_nbb;
   if (!E.d_planes || !E.d_pos || !E.d_nbf || !E.d_nbb) { E.err = "device allocation failed (sweep maps)"; return CFD3D_ERR_NOMEM; }
   if (cudaMalloc(&E.d.rec, (size_t)NREC * E.nint * 8) != cudaSuccess) { E.err = "device allocation failed (sweep records)"; return CFD3D_ERR_NOMEM; }
-  if (cudaMalloc(&E.d.done, (size_t)E.d.nchunk * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&E.d.tickets, 2 * sizeof(unsigned)) != cudaSuccess) {
-    E.err = "device allocation failed (sweep flags)";
+  if (cudaMalloc(&E.d.tickets, 2 * sizeof(unsigned)) != cudaSuccess) {
+    E.err = "device allocation failed (sweep tickets)";
     return CFD3D_ERR_NOMEM;
   }
   {
@@ -2552,7 +2651,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, SW_CH, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
     E.sweep_grid = std::max(1, std::min(std::min(per, 8) * nsm, E.d.nchunk));
   }
   CFD_CUDA(cudaDeviceSynchronize());
@@ -2586,9 +2685,6 @@ void cfd3d_destroy(cfd3d_handle* h) {
   cudaFree(E.d.done);
   cudaFree(E.d.tickets);
   cudaFree(E.d_chunk_t0);
-  cudaFree(E.d_chunk_of);
-  cudaFree(E.d.recf);
-  cudaFree(E.d.dqsf);
   cudaFree(E.d_tiles);
   cudaFree(E.d.trf);
   cudaFree(E.d.tq);
@@ -3286,7 +3382,7 @@ int cfd3d_autotune(cfd3d_handle* h, int reps, int* choice) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_tile<true>, 32, TILE_SMEM);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, SW_CH, 0);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
   const int nwork = c.mixed ? d.ntile : d.nchunk;
   int bestg = E.sweep_grid;
   tbest = 1e30f;
@@ -3297,12 +3393,14 @@ int cfd3d_autotune(cfd3d_handle* h, int reps, int* choice) {
     // rewrites the right-hand side it reads, which changes the values but not the work)
     const float t = time_calls(E, reps, [&] {
       cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), E.st);
-      cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
+      if (c.mixed) cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
+      else unset_dq(E, E.st);
       if (c.mixed) k_sweep_tile<true><<<grid, 32, TILE_SMEM, E.st>>>(d, c, SWEEP_SPIN, -1);
-      else k_sweep_df<true><<<grid, SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN, -1);
-      cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
+      else k_sweep_df<true><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN_DQ, -1);
+      if (c.mixed) cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
+      else unset_dq(E, E.st);
       if (c.mixed) k_sweep_tile<false><<<grid, 32, TILE_SMEM, E.st>>>(d, c, SWEEP_SPIN, -1);
-      else k_sweep_df<false><<<grid, SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN, -1);
+      else k_sweep_df<false><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN_DQ, -1);
     });
     if (t < tbest) { tbest = t; bestg = grid; }
   }
@@ -3334,9 +3432,10 @@ int cfd3d_sweep_stall_test(cfd3d_handle* h) {
   // raises its flags, with a short poll limit
   launch_iteration(E, false);
   CFD_CUDA(cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), E.st));
-  CFD_CUDA(cudaMemsetAsync(d.done, 0, (size_t)(c.mixed ? d.ntile : d.nchunk) * sizeof(int), E.st));
+  if (c.mixed) CFD_CUDA(cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), E.st));
+  else unset_dq(E, E.st);
   if (c.mixed) k_sweep_tile<true><<<E.sweep_grid, 32, TILE_SMEM, E.st>>>(d, c, 1 << 12, 0);
-  else k_sweep_df<true><<<E.sweep_grid, SW_CH, 0, E.st>>>(d, c, 1 << 12, 0);
+  else k_sweep_df<true><<<E.sweep_grid, 4 * SW_CH, 0, E.st>>>(d, c, 1 << 12, 0);
   CFD_CUDA(cudaStreamSynchronize(E.st));
   CFD_CUDA(cudaGetLastError());
   Scalars sc;
@@ -3463,7 +3562,7 @@ int cfd3d_set_launch_shapes(cfd3d_handle* h, const int* shapes) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_tile<true>, 32, TILE_SMEM);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, SW_CH, 0);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
   if (shapes[2] < 1 || shapes[2] > std::max(per, 1)) { E.err = "sweep CTAs per SM outside 1 .. the occupancy limit"; return CFD3D_ERR_ARG; }
   const int nb = (int)E.blk.size();
   if (shapes[3] < 1 || shapes[3] > std::min(nb, Engine::MAX_PIPE) || (!c.mixed && shapes[3] != 1)) {

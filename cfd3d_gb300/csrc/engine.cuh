@@ -170,16 +170,11 @@ struct DevPtr {
   double* rec;
   const int *cells, *pos, *nbf, *nbb;
   // dataflow sweeps: chunk starts in t (chunks of at most SW_CH cells, never across a
-  // plane; nchunk + 1 entries), the chunk of every t, per-chunk done flags, the two
-  // sweeps' chunk tickets
+  // plane; nchunk + 1 entries), the two sweeps' chunk tickets; the tile sweeps' done flags
   const int* chunk_t0;
-  const int* chunk_of;
   int nchunk;
   int* done;
   unsigned* tickets;
-  // mixed form: FP32 copy of the neighbour part of the records (the first REC_DIAG
-  // planes) and FP32 dq
-  float *recf, *dqsf;
   // mixed form: the tile sweeps (setup_tiles).  tiles in forward ticket order; trf the FP32
   // tile records; tq the own part D^-1 res per slot (k_rhs, an FP32 solve); tyf / tyb the
   // FP32 corrections of the forward / backward sweep, so that dq = tq + tyf + tyb (k_update);
@@ -202,9 +197,9 @@ enum {
   REC_EVV = 18,
   REC_SPEC = 19,   // 6 face spectral radii
   REC_FACE = 25,   // the cell's + face vectors cx, ex, tx
-  REC_DIAG = 34,   // 23 values of the closed-form diagonal block
-  REC_RES = 57,    // residual (npv)
-  NREC = 66
+  REC_SOL = 34,    // the coefficients of D^-1 (SOL_*)
+  REC_RES = 52,    // residual (npv)
+  NREC = 61
 };
 
 struct Engine {
@@ -228,7 +223,6 @@ struct Engine {
   int* d_nbb = nullptr;
   std::vector<long long> plane_off;
   int* d_chunk_t0 = nullptr;   // dataflow sweep chunks (setup_planes)
-  int* d_chunk_of = nullptr;
   TileDesc* d_tiles = nullptr;  // the mixed form's tiles (setup_tiles)
   int sweep_grid = 0;          // persistent CTAs of the dataflow sweep
   int sweep_planes = 0;        // 1: one launch per hyperplane instead (CFD3D_SWEEP=planes)

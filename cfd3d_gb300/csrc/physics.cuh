@@ -1397,11 +1397,6 @@ __device__ __forceinline__ void diag_solve_t(const Par& c, const DiagT<R>& D, co
   }
   for (int n = 0; n < c.npv; ++n) x[n] *= D.a;
 }
-__device__ __forceinline__ void diag_solve(const Par& c, const Diag& D, const double* pv, const double* dv,
-                                           const double* res, double* x) {
-  diag_solve_t<double>(c, D, pv, dv, res, x);
-}
-
 // the Diag fields as an array (the sweep record's diagonal part)
 constexpr int PREP_DIAG = 23;
 
@@ -1412,13 +1407,33 @@ __device__ __forceinline__ void diag_to_array(const DiagT<R>& D, R* o) {
   for (int q = 0; q < 4; ++q) { o[14 + q] = D.c[q]; o[19 + q] = D.t[q]; }
   o[18] = D.tt;
 }
-template <class R>
-__device__ __forceinline__ void diag_from_array(const double* o, DiagT<R>& D) {
-  D.a = (R)o[0]; D.b1 = (R)o[1]; D.i_b1 = (R)o[2]; D.ss = (R)o[3]; D.rr = (R)o[4]; D.cross = (R)o[5];
-  D.cross1 = (R)o[6]; D.cross2 = (R)o[7]; D.ssy1 = (R)o[8]; D.ssy2 = (R)o[9]; D.ssh = (R)o[10]; D.aaa1 = (R)o[11];
-  D.aaa2 = (R)o[12]; D.mm = (R)o[13];
-  for (int q = 0; q < 4; ++q) { D.c[q] = (R)o[14 + q]; D.t[q] = (R)o[19 + q]; }
-  D.tt = (R)o[18];
+// D^-1 of the FP64 sweeps as coefficients (diag_solve_t's algebra collected by its inputs):
+// x0, x4 and x5 over res0, w = u.res(1..3) - res4 + hst res0, r5 and r6 (r_v = res v - pv v
+// res0); 1 / (b1 rho) times a; the k-omega block over r7 and r8; hst = h - u^2 / 2
+enum { SOL_P = 0, SOL_T = 4, SOL_Y = 8, SOL_IA = 12, SOL_KW = 13, SOL_H = 17, NSOL = 18 };
+__device__ __forceinline__ void diag_solution(const Diag& D, const double* pv, const double* dv, double* S) {
+  const double* C = D.c;
+  const double bd = D.b1 * dv[0], m = D.mm * D.a, e2 = C[2] + bd, c3 = C[3] * D.i_b1, c1 = C[1] * D.i_b1;
+  const double k3 = -(C[2] * D.i_b1 + 1.0), dr = dv[0] * D.rr, q3 = -(bd * (1.0 - dv[10] * dv[0]));
+  S[0] = m * dv[0] * (e2 * dv[11] - C[1] * dv[12]);
+  S[1] = m * (e2 * dv[7] - C[1] * dv[8]);
+  S[2] = m * bd * D.cross1;
+  S[3] = m * (e2 * D.cross2 - C[3] * D.cross1 - C[1] * D.cross);
+  S[4] = m * (C[0] * dv[12] * dv[0] + k3 * q3);
+  S[5] = m * (C[0] * dv[8] + k3 * dr);
+  S[6] = -m * D.ssy1;
+  S[7] = m * (c3 * D.ssy1 + C[0] * D.cross + k3 * D.ssy2);
+  S[8] = m * (c1 * q3 - C[0] * dv[11] * dv[0]);
+  S[9] = m * (c1 * dr - C[0] * dv[7]);
+  S[10] = m * D.ss;
+  S[11] = m * (c1 * D.ssy2 - c3 * D.ss - C[0] * D.cross2);
+  S[SOL_H] = dv[1] - 0.5 * (pv[1] * pv[1] + pv[2] * pv[2] + pv[3] * pv[3]);
+  S[SOL_IA] = D.i_b1 * D.a;
+  const double ta = D.tt * D.a;
+  S[SOL_KW] = -(bd + D.t[3]) * ta;
+  S[SOL_KW + 1] = D.t[1] * ta;
+  S[SOL_KW + 2] = D.t[2] * ta;
+  S[SOL_KW + 3] = -(bd + D.t[0]) * ta;
 }
 
 // spectral radius of the split Jacobian for one face: 1.05 (|u'| + d)
@@ -1433,7 +1448,7 @@ __device__ __forceinline__ R face_spectral(const Par& c, const R* nx, const R* p
 }
 
 // acc += sign_acc * 0.5 * A dq with the precomputed spectral radius `spec`, beta and
-// evv = 2 eigenvis / vol of the neighbour (same algebra as jac_apply); R = float is the
+// evv = 2 eigenvis / vol of the neighbour; R = float is the
 // mixed form's neighbour product
 template <class R>
 __device__ __forceinline__ void jac_apply_pre(int npv, const R* nx, const R* pv, const R* dv, R spec, R beta, R evv,
@@ -1462,44 +1477,6 @@ __device__ __forceinline__ void jac_apply_pre(int npv, const R* nx, const R* pv,
     acc[7] += s * (pv[7] * r0 + ru * dq[7]);
     acc[8] += s * (pv[8] * r0 + ru * dq[8]);
   }
-}
-
-// acc += sign_acc * A(sign) dq for the neighbour cell state (pv, dv, tv, vol) across face nx
-__device__ __forceinline__ void jac_apply(const Par& c, const double* nx, double vol, const double* pv,
-                                          const double* dv, const double* tv, double sign, const double* dq,
-                                          double* acc, double sign_acc) {
-  const double cappa = 1.05;
-  double ds = nx[0] * nx[0] + nx[1] * nx[1] + nx[2] * nx[2];
-  double u = nx[0] * pv[1] + nx[1] * pv[2] + nx[2] * pv[3];
-  double sndp2 = sndp2_of<double>(c, dv[5], pv[1] * pv[1] + pv[2] * pv[2] + pv[3] * pv[3]);
-  double up = 0.5 * (1.0 + sndp2 / dv[5]) * u;
-  double d = 0.5 * sqrt(u * u * sq(1.0 - sndp2 / dv[5]) + 4.0 * sndp2 * ds);
-  double lamda = sign * cappa * (fabs(up) + d);
-  double vis = sign * 2.0 * eigenvis_of(c, dv, tv) * ds / vol;
-  double beta = 1.0 / sndp2 - 1.0 / dv[5] + dv[6];
-  double uuu = u + lamda + vis;
-  double lv = lamda + vis;
-  // row 1: a1..a7 (+ g, ge shifts)
-  double r0 = (u * dv[6] + lamda * beta + vis * dv[6]) * dq[0] + nx[0] * dv[0] * dq[1] + nx[1] * dv[0] * dq[2] +
-              nx[2] * dv[0] * dq[3] + (u * dv[7] + lv * dv[7]) * dq[4] + (u * dv[8] + lv * dv[8]) * dq[5] +
-              (u * dv[9] + lv * dv[9]) * dq[6];
-  double ru = dv[0] * uuu;
-  double h = dv[1] + 0.5 * (pv[1] * pv[1] + pv[2] * pv[2] + pv[3] * pv[3]);
-  double y[NPVM];
-  y[0] = r0;
-  y[1] = pv[1] * r0 + nx[0] * dq[0] + ru * dq[1];
-  y[2] = pv[2] * r0 + nx[1] * dq[0] + ru * dq[2];
-  y[3] = pv[3] * r0 + nx[2] * dq[0] + ru * dq[3];
-  y[4] = ru * (dv[10] * dq[0] + pv[1] * dq[1] + pv[2] * dq[2] + pv[3] * dq[3] + dv[11] * dq[4] + dv[12] * dq[5] +
-               dv[13] * dq[6]) + h * r0 - lv * dq[0];
-  y[5] = pv[5] * r0 + ru * dq[5];
-  y[6] = pv[6] * r0 + ru * dq[6];
-  if (c.npv > 7) {
-    y[7] = pv[7] * r0 + ru * dq[7];
-    y[8] = pv[8] * r0 + ru * dq[8];
-  }
-  double s = 0.5 * sign_acc;
-  for (int n = 0; n < c.npv; ++n) acc[n] += s * y[n];
 }
 
 }  // namespace cfd
