@@ -15,13 +15,13 @@ ROOT = os.path.dirname(HERE)
 SRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libcfd3d_gb300.so")
-UNITS = ["adjoint_face.cu", "adjoint.cu", "engine.cu", "setup.cu", "flux.cu", "flux_mixed.cu", "peak.cu"]
+UNITS = ["adjoint_face.cu", "adjoint_duals.cu", "adjoint.cu", "engine.cu", "setup.cu", "flux.cu", "flux_mixed.cu", "peak.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-I", os.path.join(ROOT, "include")]
-# the adjoint's dual-number kernels are large and off the iteration's path: the device
-# compiler's fast-compile mode keeps their build at seconds instead of minutes
-UNIT_FLAGS = {"adjoint.cu": ["-Ofc", "mid"], "adjoint_face.cu": ["-Ofc", "mid"]}
+# the adjoint's dual-number routines are large and off the common path: the device compiler's
+# fast-compile mode keeps their build at seconds instead of minutes
+UNIT_FLAGS = {"adjoint_duals.cu": ["-Ofc", "mid"]}
 
 
 def nvcc():

@@ -13,10 +13,8 @@
 // limiter, clip, upwind and branch switches are recomputed from the state):
 //   k_ghost x3        the forward boundary program, so the ghost cells hold the values the
 //                     residual saw;
-//   k_adj_face x3     per face (adjoint_face.cu): the local Jacobian of the inviscid and viscous flux with
-//                     respect to its stencil, by forward-mode dual numbers over the same
-//                     templated routines as the forward kernels (reconstruction per variable,
-//                     face EOS by its derivatives, flux core, viscous core);
+//   the face kernels  per face (adjoint_face.cu): the inviscid and viscous flux and the
+//                     reconstruction reversed, from the forward kernels' face states;
 //   k_adj_cell        per cell: cavitation, SST and dual-time sources;
 //   k_adj_ghost x3    the boundary program in reverse phase order (corners, edges, faces and
 //                     halos): each ghost's gradient pushed to the cells it was made from;
@@ -27,131 +25,6 @@
 #include "adjoint.cuh"
 
 namespace cfd {
-
-// ------------------------------------------------------------------ cell sources
-// Per interior cell: the cavitation source (res(6)), the SST sources (res(8:9)) and the
-// dual-time source, as k_rhs adds them (src/rhs_module.f90:540-642).
-__global__ void __launch_bounds__(64) k_adj_cell(DevPtr d, Par c, AdjPtr a) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double wp[3] = {0.0, 0.0, 0.0};
-  if (t < d.nint) {
-    const int b = find_block_interior(d.blk, d.nblk, t);
-    int i, j, k;
-    const BlockGeom& B = d.blk[b];
-    const long long g = interior_cell(B, t - B.int_off, i, j, k);
-    const long long n = d.ncell, sj = B.ni, sk = (long long)B.ni * B.nj;
-    const int npv = c.npv;
-    double lam[NPVM], pv2[NPVM], dv[NDV];
-    for (int v = 0; v < NPVM; ++v) {
-      lam[v] = (v < npv) ? a.lam[v * n + g] : 0.0;
-      pv2[v] = (v < npv) ? d.pv[v * n + g] : 0.0;
-    }
-    for (int v = 0; v < NDV; ++v) dv[v] = d.dv[v * n + g];
-    const double vol = d.gm[GM_GRD * n + g];
-    double gp[NPVM], gd[NGD];
-    for (int v = 0; v < NPVM; ++v) gp[v] = 0.0;
-    for (int m = 0; m < NGD; ++m) gd[m] = 0.0;
-    // ---- cavitation: res(6) += r_v - r_c; seeds p, T, y1, y2, rho, rho_l, rho_v, rho_g (Kunz's
-    // gas volume fraction), uref, c_v, c_c
-    if (c.ncav && lam[5] != 0.0) {
-      const int pvs[4] = {0, 4, 5, 6};
-      const int dvs[4] = {0, 2, 3, 4};
-      double w[11];
-      for (int k0 = 0; k0 < 11; k0 += DC) {
-        DD p2[NPVM], dd[NDV];
-        for (int v = 0; v < NPVM; ++v) p2[v] = DD(pv2[v]);
-        for (int q = 0; q < NDV; ++q) dd[q] = DD(dv[q]);
-        for (int m = 0; m < 4; ++m) p2[pvs[m]] = seed(pv2[pvs[m]], m, k0);
-        for (int m = 0; m < 4; ++m) dd[dvs[m]] = seed(dv[dvs[m]], 4 + m, k0);
-        const CavOutT<DD> o = cavsource_t<DD>(c, p2, dd, vol, seed(c.uref, 8, k0), seed(c.c_v, 9, k0),
-                                              seed(c.c_c, 10, k0));
-        for (int q = 0; q < DC && k0 + q < 11; ++q) w[k0 + q] = lam[5] * (o.r_v.d[q] - o.r_c.d[q]);
-      }
-      for (int m = 0; m < 4; ++m) gp[pvs[m]] += w[m];
-      gd[GD_RHO] += w[4]; gd[GD_RL] += w[5]; gd[GD_RV] += w[6]; gd[GD_RG] += w[7];
-      wp[0] += w[8]; wp[1] += w[9]; wp[2] += w[10];
-    }
-    // ---- SST: res(8) += r7, res(9) += r8; seeds the 15 cell gradients, k, omega, rho, mu, mu_t
-    if (c.iturb == 0 && (lam[7] != 0.0 || lam[8] != 0.0)) {
-      const long long nbr[6] = {g - 1, g + 1, g - sj, g + sj, g - sk, g + sk};
-      double fa[6][3];
-      for (int q = 0; q < 3; ++q) {
-        fa[0][q] = d.gm[(GM_CX + q) * n + g - 1]; fa[1][q] = d.gm[(GM_CX + q) * n + g];
-        fa[2][q] = d.gm[(GM_EX + q) * n + g - sj]; fa[3][q] = d.gm[(GM_EX + q) * n + g];
-        fa[4][q] = d.gm[(GM_TX + q) * n + g - sk]; fa[5][q] = d.gm[(GM_TX + q) * n + g];
-      }
-      const int gv[5] = {1, 2, 3, 7, 8};
-      double grv[5][3];
-      const double ivol = 1.0 / vol;
-      for (int q = 0; q < 5; ++q) {
-        const double* P = d.pv + gv[q] * n;
-        const double c0 = P[g];
-        const double v1 = 0.5 * (P[nbr[0]] + c0), v2 = 0.5 * (P[nbr[1]] + c0), v3 = 0.5 * (P[nbr[2]] + c0);
-        const double v4 = 0.5 * (P[nbr[3]] + c0), v5 = 0.5 * (P[nbr[4]] + c0), v6 = 0.5 * (P[nbr[5]] + c0);
-        for (int e = 0; e < 3; ++e)
-          grv[q][e] = (v2 * fa[1][e] + v4 * fa[3][e] + v6 * fa[5][e] - v1 * fa[0][e] - v3 * fa[2][e] - v5 * fa[4][e]) * ivol;
-      }
-      const double mu = d.tv[g], mut = d.tv[2 * n + g];
-      const double y5 = d.gm[(GM_GRD + 4) * n + g];
-      double w[20];
-      const double hmax = c.ides ? grid_hmax<double>(fa, vol) : 0.0;
-      for (int k0 = 0; k0 < 20; k0 += DC) {
-        DD gr[5][3];
-        for (int q = 0; q < 5; ++q)
-          for (int e = 0; e < 3; ++e) gr[q][e] = seed(grv[q][e], 3 * q + e, k0);
-        const SstOut<DD> so = sst_source<DD>(gr, seed(pv2[7], 15, k0), seed(pv2[8], 16, k0), seed(dv[0], 17, k0),
-                                             seed(mu, 18, k0), seed(mut, 19, k0), y5, vol, c.ides, hmax);
-        for (int q = 0; q < DC && k0 + q < 20; ++q) w[k0 + q] = lam[7] * so.r7.d[q] + lam[8] * so.r8.d[q];
-      }
-      // the cell gradients are linear in the face averages 0.5 (P[nbr] + P[g])
-      const double sgn[6] = {-1.0, 1.0, -1.0, 1.0, -1.0, 1.0};
-      for (int q = 0; q < 5; ++q) {
-        double gc = 0.0;
-        for (int m = 0; m < 6; ++m) {
-          double s = 0.0;
-          for (int e = 0; e < 3; ++e) s += w[3 * q + e] * fa[m][e];
-          s *= 0.5 * sgn[m] * ivol;
-          gc += s;
-          aadd(&a.gpv[gv[q] * n + nbr[m]], s);
-        }
-        gp[gv[q]] += gc;
-      }
-      gp[7] += w[15]; gp[8] += w[16];
-      gd[GD_RHO] += w[17]; gd[GD_VIS] += w[18]; gd[GD_MUT] += w[19];
-    }
-    // ---- dual-time source: res -= (nsteady bb Q(pv, dv) - history) vol / dt_phy
-    if (c.nsteady >= 1) {
-      const double bb = (c.nsteady == 1) ? 1.0 : 0.75;
-      const double cst = (double)c.nsteady * bb * vol / c.dt_phy;
-      double mu_[NPVM];
-      for (int v = 0; v < NPVM; ++v) mu_[v] = -cst * lam[v];
-      const double r = dv[0], h = dv[1], u1 = pv2[1], u2 = pv2[2], u3 = pv2[3];
-      double grho = mu_[0] + mu_[1] * u1 + mu_[2] * u2 + mu_[3] * u3 + mu_[4] * (h + 0.5 * (u1 * u1 + u2 * u2 + u3 * u3));
-      for (int v = 5; v < npv; ++v) { grho += mu_[v] * pv2[v]; gp[v] += mu_[v] * r; }
-      gp[1] += mu_[1] * r + mu_[4] * r * u1;
-      gp[2] += mu_[2] * r + mu_[4] * r * u2;
-      gp[3] += mu_[3] * r + mu_[4] * r * u3;
-      gp[0] -= mu_[4];
-      gd[GD_RHO] += grho;
-      gd[GD_H] += mu_[4] * r;
-    }
-    // ---- gravity: res(2:4) += rho vol a, res(5) += rho vol (a . u)
-    if (c.gravity) {
-      double ga[3];
-      gravity_at(d.grav, bc_time(d, c), ga);
-      const double au = ga[0] * pv2[1] + ga[1] * pv2[2] + ga[2] * pv2[3];
-      gd[GD_RHO] += vol * (lam[1] * ga[0] + lam[2] * ga[1] + lam[3] * ga[2] + lam[4] * au);
-      for (int e = 0; e < 3; ++e) gp[1 + e] += lam[4] * dv[0] * vol * ga[e];
-    }
-    for (int v = 0; v < npv; ++v) aadd(&a.gpv[v * n + g], gp[v]);
-    for (int m = 0; m < NGD; ++m) aadd(&a.gdt[m * n + g], gd[m]);
-  }
-  for (int q = 0; q < 3; ++q) {
-    double s = wp[q];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) aadd(&a.gpar[q], s);
-  }
-}
 
 // ------------------------------------------------------------------ boundary program
 // One ghost operation of k_ghost reversed.  Its destination's gradient is taken and
@@ -384,30 +257,6 @@ __global__ void k_adj_ghost(DevPtr d, Par c, AdjPtr a, const GhostOp* __restrict
   if ((threadIdx.x & 31) == 0) aadd(&a.gpar[0], wu);
 }
 
-// ------------------------------------------------------------------ interior EOS
-// dv and tv(1:2) of an interior cell are its EOS: their gradient goes to (p, T, y1, y2)
-__global__ void k_adj_eos(DevPtr d, Par c, AdjPtr a) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= d.nint) return;
-  const int b = find_block_interior(d.blk, d.nblk, t);
-  int i, j, k;
-  const long long g = interior_cell(d.blk[b], t - d.blk[b].int_off, i, j, k);
-  const long long n = d.ncell;
-  double gd[NGD];
-  bool any = false;
-  for (int m = 0; m < NGD; ++m) {
-    gd[m] = (m == GD_MUT) ? 0.0 : a.gdt[m * n + g];
-    any = any || gd[m] != 0.0;
-  }
-  if (!any) return;
-  double ge[4];
-  eos_chain(c, d.pv[g] + c.pref, d.pv[4 * n + g], d.pv[5 * n + g], d.pv[6 * n + g], gd, ge);
-  a.gpv[g] += ge[0];
-  a.gpv[4 * n + g] += ge[1];
-  a.gpv[5 * n + g] += ge[2];
-  a.gpv[6 * n + g] += ge[3];
-}
-
 // ------------------------------------------------------------------ host side
 namespace {
 inline unsigned adj_blocks(long long n, int T) { return (unsigned)((n + T - 1) / T); }
@@ -423,6 +272,14 @@ int adjoint_buffers(Engine& E) {
       return CFD3D_ERR_NOMEM;
     }
   }
+  // the face kernels' states and scratch planes: the FP64 form's own, else one direction's
+  if (E.par.mixed && !E.adj_fi && E.par.nmuscl > 0) {
+    const size_t nfs = (E.par.nmuscl == 2) ? 5 : 1;
+    if (cudaMalloc(&E.adj_fi, n * npv * 3 * 8) != cudaSuccess || cudaMalloc(&E.adj_fsc, n * npv * nfs * 8) != cudaSuccess) {
+      E.err = "device allocation failed (adjoint buffers)";
+      return CFD3D_ERR_NOMEM;
+    }
+  }
   cudaMemsetAsync(E.adj_lam, 0, n * npv * 8, E.st);
   cudaMemsetAsync(E.adj_gpv, 0, n * npv * 8, E.st);
   cudaMemsetAsync(E.adj_gdt, 0, n * NGD * 8, E.st);
@@ -432,7 +289,20 @@ int adjoint_buffers(Engine& E) {
 
 void adjoint_free(Engine& E) {
   cudaFree(E.adj_lam); cudaFree(E.adj_gpv); cudaFree(E.adj_gdt); cudaFree(E.adj_gpar);
-  E.adj_lam = E.adj_gpv = E.adj_gdt = E.adj_gpar = nullptr;
+  cudaFree(E.adj_fi); cudaFree(E.adj_fsc);
+  E.adj_lam = E.adj_gpv = E.adj_gdt = E.adj_gpar = E.adj_fi = E.adj_fsc = nullptr;
+}
+
+// the engine's device pointers with the face reconstruction's buffers
+static DevPtr adj_dev(const Engine& E) {
+  DevPtr d = E.d;
+  if (E.par.mixed) {
+    d.fi = E.adj_fi;
+    d.fsc = E.adj_fsc;
+    d.nfs = (E.par.nmuscl == 2) ? 5 : (E.par.nmuscl > 0 ? 1 : 0);
+    d.fslots = 1;
+  }
+  return d;
 }
 
 // the reverse pass; the cotangent is in adj_lam and the ghost cells hold the values of the
@@ -442,11 +312,12 @@ int adjoint_launch(Engine& E) {
   const Par& c = E.par;
   cudaStream_t s = E.st;
   const AdjPtr a{E.adj_lam, E.adj_gpv, E.adj_gdt, E.adj_gpar};
-  launch_adj_face(E, a, s);
-  k_adj_cell<<<adj_blocks(E.nint, 64), 64, 0, s>>>(d, c, a);
+  launch_adj_face(E, adj_dev(E), a, s);
+  if (c.ncav <= 1 && c.ides == 0) launch_adj_cell_plain(E, a, s);
+  else launch_adj_cell(E, a, s);
   for (int p = 2; p >= 0; --p)
     if (E.nops[p]) k_adj_ghost<<<adj_blocks(E.nops[p], 64), 64, 0, s>>>(d, c, a, E.d_ops[p], E.nops[p]);
-  k_adj_eos<<<adj_blocks(E.nint, 64), 64, 0, s>>>(d, c, a);
+  launch_adj_eos(E, a, s);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { E.err = std::string("adjoint launch: ") + cudaGetErrorString(e); return CFD3D_ERR_CUDA; }
   return CFD3D_OK;

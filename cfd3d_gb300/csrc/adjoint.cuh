@@ -55,7 +55,7 @@ static __device__ __noinline__ void eos_chain(const Par& c, double p, double t, 
 // Local Jacobians are taken DC seed directions at a time (a few passes of the same code
 // on Dual<DC>), which keeps the per-thread dual arrays small.
 constexpr int DC = 8;
-using DD = Dual<DC>;
+using DD = Dual<DC, 1>;   // (rolled loops: these kernels hold dozens of duals)
 __device__ __forceinline__ DD seed(double v, int i, int k0) {
   DD r(v);
   if (i >= k0 && i < k0 + DC) r.d[i - k0] = 1.0;
@@ -85,6 +85,36 @@ __device__ __forceinline__ void clip_flags(const Par& c, const double* c9, const
   }
 }
 
+// the dual-time and gravity sources of one cell reversed: gradients added to gp (pv) and gd
+__device__ __forceinline__ void cell_sources_back(const DevPtr& d, const Par& c, const double* lam, const double* pv2,
+                                                  const double* dv, double vol, double* gp, double* gd) {
+  const int npv = c.npv;
+  // ---- dual-time source: res -= (nsteady bb Q(pv, dv) - history) vol / dt_phy
+  if (c.nsteady >= 1) {
+    const double bb = (c.nsteady == 1) ? 1.0 : 0.75;
+    const double cst = (double)c.nsteady * bb * vol / c.dt_phy;
+    double mu_[NPVM];
+    for (int v = 0; v < NPVM; ++v) mu_[v] = -cst * lam[v];
+    const double r = dv[0], h = dv[1], u1 = pv2[1], u2 = pv2[2], u3 = pv2[3];
+    double grho = mu_[0] + mu_[1] * u1 + mu_[2] * u2 + mu_[3] * u3 + mu_[4] * (h + 0.5 * (u1 * u1 + u2 * u2 + u3 * u3));
+    for (int v = 5; v < npv; ++v) { grho += mu_[v] * pv2[v]; gp[v] += mu_[v] * r; }
+    gp[1] += mu_[1] * r + mu_[4] * r * u1;
+    gp[2] += mu_[2] * r + mu_[4] * r * u2;
+    gp[3] += mu_[3] * r + mu_[4] * r * u3;
+    gp[0] -= mu_[4];
+    gd[GD_RHO] += grho;
+    gd[GD_H] += mu_[4] * r;
+  }
+  // ---- gravity: res(2:4) += rho vol a, res(5) += rho vol (a . u)
+  if (c.gravity) {
+    double ga[3];
+    gravity_at(d.grav, bc_time(d, c), ga);
+    const double au = ga[0] * pv2[1] + ga[1] * pv2[2] + ga[2] * pv2[3];
+    gd[GD_RHO] += vol * (lam[1] * ga[0] + lam[2] * ga[1] + lam[3] * ga[2] + lam[4] * au);
+    for (int e = 0; e < 3; ++e) gp[1 + e] += lam[4] * dv[0] * vol * ga[e];
+  }
+}
+
 // coefficients of the face-gradient stencil (face_gradient): d/dx_l of the normal
 // difference, the two transverse sums, and the face average
 __device__ __forceinline__ void grad_coeffs(int l, double& cn, double& ce, double& ct, double& cc) {
@@ -96,11 +126,14 @@ __device__ __forceinline__ void grad_coeffs(int l, double& cn, double& ce, doubl
   cc = (l == 8 || l == 9) ? 0.5 : 0.0;
 }
 
-// the stencil cells that MUSCL reads (MLP reads all 38)
-static __constant__ int kMusclCells[6] = {8, 9, 22, 31, 36, 37};
-
-
-// the face VJP, one launch per direction (adjoint_face.cu)
-void launch_adj_face(const Engine& E, const AdjPtr& a, cudaStream_t s);
+// the face VJP (adjoint_face.cu); d: the engine's, with the reconstruction's scratch planes
+void launch_adj_face(const Engine& E, const DevPtr& d, const AdjPtr& a, cudaStream_t s);
+// the cell sources without DES lengths and with Merkle's cavitation or none, and the interior
+// cells' dv / tv gradient through their EOS (adjoint_face.cu)
+void launch_adj_cell_plain(const Engine& E, const AdjPtr& a, cudaStream_t s);
+// Roe-M's and AUSMPW+'s flux, and the cell sources of any model, by duals (adjoint_duals.cu)
+void launch_adj_flux_duals(const Engine& E, const DevPtr& d, const AdjPtr& a, int dir, long long nf, cudaStream_t s);
+void launch_adj_cell(const Engine& E, const AdjPtr& a, cudaStream_t s);
+void launch_adj_eos(const Engine& E, const AdjPtr& a, cudaStream_t s);
 
 }  // namespace cfd

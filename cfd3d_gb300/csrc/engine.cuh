@@ -247,6 +247,7 @@ struct Engine {
   // discrete adjoint (allocated by the first cfd3d_residual_vjp): padded cotangent and
   // gradients, and the three parameter gradients
   double *adj_lam = nullptr, *adj_gpv = nullptr, *adj_gdt = nullptr, *adj_gpar = nullptr;
+  double *adj_fi = nullptr, *adj_fsc = nullptr;   // mixed form: its face states and scratch planes
 };
 
 // ------------------------------------------------------------------ index helpers

@@ -20,62 +20,11 @@
 // variable) the stage took 13.9 ms on 128x64x64 cells (cavitating, MLP, AUSM+-up) and
 // 0.70 ms on 64x32x32 (Euler, TVD, Roe).
 #include <algorithm>
-#include "engine.cuh"
+#include "faces64.cuh"
 
 namespace cfd {
 
-// the faces (EXT = 0) or the cells -1 .. +1 around them along the normal (EXT = 3) of direction
-// dir: the cell of flat index t, block-major, then (k, j, i) of the (left) cell
-struct DirCell {
-  long long g, sn, s1, s2;   // cell, normal and transverse strides
-  int b;
-};
-template <int EXT>
-__device__ __forceinline__ bool dir_cell(const DevPtr& d, int dir, long long t, DirCell& o) {
-  const BlockGeom* blk = d.blk;
-  int b = 0;
-  while (b + 1 < d.nblk && t >= (EXT ? blk[b + 1].plane_off[dir] : blk[b + 1].face_off[dir])) ++b;
-  const BlockGeom& B = blk[b];
-  const long long loc = t - (EXT ? B.plane_off[dir] : B.face_off[dir]);
-  const int fi = B.imax - 1 + (dir == 0 ? 1 + EXT : 0), fj = B.jmax - 1 + (dir == 1 ? 1 + EXT : 0);
-  const int fk = B.kmax - 1 + (dir == 2 ? 1 + EXT : 0);
-  if (loc >= (long long)fi * fj * fk) return false;
-  const int first = EXT ? 0 : 1;   // the first left cell, less one with EXT
-  const int i = (int)(loc % fi) + (dir == 0 ? first : 2);
-  const long long r = loc / fi;
-  const int j = (int)(r % fj) + (dir == 1 ? first : 2);
-  const int k = (int)(r / fj) + (dir == 2 ? first : 2);
-  const long long sj = B.ni, sk = (long long)B.ni * B.nj;
-  o.b = b;
-  o.g = B.off + (i + 1) + sj * (j + 1) + sk * (k + 1);
-  if (dir == 0) { o.sn = 1; o.s1 = sj; o.s2 = sk; }
-  else if (dir == 1) { o.sn = sj; o.s1 = sk; o.s2 = 1; }
-  else { o.sn = sk; o.s1 = 1; o.s2 = sj; }
-  return true;
-}
-
 // ------------------------------------------------------------------ reconstruction
-// A double's order-preserving integer key (and back: the map is its own inverse): minima
-// and maxima of keys run on the integer pipe.  -0 orders below +0; a NaN orders beyond the
-// infinities.
-__device__ __forceinline__ long long okey(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
-__device__ __forceinline__ double okey_value(long long k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
-}
-// minima and maxima of numbers (no NaN) by their keys
-__device__ __forceinline__ double kmin(double a, double b) { return okey(b) < okey(a) ? b : a; }
-__device__ __forceinline__ double kmax(double a, double b) { return okey(b) > okey(a) ? b : a; }
-__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
-
-// scratch planes of one direction slot and variable
-enum { FS_MN = 0, FS_MX, FS_DEN, FS_IDQ, FS_R, NFS };
-__device__ __forceinline__ double* fs_plane(const DevPtr& d, int slot, int npv, int v, int q) {
-  return d.fsc + ((long long)(slot * npv + v) * d.nfs + (d.nfs == 1 ? 0 : q)) * d.ncell;
-}
-
 // |num / den| of MLP's transverse ratios; a zero numerator needs no division (and would take
 // the quotient's slow path)
 __device__ __forceinline__ double abs_ratio(double num, double den) {
@@ -395,23 +344,33 @@ __global__ void __launch_bounds__(256) k_visc64(DevPtr d, Par c, int dir0) {
     if (v < npv) fvp[v * n + g] = fv[v];
 }
 
+// the threads that cover the faces, or the planes, of the directions of one launch
+static long long most(const long long* n, int dir, int slots) {
+  long long m = 0;
+  for (int q = dir; q < dir + slots; ++q) m = std::max(m, n[q]);
+  return m;
+}
+static unsigned nb_of(long long n, int t) { return (unsigned)((n + t - 1) / t); }
+
+void launch_recon64(const Engine& E, const DevPtr& d, int dir, cudaStream_t s) {
+  const int T = E.tpb_face;
+  const Par& c = E.par;
+  const unsigned z = (unsigned)d.fslots, y = (unsigned)c.npv;
+  if (c.nmuscl == 2) k_plane64<<<dim3(nb_of(most(E.nplane, dir, d.fslots), T), y, z), T, 0, s>>>(d, c, dir);
+  if (c.nmuscl > 0) k_recon64<<<dim3(nb_of(most(E.nface, dir, d.fslots), T), y, z), T, 0, s>>>(d, c, dir);
+}
+
 // Three directions per launch where the scratch planes hold them (small cases, whose launches
 // would not fill the GPU one direction at a time), else one direction after the other.
 void launch_face_flux(const Engine& E, cudaStream_t s) {
   const int T = E.tpb_face;
   const Par& c = E.par;
-  auto nb = [](long long n, int t) { return (unsigned)((n + t - 1) / t); };
+  const unsigned z = (unsigned)E.d.fslots;
   for (int dir = 0; dir < 3; dir += E.d.fslots) {
-    long long nf = 0, np = 0;
-    for (int q = dir; q < dir + E.d.fslots; ++q) {
-      nf = std::max(nf, E.nface[q]);
-      np = std::max(np, E.nplane[q]);
-    }
-    const unsigned z = (unsigned)E.d.fslots, y = (unsigned)c.npv;
-    if (c.nmuscl == 2) k_plane64<<<dim3(nb(np, T), y, z), T, 0, s>>>(E.d, c, dir);
-    if (c.nmuscl > 0) k_recon64<<<dim3(nb(nf, T), y, z), T, 0, s>>>(E.d, c, dir);
-    k_flux64<<<dim3(nb(nf, F64_FACES), 1, z), 3 * F64_FACES, 0, s>>>(E.d, c, dir);
-    if (c.iturb != -3) k_visc64<<<dim3(nb(nf, T), 1, z), T, 0, s>>>(E.d, c, dir);
+    const long long nf = most(E.nface, dir, E.d.fslots);
+    launch_recon64(E, E.d, dir, s);
+    k_flux64<<<dim3(nb_of(nf, F64_FACES), 1, z), 3 * F64_FACES, 0, s>>>(E.d, c, dir);
+    if (c.iturb != -3) k_visc64<<<dim3(nb_of(nf, T), 1, z), T, 0, s>>>(E.d, c, dir);
   }
 }
 
