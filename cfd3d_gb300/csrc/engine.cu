@@ -1659,7 +1659,7 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
 // iteration (kept in dqs at t by stage 1).  The residual norms measure the change over
 // the whole iteration (they are final after the last stage).
 template <bool MX, bool EX = false>
-__global__ void __launch_bounds__(128, 3) k_update(DevPtr d, Par c, int stage) {
+__global__ void __launch_bounds__(128, MX && !EX ? 8 : 3) k_update(DevPtr d, Par c, int stage) {
   // grid-stride over the interior cells: the grid is a fixed multiple of the SM count,
   // so the per-CTA partials (and the order they are summed in) do not depend on size
   const int npv = c.npv;
@@ -1734,20 +1734,21 @@ __global__ void __launch_bounds__(128, 3) k_update(DevPtr d, Par c, int stage) {
     }
     double dp = fabs(old[0] - p[0]);
     if (dp > dpmax) { dpmax = dp; dpidx = t; }   // t increases: ties keep the first cell
-    const double pe = p[0] + c.pref, te = p[4], y1 = p[5], y2 = p[6];
-    double dv[NDV], tv[3] = {0.0, 0.0, 0.0};
+    if constexpr (!MX) {   // (the mixed form's EOS follows in passes of its own: launch_eos_cells)
+      const double pe = p[0] + c.pref, te = p[4], y1 = p[5], y2 = p[6];
+      double dv[NDV], tv[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int v = 0; v < 3; ++v)
-      if (v < c.ntv) tv[v] = d.tv[v * n + g];
-    if (MX) deteos_split(c.fluid, c.with_prop, pe, te, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
-    else deteos(c.fluid, c.with_prop, pe, te, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
-    for (int v = 0; v < NDV; ++v) {
-      d.dv[v * n + g] = dv[v];
-      if (!finite_bits(dv[v])) bad = 1;
+      for (int v = 0; v < 3; ++v)
+        if (v < c.ntv) tv[v] = d.tv[v * n + g];
+      deteos(c.fluid, c.with_prop, pe, te, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
+      for (int v = 0; v < NDV; ++v) {
+        d.dv[v * n + g] = dv[v];
+        if (!finite_bits(dv[v])) bad = 1;
+      }
+#pragma unroll
+      for (int v = 0; v < 3; ++v)
+        if (v < c.ntv) d.tv[v * n + g] = tv[v];
     }
-#pragma unroll
-    for (int v = 0; v < 3; ++v)
-      if (v < c.ntv) d.tv[v * n + g] = tv[v];
   }
   if (bad) atomicExch(&d.sc->nonfinite, 1);
   // per-CTA partial sums (deterministic order: warp shuffles then warps in order)
@@ -2052,7 +2053,7 @@ int face_rhs_launches(const Engine& E) {
   if (!c.mixed) return face_flux_launches(E) + 1;
   const int nb = (int)E.blk.size();
   const int ng = std::min(std::max(E.pipe_groups, 1), std::min(nb, Engine::MAX_PIPE));
-  return ng * (8 + (c.nmuscl > 0 ? 2 : 0) + (c.iturb != -3 ? 3 : 0));
+  return ng * (8 + (c.nmuscl > 0 ? 2 : 0) + (c.nmuscl > 0 && c.fluid != 1 ? 9 : 0) + (c.iturb != -3 ? 3 : 0));
 }
 
 // The boundary program -- the total-pressure pools, then faces + halos, edges, corners -- and,
@@ -2122,8 +2123,13 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
         n += face_rhs_launches(E);
       }
       if (m == nstage) { stage(5); stage(6); }
-      if (c.mixed) k_update<true, true><<<E.red_grid, T, 0, s>>>(d, c, m);
-      else k_update<false, true><<<E.red_grid, T, 0, s>>>(d, c, m);
+      if (c.mixed) {
+        k_update<true, true><<<E.red_grid, T, 0, s>>>(d, c, m);
+        launch_eos_cells(E, s, nullptr, nullptr, E.nint);
+        n += eos_cells_launches(E);
+      } else {
+        k_update<false, true><<<E.red_grid, T, 0, s>>>(d, c, m);
+      }
       ++n;
       if (m == nstage) stage(7);
       if (c.iturb >= -1) {
@@ -2170,8 +2176,13 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
     }
   }
   stage(6);
-  if (c.mixed) k_update<true><<<E.red_grid, T, 0, s>>>(d, c, 0);
-  else k_update<false><<<E.red_grid, T, 0, s>>>(d, c, 0);
+  if (c.mixed) {
+    k_update<true><<<E.red_grid, T, 0, s>>>(d, c, 0);
+    launch_eos_cells(E, s, nullptr, nullptr, E.nint);
+    n += eos_cells_launches(E);
+  } else {
+    k_update<false><<<E.red_grid, T, 0, s>>>(d, c, 0);
+  }
   ++n;
   stage(7);
   if (c.iturb >= -1) {
@@ -2503,6 +2514,13 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   if (c.mixed)
     ok = ok && allocf(E.d.pvf, c.npv) && allocf(E.d.fi32, 3 * c.npv) && allocf(E.d.fv32, (c.iturb == -3) ? 1 : 3 * c.npv) &&
          allocf(E.d.frec, 2 * 12) && allocf(E.d.lqf, NLQ);
+  if (c.mixed) {
+    // lists of face states (two per face of a direction) and of cells
+    const long long most = std::max({2 * E.nface[0], 2 * E.nface[1], 2 * E.nface[2], E.nint});
+    E.d.mxcap = (int)std::min<long long>(most, 0x7fffffffll);
+    ok = ok && cudaMalloc(&E.d.mxl, (size_t)E.d.mxcap * MX_KINDS * sizeof(int)) == cudaSuccess &&
+         cudaMalloc(&E.d.mxn, MXN * sizeof(int)) == cudaSuccess;
+  }
   else {
     // the face reconstruction's scratch: all three directions at once up to 128 MB of it.  A
     // launch per direction leaves three partial last waves (the face stage of 128x64x64 cells
@@ -2686,6 +2704,8 @@ void cfd3d_destroy(cfd3d_handle* h) {
   cudaFree(E.d.tickets);
   cudaFree(E.d_chunk_t0);
   cudaFree(E.d_tiles);
+  cudaFree(E.d.mxl);
+  cudaFree(E.d.mxn);
   cudaFree(E.d.trf);
   cudaFree(E.d.tq);
   cudaFree(E.d.tyf);

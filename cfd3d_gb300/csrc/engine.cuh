@@ -182,12 +182,37 @@ struct DevPtr {
   // sweep); done flags per tile
   int ntile;
   long long nslot;
+  // mixed form: index lists of the states that need further IF97 sums, by kind (MX_*), mxcap
+  // entries each, and their counters: three directions' faces, then the cells
+  int* mxl;
+  int* mxn;
+  int mxcap;
   const TileDesc* tiles;
   float* trf;
   float* tq;
   float *tyf, *tyb;
   float* tin;
 };
+
+// kinds of the mixed form's lists: liquid alone, with metastable, with stable vapour
+enum { MX_LIQ = 0, MX_META, MX_STABLE, MX_KINDS };
+constexpr int MXN_FACE = 3 * MX_KINDS, MXN = MXN_FACE + MX_KINDS;
+
+// item appended to the list of its kind: one atomic per kind of the lanes that call together.
+// (The order of a list is arbitrary; every entry's result goes to its own place.)
+__device__ __forceinline__ void list_add(const DevPtr& d, int* cnt, int kind, int item) {
+  const unsigned same = __match_any_sync(__activemask(), kind);
+  const int lane = threadIdx.x & 31, lead = __ffs(same) - 1;
+  int base = 0;
+  if (lane == lead) base = atomicAdd(cnt + kind, __popc(same));
+  base = __shfl_sync(same, base, lead) + __popc(same & ((1u << lane) - 1u));
+  if (base < d.mxcap) d.mxl[(long long)kind * d.mxcap + base] = item;
+}
+// a kind's list and its length
+__device__ __forceinline__ int list_of(const DevPtr& d, const int* cnt, int kind, const int*& list) {
+  list = d.mxl + (long long)kind * d.mxcap;
+  return min(cnt[kind], d.mxcap);
+}
 
 // sweep record planes: what the sweeps read of a cell, as itself and as a neighbour
 enum {
@@ -343,6 +368,10 @@ constexpr int SW_CH = 32;
 void launch_face_flux(const Engine& E, cudaStream_t s);
 int face_flux_launches(const Engine& E);
 void launch_face_flux_mixed(const Engine& E, cudaStream_t s, int b0, int b1);
+// the mixed form's cell EOS (eos_mixed.cu): dv and tv(1:2) of every interior cell, or of the
+// cells of a list, from pv
+void launch_eos_cells(const Engine& E, cudaStream_t s, const int* list, const int* count, long long most);
+int eos_cells_launches(const Engine& E);
 // discrete adjoint (adjoint.cu): buffers (allocated once, zeroed per call), the reverse
 // pass, and release
 int adjoint_buffers(Engine& E);

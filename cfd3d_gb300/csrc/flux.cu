@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(3 * F64_FACES) k_flux64(DevPtr d, Par c, int d
       deteos_simple(c.fluid, x[0] + c.pref, x[4], x[5], x[6], dv, &d.sc->snd2_fallbacks, x[5] != 0.0);
       rho = dv[0]; h = dv[1]; c2 = dv[5];
     } else {
-      eos_rho_h<false>(c.fluid, x[0] + c.pref, x[4], x[5], x[6], rho, h);
+      eos_rho_h(c.fluid, x[0] + c.pref, x[4], x[5], x[6], rho, h);
     }
     s_eos[role][0][q] = rho; s_eos[role][1][q] = h; s_eos[role][2][q] = c2;
   }

@@ -234,6 +234,49 @@ __global__ void __launch_bounds__(128) k_muscl_march(DevPtr d, Par c, long long 
   }
 }
 
+// A face state that needs the IF97 sums (side 0 left, 1 right of the face at g): listed by the
+// phases it needs, for k_face_eos; stiffened water, whose EOS is a few products, at once.
+__device__ __forceinline__ void face_eos_later(const DevPtr& d, const Par& c, int* cnt, int g, int side, const float* x,
+                                               float& rdev, float& hdev) {
+  const double p = c.pref + (double)x[0], t = c.tref + (double)x[4];
+  if (c.fluid == 1) {
+    double rho, h;
+    eos_rho_h(1, p, t, x[5], x[6], rho, h);
+    rdev = (float)(rho - c.rhoref);
+    hdev = (float)(h - c.href);
+    return;
+  }
+  const int kind = (x[5] == 0.0f) ? MX_LIQ : (above_psat(p, t) ? MX_META : MX_STABLE);
+  list_add(d, cnt, kind, 2 * g + side);
+}
+
+// rho - rhoref and h - href of the listed face states by the df64 IF97 sums, one launch per
+// kind: liquid alone, with metastable vapour, with stable vapour.  In the reconstruction
+// kernel these sums -- 1500 to 3500 instructions of straight code per state -- ran in warps
+// where a few lanes needed them, once for the lanes without and once for those with vapour,
+// and evicted one another from the instruction cache (no-instruction stalls half of all, the
+// three reconstruction kernels 3.8 ms on the 3.0 M-cell batched case); listed, the lanes of a warp all need
+// the same sums and each kernel's code stays in the cache.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_face_eos(DevPtr d, Par c, const int* cnt) {
+  const int* L;
+  const int m = list_of(d, cnt, KIND, L);
+  const long long n = d.ncell;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
+    const int it = L[q], side = it & 1;
+    const long long g = (unsigned)it >> 1;
+    float* F = d.frec + (long long)(side * FREC_SIDE) * n + g;
+    const double t = c.tref + (double)F[4 * n];
+    const df64 P(c.pref + (double)F[0]), T(t);
+    double il, hl, ig, iv = 0.0, hv = 0.0, rho, h;
+    liquid_inv_df64(P, T, &il, &hl, &ig);
+    if constexpr (KIND != MX_LIQ) vapour_inv_df64(P, T, KIND == MX_META, &iv, &hv);
+    mix_face_mx(t, F[5 * n], F[6 * n], il, hl, iv, hv, ig, rho, h);
+    F[NPVM * n] = (float)(rho - c.rhoref);
+    F[(NPVM + 1) * n] = (float)(h - c.href);
+  }
+}
+
 // Second order (nmuscl > 0): with MARCH the face states come from k_muscl_march (frec,
 // before the clips), otherwise from the face's 38-cell stencil; first order: the face states
 // are the cells' own.  (The per-variable loops run over the compile-time bound, guarded by
@@ -241,7 +284,7 @@ __global__ void __launch_bounds__(128) k_muscl_march(DevPtr d, Par c, long long 
 template <int DIR, bool MARCH = false>
 // (the column-fed instantiations at 4 CTAs of 256 threads per SM, the stencil one at 3:
 // 0.55 and 0.65 ms faster than at the compiler's choice of 2)
-__global__ void __launch_bounds__(256, MARCH ? 4 : 3) k_recon_mx(DevPtr d, Par c, long long t0, long long t1) {
+__global__ void __launch_bounds__(256, MARCH ? 4 : 3) k_recon_mx(DevPtr d, Par c, long long t0, long long t1, int* cnt) {
   const long long t = t0 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= t1) return;
   const FaceIdx f = face_of<DIR>(d, t);
@@ -286,18 +329,11 @@ __global__ void __launch_bounds__(256, MARCH ? 4 : 3) k_recon_mx(DevPtr d, Par c
     // direction, two in every warp's row of faces, would send their warps through the sums.)
     const float bl0 = f.lin ? c9[0] : c10[0], bl4 = f.lin ? c9[4] : c10[4], bl6 = f.lin ? c9[6] : c10[6];
     const float br0 = f.rin ? c10[0] : c9[0], br4 = f.rin ? c10[4] : c9[4], br6 = f.rin ? c10[6] : c9[6];
-    if (!(gl[5] == 0.0f && liquid_expand(d, c, f.lin ? g : gr, gl, bl0, bl4, bl6, rdl, hdl))) {
-      double rho, h;
-      eos_rho_h<true>(c.fluid, c.pref + (double)gl[0], c.tref + (double)gl[4], gl[5], gl[6], rho, h);
-      rdl = (float)(rho - c.rhoref);
-      hdl = (float)(h - c.href);
-    }
-    if (!(gR[5] == 0.0f && liquid_expand(d, c, f.rin ? gr : g, gR, br0, br4, br6, rdr, hdr))) {
-      double rho, h;
-      eos_rho_h<true>(c.fluid, c.pref + (double)gR[0], c.tref + (double)gR[4], gR[5], gR[6], rho, h);
-      rdr = (float)(rho - c.rhoref);
-      hdr = (float)(h - c.href);
-    }
+    rdl = hdl = rdr = hdr = 0.0f;
+    if (!(gl[5] == 0.0f && liquid_expand(d, c, f.lin ? g : gr, gl, bl0, bl4, bl6, rdl, hdl)))
+      face_eos_later(d, c, cnt, (int)g, 0, gl, rdl, hdl);
+    if (!(gR[5] == 0.0f && liquid_expand(d, c, f.rin ? gr : g, gR, br0, br4, br6, rdr, hdr)))
+      face_eos_later(d, c, cnt, (int)g, 1, gR, rdr, hdr);
     if (c.nscheme == 2 || c.nscheme == 3) {
       cl = eos_c2_f(c.fluid, (float)c.pref + gl[0], (float)c.tref + gl[4], gl[5], gl[6], &d.sc->snd2_fallbacks);
       cr = eos_c2_f(c.fluid, (float)c.pref + gR[0], (float)c.tref + gR[4], gR[5], gR[6], &d.sc->snd2_fallbacks);
@@ -508,19 +544,33 @@ void launch_face_flux_mixed(const Engine& E, cudaStream_t s, int b0, int b1) {
   k_shadow<<<(unsigned)std::max<long long>(share, 1), 256, 0, s>>>(E.d, E.par, g0, g1);
   // the i faces from their 38-cell stencils, the j and k faces by columns (k_muscl_march)
   // under MUSCL; then the clips and the face EOS
-  const bool march = E.par.nmuscl > 0, visc = E.par.iturb != -3;
+  const bool march = E.par.nmuscl > 0, visc = E.par.iturb != -3, sums = march && E.par.fluid != 1;
   auto cols = [&](int q) { return (unsigned)(((c1[q] - c0[q]) * E.par.npv + 127) / 128); };
-  k_recon_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0]);
+  // (the groups of the pipeline follow one another on s, so they can share lists and counters)
+  int* cnt = E.d.mxn;
+  if (sums) cudaMemsetAsync(cnt, 0, MXN_FACE * sizeof(int), s);
+  auto face_eos = [&](int q) {
+    if (!sums) return;
+    // grids that fill the GPU at most, and no more than every state listed needs
+    const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>((2 * (f1[q] - f0[q]) + 255) / 256, 4ll * nsm));
+    k_face_eos<MX_LIQ><<<g, 256, 0, s>>>(E.d, E.par, cnt + 3 * q);
+    k_face_eos<MX_META><<<g, 256, 0, s>>>(E.d, E.par, cnt + 3 * q);
+    k_face_eos<MX_STABLE><<<g, 256, 0, s>>>(E.d, E.par, cnt + 3 * q);
+  };
+  k_recon_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0], cnt);
+  face_eos(0);
   k_flux_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0]);
   if (visc) k_visc_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0]);
   if (march) k_muscl_march<1><<<cols(1), 128, 0, s>>>(E.d, E.par, c0[1], c1[1]);
-  if (march) k_recon_mx<1, true><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1]);
-  else k_recon_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1]);
+  if (march) k_recon_mx<1, true><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1], cnt + 3);
+  else k_recon_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1], cnt + 3);
+  face_eos(1);
   k_flux_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1]);
   if (visc) k_visc_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1]);
   if (march) k_muscl_march<2><<<cols(2), 128, 0, s>>>(E.d, E.par, c0[2], c1[2]);
-  if (march) k_recon_mx<2, true><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2]);
-  else k_recon_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2]);
+  if (march) k_recon_mx<2, true><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2], cnt + 6);
+  else k_recon_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2], cnt + 6);
+  face_eos(2);
   k_flux_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2]);
   if (visc) k_visc_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2]);
 }

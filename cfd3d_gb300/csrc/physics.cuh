@@ -233,25 +233,31 @@ __device__ __forceinline__ void if97_r2_rh(df64 P, df64 T, bool meta, df64& gp, 
   gt = dadd(iy, ry);
 }
 
-// The mixed form's face-state EOS: 1/rho and h of the liquid (and of the vapour when VAP)
-// from the df64 sums, the reciprocal also taken in df64 (on the FP32 pipes: an FP64
-// division costs a GB300 far more), and the gas's 1/rho = t / (p r1) from the same df64
-// splits of p and t (each split costs FP64-pipe conversions)
-template <bool VAP>
-__device__ __noinline__ void iapws_inv_df64(double p, double t, bool meta, double* il, double* hl, double* iv,
-                                            double* hv, double* ig) {
+// The mixed form's phases: 1/rho and h of the liquid, and of the vapour, from the df64 sums,
+// the reciprocal also taken in df64 (on the FP32 pipes: an FP64 division costs a GB300 far
+// more), and the gas's 1/rho = t / (p r1) from the same df64 splits of p and t (each split
+// costs FP64-pipe conversions).  Two functions: a warp whose states carry vapour in part runs
+// the liquid's sums once.
+__device__ __forceinline__ void liquid_inv_df64(df64 P, df64 T, double* il, double* hl, double* ig) {
   // 1/rho = gamma_pi / (c tau) = gamma_pi T / (c T* ): no division beyond tau's
-  const df64 P(p), T(t);
   *ig = (double)(T / (P * df64(0.00348383500557)));
   df64 gp, gt, tau;
   if97_r1_rh(P, T, gp, gt, tau);
   *il = (double)(gp * T * df64(1.0 / ((double)25.841246054191803727f * 1386.0)));
   *hl = (double)(df64(639675.036) * gt);
-  if constexpr (VAP) {
-    if97_r2_rh(P, T, meta, gp, gt, tau);
-    *iv = (double)(gp * T * df64(1.0 / (4.01245401527075799 * 540.0)));
-    *hv = (double)(df64(249224.04) * gt);
-  }
+}
+__device__ __forceinline__ void vapour_inv_df64(df64 P, df64 T, bool meta, double* iv, double* hv) {
+  df64 gp, gt, tau;
+  if97_r2_rh(P, T, meta, gp, gt, tau);
+  *iv = (double)(gp * T * df64(1.0 / (4.01245401527075799 * 540.0)));
+  *hv = (double)(df64(249224.04) * gt);
+}
+// (out of line for the callers that are not split by phase)
+static __device__ __noinline__ void liquid_inv_call(double p, double t, double* il, double* hl, double* ig) {
+  liquid_inv_df64(df64(p), df64(t), il, hl, ig);
+}
+static __device__ __noinline__ void vapour_inv_call(double p, double t, bool meta, double* iv, double* hv) {
+  vapour_inv_df64(df64(p), df64(t), meta, iv, hv);
 }
 
 // Phase properties of liquid, vapour and gas in FP64, with their reciprocal densities ir[3].
@@ -344,8 +350,9 @@ __device__ __forceinline__ void mixture_split(double il, double hl, double iv, d
   const float il2 = fil * fil, iv2 = fiv * fiv, ig2 = fig * fig;
   const float d6 = r2 * (fyl * il2 * lf.drdp + fy1 * iv2 * vf.drdp + fy2 * ig2 * gf.drdp);
   const float d7 = r2 * (fyl * il2 * lf.drdt + fy1 * iv2 * vf.drdt + fy2 * ig2 * gf.drdt);
-  const float d10 = fyl * lf.dhdp + fy1 * vf.dhdp + fy2 * gf.dhdp;
-  const float d11 = fyl * lf.dhdt + fy1 * vf.dhdt + fy2 * gf.dhdt;
+  // (contraction spelled out: the mixture's dh/dp and dh/dT round the same in every kernel)
+  const float d10 = __fmaf_rn(fy2, gf.dhdp, __fmaf_rn(fy1, vf.dhdp, __fmul_rn(fyl, lf.dhdp)));
+  const float d11 = __fmaf_rn(fy2, gf.dhdt, __fmaf_rn(fy1, vf.dhdt, __fmul_rn(fyl, lf.dhdt)));
   dv[6] = d6; dv[7] = d7;
   dv[8] = r2 * (fil - fiv);
   dv[9] = r2 * (fil - fig);
@@ -422,18 +429,7 @@ __device__ __forceinline__ void mix_face_mx(double t, double y1, double y2, doub
   h = yl * hl + y1 * hv + y2 * (1004.64 * t);
 }
 
-template <bool MX = false>
 __device__ __forceinline__ void eos_rho_h(int fluid, double p, double t, double y1, double y2, double& rho, double& h) {
-  if constexpr (MX) {
-    if (fluid != 1) {
-      // phase reciprocals in df64
-      double il, hl, iv = 0.0, hv = 0.0, ig;
-      if (y1 != 0.0) iapws_inv_df64<true>(p, t, above_psat(p, t), &il, &hl, &iv, &hv, &ig);
-      else iapws_inv_df64<false>(p, t, false, &il, &hl, &iv, &hv, &ig);
-      mix_face_mx(t, y1, y2, il, hl, iv, hv, ig, rho, h);
-      return;
-    }
-  }
   Phase<double> l, v, g;
   double ir[3];
   phases<false>(fluid, p, t, l, v, g, ir, y1 != 0.0);
@@ -470,35 +466,20 @@ __device__ __forceinline__ void deteos(int fluid, int with_prop, double p, doubl
 // (they enter the residual: dual-time source, face states of first-order schemes), their
 // p / T derivatives and the transport properties in FP32 (they only shape the implicit
 // operator, the preconditioning speed and the FP32 viscous fluxes); mixture in FP64.
-__device__ __forceinline__ void deteos_split(int fluid, int with_prop, double p, double t, double y1, double y2,
-                                             double* dv, double* tv, unsigned long long* fb) {
-  double il, hl, iv, hv, ig;
+// deteos_split_mix: everything after the df64 sums il, hl, ig and (y1 != 0) iv, hv.
+__device__ __forceinline__ void deteos_split_mix(int with_prop, double p, double t, double y1, double y2, bool meta,
+                                                 double il, double hl, double iv, double hv, double ig, double* dv,
+                                                 double* tv, unsigned long long* fb) {
   Phase<float> lf, vf, gf;
   const float pf = (float)p, tf = (float)t;
-  if (fluid == 1) {
-    Phase<double> l, v;
-    stiffened(p, t, l);
-    ideal_gas(p, t, v);
-    il = 1.0 / l.rho; hl = l.h; iv = 1.0 / v.rho; hv = v.h;
-    ig = (double)(df64(t) / (df64(p) * df64(0.00348383500557)));   // the gas: t / (p r1)
-    lf.drdp = (float)l.drdp; lf.drdt = (float)l.drdt; lf.dhdp = (float)l.dhdp; lf.dhdt = (float)l.dhdt;
-    vf.drdp = (float)v.drdp; vf.drdt = (float)v.drdt; vf.dhdp = (float)v.dhdp; vf.dhdt = (float)v.dhdt;
-  } else {
-    // (the gas's 1/rho = t / (p r1) comes with the phases, from the same df64 splits)
-    const bool meta = above_psat(p, t);
-    iapws_l<float, true>(pf, tf, lf);
-    iapws_v_meta<float, true>(pf, tf, meta, vf);
-    if (y1 != 0.0) {
-      iapws_inv_df64<true>(p, t, meta, &il, &hl, &iv, &hv, &ig);
-    } else {
-      // without vapour the vapour's 1/rho and h enter the mixture with the factor y1 = 0:
-      // its df64 sums are skipped, and the phase's FP32 values serve the vapour density,
-      // enthalpy difference and derivatives the implicit operator and the cavitation
-      // source read
-      iapws_inv_df64<false>(p, t, meta, &il, &hl, &iv, &hv, &ig);
-      iv = (double)(1.0f / vf.rho);
-      hv = (double)vf.h;
-    }
+  iapws_l<float, true>(pf, tf, lf);
+  iapws_v_meta<float, true>(pf, tf, meta, vf);
+  if (y1 == 0.0) {
+    // without vapour the vapour's 1/rho and h enter the mixture with the factor y1 = 0: its
+    // df64 sums are skipped, and the phase's FP32 values serve the vapour density, enthalpy
+    // difference and derivatives the implicit operator and the cavitation source read
+    iv = (double)(1.0f / vf.rho);
+    hv = (double)vf.h;
   }
   ideal_gas<float>(pf, tf, gf);
   const double hg = 1004.64 * t;   // the gas's h = cp T
@@ -507,19 +488,52 @@ __device__ __forceinline__ void deteos_split(int fluid, int with_prop, double p,
     // the transport properties in FP32: they feed the FP32 viscous fluxes, the SST terms
     // and the operator's viscous eigenvalue
     float lv, lc, vv, vc;
-    if (fluid == 1) {
-      lv = stiffened_vis<float>(tf); lc = 4598.0f * lv;
-      vv = ideal_vis<float>(tf); vc = 1395.333333f * vv;
-    } else {
-      iapws_transport<float>(tf, (float)dv[2], lv, lc);
-      iapws_transport<float>(tf, (float)dv[3], vv, vc);
-    }
-    float gv = ideal_vis<float>(tf), gc = 1395.333333f * gv;
+    iapws_transport<float>(tf, (float)dv[2], lv, lc);
+    iapws_transport<float>(tf, (float)dv[3], vv, vc);
+    const float gv = ideal_vis<float>(tf), gc = 1395.333333f * gv;
     const float r0 = (float)dv[0], fyl = (float)(1.0 - y1 - y2), fy1 = (float)y1, fy2 = (float)y2;
     const float fil = (float)il, fiv = (float)iv, fig = (float)ig;
     tv[0] = r0 * (lv * fyl * fil + vv * fy1 * fiv + gv * fy2 * fig);
     tv[1] = r0 * (lc * fyl * fil + vc * fy1 * fiv + gc * fy2 * fig);
   }
+}
+
+// stiffened water and ideal vapour (fluid = 1) of the mixed form
+__device__ __forceinline__ void deteos_split_stiffened(int with_prop, double p, double t, double y1, double y2,
+                                                       double* dv, double* tv, unsigned long long* fb) {
+  Phase<float> lf, vf, gf;
+  const float pf = (float)p, tf = (float)t;
+  Phase<double> l, v;
+  stiffened(p, t, l);
+  ideal_gas(p, t, v);
+  const double il = 1.0 / l.rho, iv = 1.0 / v.rho;
+  const double ig = (double)(df64(t) / (df64(p) * df64(0.00348383500557)));   // the gas: t / (p r1)
+  lf.drdp = (float)l.drdp; lf.drdt = (float)l.drdt; lf.dhdp = (float)l.dhdp; lf.dhdt = (float)l.dhdt;
+  vf.drdp = (float)v.drdp; vf.drdt = (float)v.drdt; vf.dhdp = (float)v.dhdp; vf.dhdt = (float)v.dhdt;
+  ideal_gas<float>(pf, tf, gf);
+  mixture_split(il, l.h, iv, v.h, ig, 1004.64 * t, lf, vf, gf, y1, y2, dv, fb);
+  if (with_prop) {
+    const float lv = stiffened_vis<float>(tf), lc = 4598.0f * lv;
+    const float vv = ideal_vis<float>(tf), vc = 1395.333333f * vv;
+    const float gv = ideal_vis<float>(tf), gc = 1395.333333f * gv;
+    const float r0 = (float)dv[0], fyl = (float)(1.0 - y1 - y2), fy1 = (float)y1, fy2 = (float)y2;
+    const float fil = (float)il, fiv = (float)iv, fig = (float)ig;
+    tv[0] = r0 * (lv * fyl * fil + vv * fy1 * fiv + gv * fy2 * fig);
+    tv[1] = r0 * (lc * fyl * fil + vc * fy1 * fiv + gc * fy2 * fig);
+  }
+}
+
+__device__ __forceinline__ void deteos_split(int fluid, int with_prop, double p, double t, double y1, double y2,
+                                             double* dv, double* tv, unsigned long long* fb) {
+  if (fluid == 1) {
+    deteos_split_stiffened(with_prop, p, t, y1, y2, dv, tv, fb);
+    return;
+  }
+  double il, hl, iv = 0.0, hv = 0.0, ig;
+  const bool meta = above_psat(p, t);
+  liquid_inv_call(p, t, &il, &hl, &ig);
+  if (y1 != 0.0) vapour_inv_call(p, t, meta, &iv, &hv);
+  deteos_split_mix(with_prop, p, t, y1, y2, meta, il, hl, iv, hv, ig, dv, tv, fb);
 }
 
 // isfinite by the exponent bits (integer instructions: the FP64 pipe is the scarce one)
