@@ -1114,12 +1114,9 @@ __global__ void __launch_bounds__(256, MX ? 4 : 1) k_rhs(DevPtr d, Par c, long l
 #pragma unroll
       for (int q = 0; q < PREP_DIAG; ++q) R[(TR_DIAG + q) * TILE_SLOTS] = od[q];
     }
-    // the spectral radii only scale the implicit operator: FP32
+    // the spectral radii only scale the implicit operator: FP32 (the face vectors stay as
+    // k_record_faces wrote them)
     for (int dir = 0; dir < 3; ++dir) {
-      for (int e = 0; e < 3; ++e) {
-        R[(TR_FACEP + 3 * dir + e) * TILE_SLOTS] = fcf[6 * dir + 3 + e];   // cx2, ex2, tx2
-        R[(TR_FACEM + 3 * dir + e) * TILE_SLOTS] = fcf[6 * dir + e];       // cx1, ex1, tx1
-      }
       R[(TR_SPECP + dir) * TILE_SLOTS] = face_spectral<float>(c, fcf + 3 * (2 * dir + 1), p2f, dvf);
       R[(TR_SPECM + dir) * TILE_SLOTS] = face_spectral<float>(c, fcf + 3 * (2 * dir), p2f, dvf);
     }
@@ -1147,6 +1144,24 @@ __global__ void __launch_bounds__(256, MX ? 4 : 1) k_rhs(DevPtr d, Par c, long l
     const long long nint = d.nint, tp = d.pos[g];
     for (int q = 0; q < NREC; ++q) d.rec[q * nint + tp] = o[q];
   }
+}
+
+// the face vectors of the mixed form's tile records (once, at create: they do not change)
+__global__ void k_record_faces(DevPtr d) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= d.nint) return;
+  int b = find_block_interior(d.blk, d.nblk, t), i, j, k;
+  const BlockGeom& B = d.blk[b];
+  const long long g = interior_cell(B, t - B.int_off, i, j, k);
+  const long long n = d.ncell, st[3] = {1, B.ni, (long long)B.ni * B.nj};
+  const int planes[3] = {GM_CX, GM_EX, GM_TX};
+  float* R = d.trf + trf_at(d.pos[g], 0);
+  for (int dir = 0; dir < 3; ++dir)
+    for (int e = 0; e < 3; ++e) {
+      const float* G = d.gmf + (planes[dir] + e) * n;
+      R[(TR_FACEP + 3 * dir + e) * TILE_SLOTS] = G[g];
+      R[(TR_FACEM + 3 * dir + e) * TILE_SLOTS] = G[g - st[dir]];
+    }
 }
 
 // ------------------------------------------------------------------ LU-SGS sweeps
@@ -1687,7 +1702,7 @@ __global__ void __launch_bounds__(128, MX && !EX ? 8 : 3) k_update(DevPtr d, Par
           // an FP64 sum would add digits none of them carries
           const long long q = tq_at(pq, v);
           const float dqf = (d.tq[q] + d.tyf[q]) + d.tyb[q];
-          p[v] = old[v] + (double)dqf;
+          p[v] = old[v] + to_f64(dqf);
         } else {
           p[v] = old[v] + d.dqs[v * d.nint + pq];
         }
@@ -1716,12 +1731,12 @@ __global__ void __launch_bounds__(128, MX && !EX ? 8 : 3) k_update(DevPtr d, Par
 #pragma unroll
     for (int v = 0; v < NPVM; ++v)
       if (v < npv && !finite_bits(p[v])) bad = 1;   // checked before the clips, which would hide a NaN (fmax/fmin)
-    p[0] = fmax(-c.pref + 1.0e1, p[0]);
-    p[5] = fmin(1.0, fmax(0.0, p[5]));
-    p[6] = fmin(1.0, fmax(0.0, p[6]));
+    p[0] = max_num(-c.pref + 1.0e1, p[0]);
+    p[5] = min_num(1.0, max_num(0.0, p[5]));
+    p[6] = min_num(1.0, max_num(0.0, p[6]));
     if (c.iturb >= -1) {
-      p[7] = fmax(p[7], 1.0e-16);
-      p[8] = fmax(fmax(p[8], 1.0e-16), d.ocut[g]);
+      p[7] = max_num(p[7], 1.0e-16);
+      p[8] = max_num(max_num(p[8], 1.0e-16), d.ocut[g]);
     }
     // the state, its change norms and the largest |dp| before the EOS, so that only the EOS's
     // inputs stay live across it
@@ -1732,8 +1747,9 @@ __global__ void __launch_bounds__(128, MX && !EX ? 8 : 3) k_update(DevPtr d, Par
       double df = fabs(old[v] - p[v]);
       sq_[v] += df * df;   // (the clips keep a finite p finite)
     }
-    double dp = fabs(old[0] - p[0]);
-    if (dp > dpmax) { dpmax = dp; dpidx = t; }   // t increases: ties keep the first cell
+    // (numbers not below -1 order like their bit patterns; t increases: ties keep the first cell)
+    const double dp = fabs(old[0] - p[0]);
+    if (__double_as_longlong(dp) > __double_as_longlong(dpmax)) { dpmax = dp; dpidx = t; }
     if constexpr (!MX) {   // (the mixed form's EOS follows in passes of its own: launch_eos_cells)
       const double pe = p[0] + c.pref, te = p[4], y1 = p[5], y2 = p[6];
       double dv[NDV], tv[3] = {0.0, 0.0, 0.0};
@@ -2642,6 +2658,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   if (c.mixed) {
     // the mixed form sweeps by tiles (its records are tile records)
     if (!setup_tiles(E)) return CFD3D_ERR_NOMEM;
+    k_record_faces<<<nblk_of(E.nint, 256), 256, 0, E.st>>>(E.d);
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

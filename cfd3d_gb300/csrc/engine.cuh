@@ -87,8 +87,13 @@ enum { LQ_VP = 0, LQ_VT, LQ_HP, LQ_HT, LQ_RP, LQ_RT, LQ_RDEV, LQ_HDEV, LQ_RHO, L
 // the lane's own previous cell and the previous cells of lanes -1 and -TILE_J (+1, +TILE_J).
 constexpr int TILE_I = 8, TILE_J = 8, TILE_K = 4;
 static_assert(TILE_J * TILE_K == 32, "one lane per (j, k) column of a tile");
-constexpr int TILE_LS = TILE_I + 1;          // slots per lane: odd, so lanes hit distinct banks
+constexpr int TILE_LS = TILE_I;              // slots per lane
 constexpr int TILE_SLOTS = 32 * TILE_LS;     // slots per tile
+// (a lane's eight cells fill one 32-byte sector, so the records are written in whole sectors;
+// at nine slots a lane -- padded against bank conflicts -- the residual kernel took 6.9 ms
+// against 6.2 on 14.2 M cells.  In shared memory the lanes of a step still hit distinct banks:
+// lane (lj, lk) reads slot 8 (lj + 8 lk) + s - lj - lk, and the eight lanes whose 8 lj agree
+// modulo 32 have eight different s - lj - lk.)
 // contributions entering a tile, by face cell: the i face (one per lane), then the j face
 // (TILE_K x TILE_I cells) from TILE_IN_J, then the k face (TILE_J x TILE_I) from TILE_IN_K
 constexpr int TILE_IN_J = 32, TILE_IN_K = TILE_IN_J + TILE_K * TILE_I, TILE_IN = TILE_IN_K + TILE_J * TILE_I;
@@ -103,7 +108,7 @@ enum {
   TR_DIAG = 18,    // 23 values of the closed-form diagonal block
   TR_X = 41,       // the own part of dq (npv)
   TR_COMMON = 50,
-  TR_FACEP = 50,   // + face vectors cx, ex, tx
+  TR_FACEP = 50,   // + face vectors cx, ex, tx (written once, k_record_faces, as are the - ones)
   TR_SPECP = 59,   // + face spectral radii of the three directions
   TR_FACEM = 62,   // - face vectors
   TR_SPECM = 71,   // - face spectral radii

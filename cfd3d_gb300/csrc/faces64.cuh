@@ -36,19 +36,6 @@ __device__ __forceinline__ bool dir_cell(const DevPtr& d, int dir, long long t, 
   return true;
 }
 
-// A double's order-preserving integer key (and back: the map is its own inverse): minima
-// and maxima of keys run on the integer pipe.  -0 orders below +0; a NaN orders beyond the
-// infinities.
-__device__ __forceinline__ long long okey(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
-__device__ __forceinline__ double okey_value(long long k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
-}
-// minima and maxima of numbers (no NaN) by their keys
-__device__ __forceinline__ double kmin(double a, double b) { return okey(b) < okey(a) ? b : a; }
-__device__ __forceinline__ double kmax(double a, double b) { return okey(b) > okey(a) ? b : a; }
 __device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 
 // scratch planes of one direction slot and variable

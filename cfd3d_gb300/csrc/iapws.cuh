@@ -75,23 +75,6 @@ constexpr IJN kR2MR[13] = {
     {4, 7, 0.75321581522770e-2},  {4, 10, -0.79238375446139e-2}, {5, 9, -0.22888160778447e-3},
     {5, 10, -0.26456501482810e-2}};
 
-// IAPWS transport correlations: mu0/lambda0 denominators and the rho-T double series
-__constant__ double kVisH[4] = {1.0, 0.978197, 0.579829, -0.202354};
-__constant__ double kConL[4] = {1.0, 6.978267, 2.599096, -0.998254};
-__constant__ double kVisHH[6][7] = {
-    {0.5132047, 0.2151778, -0.2818107, 0.1778064, -0.0417661, 0.0, 0.0},
-    {0.3205656, 0.7317883, -1.070786, 0.460504, 0.0, -0.01578386, 0.0},
-    {0.0, 1.241044, -1.263184, 0.2340379, 0.0, 0.0, 0.0},
-    {0.0, 1.476783, 0.0, -0.4924179, 0.1600435, 0.0, -0.003629481},
-    {-0.7782567, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {0.1885447, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}};
-__constant__ double kConLL[5][6] = {
-    {1.3293046, -0.40452437, 0.24409490, 0.018660751, -0.12961068, 0.044809953},
-    {1.7018363, -2.2156845, 1.6511057, -0.76736002, 0.37283344, -0.11203160},
-    {5.2246158, -10.124111, 4.9874687, -0.27297694, -0.43083393, 0.13333849},
-    {8.7127675, -9.5000611, 4.3786606, -0.91783782, 0.0, 0.0},
-    {-1.8525999, 0.93404690, 0.0, 0.0, 0.0, 0.0}};
-
 // ---- compile-time powers ----------------------------------------------------------
 template <int N, class T>
 __device__ __forceinline__ T cpow(T x, T xi) {
@@ -279,34 +262,54 @@ __device__ __forceinline__ T stiffened_vis(T t) {
   return T(1.788e-3) * exp(T(-1.704) - T(5.306 * 273.0) / temp + T(7.003) * (r * r));
 }
 
+// sum over i, j of c[i][j] a^i b^j by Horner's rule in both.  The tables are local constants of
+// the unrolled loops, so that the FP32 instance reads FP32 literals (as __constant__ doubles
+// they were converted at run time, 70 FP64-pipe slots a cell), and a row's leading zeros --
+// fma(0, b, 0) = 0 for the finite b here -- are not evaluated.
+template <class T, int NI, int NJ>
+__device__ __forceinline__ T transport_series(const double (&c)[NI][NJ], T a, T b) {
+  T s = T(0.0);
+#pragma unroll
+  for (int i = NI - 1; i >= 0; --i) {
+    T row = T(0.0);
+    bool lead = true;
+#pragma unroll
+    for (int j = NJ - 1; j >= 0; --j) {
+      if (lead && c[i][j] == 0.0) continue;
+      lead = false;
+      row = row * b + T(c[i][j]);
+    }
+    s = s * a + row;
+  }
+  return s;
+}
+
 // IAPWS viscosity and conductivity (critical enhancement off, as in the reference)
 template <class T>
 __device__ __forceinline__ void iapws_transport(T t, T rho, T& vis, T& cond) {
+  constexpr double kVisHH[6][7] = {
+      {0.5132047, 0.2151778, -0.2818107, 0.1778064, -0.0417661, 0.0, 0.0},
+      {0.3205656, 0.7317883, -1.070786, 0.460504, 0.0, -0.01578386, 0.0},
+      {0.0, 1.241044, -1.263184, 0.2340379, 0.0, 0.0, 0.0},
+      {0.0, 1.476783, 0.0, -0.4924179, 0.1600435, 0.0, -0.003629481},
+      {-0.7782567, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0},
+      {0.1885447, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}};
+  constexpr double kConLL[5][6] = {
+      {1.3293046, -0.40452437, 0.24409490, 0.018660751, -0.12961068, 0.044809953},
+      {1.7018363, -2.2156845, 1.6511057, -0.76736002, 0.37283344, -0.11203160},
+      {5.2246158, -10.124111, 4.9874687, -0.27297694, -0.43083393, 0.13333849},
+      {8.7127675, -9.5000611, 4.3786606, -0.91783782, 0.0, 0.0},
+      {-1.8525999, 0.93404690, 0.0, 0.0, 0.0, 0.0}};
   T tt = t * T(0.00154495032985);
   T rr = fmax(T(1.0e-3), fmin(T(1332.4), rho)) * T(0.00314699949333);
   T tt1 = T(647.27) / t;
   T a = tt1 - T(1.0), b = rr - T(1.0);
   T st = sqrt(tt);
-  T mu0 = st / (T(kVisH[0]) + T(kVisH[1]) * tt1 + T(kVisH[2]) * (tt1 * tt1) + T(kVisH[3]) * (tt1 * tt1 * tt1));
-  T mu1 = T(0.0);
-#pragma unroll
-  for (int i = 5; i >= 0; --i) {
-    T row = T(0.0);
-#pragma unroll
-    for (int j = 6; j >= 0; --j) row = row * b + T(kVisHH[i][j]);
-    mu1 = mu1 * a + row;
-  }
-  vis = T(55.071e-6) * mu0 * exp(rr * mu1);
-  T lam0 = st / (T(kConL[0]) + T(kConL[1]) * tt1 + T(kConL[2]) * (tt1 * tt1) + T(kConL[3]) * (tt1 * tt1 * tt1));
-  T lam1 = T(0.0);
-#pragma unroll
-  for (int i = 4; i >= 0; --i) {
-    T row = T(0.0);
-#pragma unroll
-    for (int j = 5; j >= 0; --j) row = row * b + T(kConLL[i][j]);
-    lam1 = lam1 * a + row;
-  }
-  cond = T(0.4945) * (lam0 * exp(rr * lam1));
+  // mu0 / lambda0 denominators
+  T mu0 = st / (T(1.0) + T(0.978197) * tt1 + T(0.579829) * (tt1 * tt1) + T(-0.202354) * (tt1 * tt1 * tt1));
+  vis = T(55.071e-6) * mu0 * exp(rr * transport_series<T>(kVisHH, a, b));
+  T lam0 = st / (T(1.0) + T(6.978267) * tt1 + T(2.599096) * (tt1 * tt1) + T(-0.998254) * (tt1 * tt1 * tt1));
+  cond = T(0.4945) * (lam0 * exp(rr * transport_series<T>(kConLL, a, b)));
 }
 
 }  // namespace cfd

@@ -541,6 +541,27 @@ __device__ __forceinline__ bool finite_bits(double x) {
   return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
 
+// A double's order-preserving integer key (and back: the map is its own inverse): minima
+// and maxima of keys run on the integer pipe.  -0 orders below +0; a NaN orders beyond the
+// infinities.
+__device__ __forceinline__ long long okey(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double okey_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+// minima and maxima of numbers (no NaN) by their keys
+__device__ __forceinline__ double kmin(double a, double b) { return okey(b) < okey(a) ? b : a; }
+__device__ __forceinline__ double kmax(double a, double b) { return okey(b) > okey(a) ? b : a; }
+// fmin and fmax on the integer pipe (an FP64 comparison takes a slot of the FP64 pipe); anything
+// with a NaN takes the functions themselves
+__device__ __forceinline__ bool is_num(double x) {
+  return (unsigned long long)(__double_as_longlong(x) & 0x7fffffffffffffffLL) <= 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ double min_num(double a, double b) { return is_num(a) && is_num(b) ? kmin(a, b) : fmin(a, b); }
+__device__ __forceinline__ double max_num(double a, double b) { return is_num(a) && is_num(b) ? kmax(a, b) : fmax(a, b); }
+
 // ------------------------------------------------------------------ MUSCL / MLP
 // Products and sums without FMA contraction.  A reconstructed state often lands exactly
 // on a clip bound (y1 = 0 next to a cell without vapour, when the MLP factor is exactly 2),
