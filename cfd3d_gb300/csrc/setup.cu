@@ -1007,13 +1007,15 @@ bool setup_tiles(Engine& E) {
   }
   cudaMemcpy(E.d_tiles, tiles.data(), ntile * sizeof(TileDesc), cudaMemcpyHostToDevice);
   cudaMemcpy(E.d_pos, pos.data(), E.ncell * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemset(E.d.tq, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float));
-  cudaMemset(E.d.tyf, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float));
-  cudaMemset(E.d.tyb, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float));
-  cudaMemset(E.d.trf, 0, (size_t)ntile * NTR * TILE_SLOTS * sizeof(float));
-  cudaMemset(E.d.tin, 0, (size_t)ntile * NPVM * TILE_IN * sizeof(float));
-  cudaMemset(E.d.done, 0, (size_t)ntile * sizeof(int));
-  cudaMemset(E.d.tickets, 0, 2 * sizeof(unsigned));
+  // (on the engine's stream, which is not ordered after the default one: k_record_faces writes
+  // the records next)
+  cudaMemsetAsync(E.d.tq, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
+  cudaMemsetAsync(E.d.tyf, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
+  cudaMemsetAsync(E.d.tyb, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
+  cudaMemsetAsync(E.d.trf, 0, (size_t)ntile * NTR * TILE_SLOTS * sizeof(float), E.st);
+  cudaMemsetAsync(E.d.tin, 0, (size_t)ntile * NPVM * TILE_IN * sizeof(float), E.st);
+  cudaMemsetAsync(E.d.done, 0, (size_t)ntile * sizeof(int), E.st);
+  cudaMemsetAsync(E.d.tickets, 0, 2 * sizeof(unsigned), E.st);
   E.d.tiles = E.d_tiles;
   E.d.pos = E.d_pos;
   return true;
