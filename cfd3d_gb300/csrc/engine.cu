@@ -1097,7 +1097,7 @@ __global__ void __launch_bounds__(256, MX ? 4 : 1) k_rhs(DevPtr d, Par c, long l
     float rf[NPVM], xf[NPVM];
 #pragma unroll
     for (int v = 0; v < NPVM; ++v) { rf[v] = (v < npv) ? (float)res[v] : 0.0f; xf[v] = 0.0f; }
-    diag_solve_t<float>(c, Df, p2f, dvf, rf, xf);
+    diag_solve_t<float>(c.npv, Df, p2f, dvf, rf, xf);
     float* R = d.trf + trf_at(sl, 0);
 #pragma unroll
     for (int v = 0; v < NPVM; ++v)
@@ -1502,13 +1502,13 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                : : "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
-template <bool FWD>
+template <bool FWD, int npv>
 __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long spin, int withhold) {
   extern __shared__ __align__(128) unsigned char smem[];
   float* S32 = reinterpret_cast<float*>(smem);
   float* SIN = reinterpret_cast<float*>(smem + TILE_B32);
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + TILE_B32 + TILE_BIN);
-  const int lane = threadIdx.x, npv = c.npv;
+  const int lane = threadIdx.x;
   const int lj = lane % TILE_J, lk = lane / TILE_J;
   const float sgn = FWD ? 1.0f : -1.0f;
   unsigned* ticket = d.tickets + (FWD ? 0 : 1);
@@ -1608,7 +1608,7 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
         float y[NPVM];
 #pragma unroll
         for (int v = 0; v < NPVM; ++v) y[v] = 0.0f;
-        diag_solve_t<float>(c, D, pv, dv, acc, y);
+        diag_solve_t<float>(npv, D, pv, dv, acc, y);
         // dq in FP32 for the products: own part + correction; the correction kept for the
         // update, and (forward) dq* as the backward sweep's own part
         float dqf[NPVM];
@@ -1665,6 +1665,15 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
       st_release(d.done + tile, 1);
     }
   }
+}
+
+using SweepTile = void (*)(DevPtr, Par, long long, int);
+static SweepTile sweep_tile_kernel(bool fwd, int npv) {
+  return npv > 7 ? (fwd ? k_sweep_tile<true, 9> : k_sweep_tile<false, 9>)
+                 : (fwd ? k_sweep_tile<true, 7> : k_sweep_tile<false, 7>);
+}
+static void launch_sweep_tile(const Engine& E, bool fwd, int grid, cudaStream_t s, long long spin, int withhold) {
+  sweep_tile_kernel(fwd, E.par.npv)<<<grid, 32, TILE_SMEM, s>>>(E.d, E.par, spin, withhold);
 }
 
 // ------------------------------------------------------------------ update + residual
@@ -2164,10 +2173,10 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
     // tile sweeps: flags and tickets cleared, one persistent launch per sweep
     cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), s);
     cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), s);
-    k_sweep_tile<true><<<E.sweep_grid, 32, TILE_SMEM, s>>>(d, c, SWEEP_SPIN, -1);
+    launch_sweep_tile(E, true, E.sweep_grid, s, SWEEP_SPIN, -1);
     stage(5);
     cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), s);
-    k_sweep_tile<false><<<E.sweep_grid, 32, TILE_SMEM, s>>>(d, c, SWEEP_SPIN, -1);
+    launch_sweep_tile(E, false, E.sweep_grid, s, SWEEP_SPIN, -1);
     n += 2;
   } else if (!E.sweep_planes) {
     // dataflow sweeps: tickets cleared and dq unset, one persistent launch per sweep
@@ -2662,12 +2671,12 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    CFD_CUDA(cudaFuncSetAttribute(k_sweep_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
-    CFD_CUDA(cudaFuncSetAttribute(k_sweep_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
+    for (bool fwd : {true, false})
+      CFD_CUDA(cudaFuncSetAttribute(sweep_tile_kernel(fwd, c.npv), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
     // the largest shared-memory carveout: three tiles' records per SM
-    CFD_CUDA(cudaFuncSetAttribute(k_sweep_tile<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    CFD_CUDA(cudaFuncSetAttribute(k_sweep_tile<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_tile<true>, 32, TILE_SMEM);
+    for (bool fwd : {true, false})
+      CFD_CUDA(cudaFuncSetAttribute(sweep_tile_kernel(fwd, c.npv), cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), 32, TILE_SMEM);
     E.sweep_grid = std::max(1, std::min(std::max(per, 1) * nsm, E.d.ntile));
     CFD_CUDA(cudaDeviceSynchronize());
     return CFD3D_OK;
@@ -3418,7 +3427,7 @@ int cfd3d_autotune(cfd3d_handle* h, int reps, int* choice) {
   int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_tile<true>, 32, TILE_SMEM);
+  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), 32, TILE_SMEM);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
   const int nwork = c.mixed ? d.ntile : d.nchunk;
   int bestg = E.sweep_grid;
@@ -3432,11 +3441,11 @@ int cfd3d_autotune(cfd3d_handle* h, int reps, int* choice) {
       cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), E.st);
       if (c.mixed) cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
       else unset_dq(E, E.st);
-      if (c.mixed) k_sweep_tile<true><<<grid, 32, TILE_SMEM, E.st>>>(d, c, SWEEP_SPIN, -1);
+      if (c.mixed) launch_sweep_tile(E, true, grid, E.st, SWEEP_SPIN, -1);
       else k_sweep_df<true><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN_DQ, -1);
       if (c.mixed) cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
       else unset_dq(E, E.st);
-      if (c.mixed) k_sweep_tile<false><<<grid, 32, TILE_SMEM, E.st>>>(d, c, SWEEP_SPIN, -1);
+      if (c.mixed) launch_sweep_tile(E, false, grid, E.st, SWEEP_SPIN, -1);
       else k_sweep_df<false><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN_DQ, -1);
     });
     if (t < tbest) { tbest = t; bestg = grid; }
@@ -3471,7 +3480,7 @@ int cfd3d_sweep_stall_test(cfd3d_handle* h) {
   CFD_CUDA(cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), E.st));
   if (c.mixed) CFD_CUDA(cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), E.st));
   else unset_dq(E, E.st);
-  if (c.mixed) k_sweep_tile<true><<<E.sweep_grid, 32, TILE_SMEM, E.st>>>(d, c, 1 << 12, 0);
+  if (c.mixed) launch_sweep_tile(E, true, E.sweep_grid, E.st, 1 << 12, 0);
   else k_sweep_df<true><<<E.sweep_grid, 4 * SW_CH, 0, E.st>>>(d, c, 1 << 12, 0);
   CFD_CUDA(cudaStreamSynchronize(E.st));
   CFD_CUDA(cudaGetLastError());
@@ -3598,7 +3607,7 @@ int cfd3d_set_launch_shapes(cfd3d_handle* h, const int* shapes) {
   int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_tile<true>, 32, TILE_SMEM);
+  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), 32, TILE_SMEM);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
   if (shapes[2] < 1 || shapes[2] > std::max(per, 1)) { E.err = "sweep CTAs per SM outside 1 .. the occupancy limit"; return CFD3D_ERR_ARG; }
   const int nb = (int)E.blk.size();

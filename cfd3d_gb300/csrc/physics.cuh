@@ -1406,8 +1406,9 @@ __device__ __forceinline__ void diag_spectral_f(const Par& c, const float* pv, f
 }
 
 // x = D^-1 res (lhs%getx)
+// (npv is 7 or 9: a caller that knows it at compile time keeps x in registers)
 template <class R>
-__device__ __forceinline__ void diag_solve_t(const Par& c, const DiagT<R>& D, const R* pv, const R* dv, const R* res,
+__device__ __forceinline__ void diag_solve_t(int npv, const DiagT<R>& D, const R* pv, const R* dv, const R* res,
                                              R* x) {
   const R* C4 = D.c;
   R uuu = res[1] * pv[1] + res[2] * pv[2] + res[3] * pv[3] - res[4];
@@ -1424,13 +1425,15 @@ __device__ __forceinline__ void diag_solve_t(const Par& c, const DiagT<R>& D, co
           (coeff3 - D.ssy1 * pv[5] * res[0] + res[5] * D.ssy1)) * D.mm;
   x[5] = (D.ss * (res[5] - res[0] * pv[5]) - C4[3] * D.ss * D.i_b1 * r6 - C4[0] * coeff2 + C4[1] * D.i_b1 * coeff3) * D.mm;
   x[6] = r6 * D.i_b1;
-  if (c.npv > 7) {
+  if (npv > 7) {
     R bd = D.b1 * dv[0];
     R r7 = res[7] - res[0] * pv[7], r8 = res[8] - res[0] * pv[8];
     x[7] = (r8 * D.t[1] - (bd + D.t[3]) * r7) * D.tt;
     x[8] = (r7 * D.t[2] - (bd + D.t[0]) * r8) * D.tt;
   }
-  for (int n = 0; n < c.npv; ++n) x[n] *= D.a;
+#pragma unroll
+  for (int n = 0; n < NPVM; ++n)
+    if (n < npv) x[n] *= D.a;
 }
 // the Diag fields as an array (the sweep record's diagonal part)
 constexpr int PREP_DIAG = 23;
