@@ -425,8 +425,9 @@ __device__ __forceinline__ void deteos_simple(int fluid, double p, double t, dou
 __device__ __forceinline__ void mix_face_mx(double t, double y1, double y2, double il, double hl, double iv,
                                             double hv, double ig, double& rho, double& h) {
   const double yl = 1.0 - y1 - y2;
-  rho = 1.0 / (yl * il + y1 * iv + y2 * ig);
-  h = yl * hl + y1 * hv + y2 * (1004.64 * t);
+  // (contraction spelled out: the states round the same in every kernel)
+  rho = 1.0 / __fma_rn(y2, ig, __fma_rn(yl, il, __dmul_rn(y1, iv)));
+  h = __fma_rn(y2, __dmul_rn(1004.64, t), __fma_rn(yl, hl, __dmul_rn(y1, hv)));
 }
 
 __device__ __forceinline__ void eos_rho_h(int fluid, double p, double t, double y1, double y2, double& rho, double& h) {
