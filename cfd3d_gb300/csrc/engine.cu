@@ -1294,30 +1294,6 @@ __global__ void __launch_bounds__(64) k_sweep(DevPtr d, Par c, long long p0, lon
   sweep_cell<FWD>(d, c, t);
 }
 
-// the tile sweeps' done flags: a release store by one thread after a barrier publishes
-// what the barrier ordered before it (release is cumulative), an acquire load followed by a
-// barrier makes it visible to the threads that passed the barrier
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" : : "l"(p), "r"(v) : "memory");
-}
-
-// a bounded wait for a done flag: gives up (recording sweep_stall, which ends every other
-// wait too) after `spin` polls
-__device__ __forceinline__ void wait_flag(const DevPtr& d, const int* flag, long long spin) {
-  long long it = 0;
-  while (ld_acquire(flag) == 0) {
-    ++it;
-    if ((it & 63) == 0 && *(volatile int*)&d.sc->sweep_stall) break;
-    if (it > spin) { atomicExch(&d.sc->sweep_stall, 1); break; }
-    if (it > 8) __nanosleep(32);
-  }
-}
-
 // Dataflow sweep of the FP64 form: one persistent launch per sweep.  CTAs take chunks
 // (runs of at most SW_CH cells of one plane) in plane order -- reversed for the backward
 // sweep -- from a ticket counter.  What bounds it is the chain over the ni + nj + nk planes:
@@ -1464,28 +1440,44 @@ __global__ void __launch_bounds__(4 * SW_CH) k_sweep_df(DevPtr d, Par c, long lo
 // k_rhs writes x0 (FP32) into tq and into the cell's tile record; the sweeps work in FP32
 // alone -- the products take dq in FP32 -- and store their corrections y_f, y_b; the update
 // forms dq = x0 + y_f + y_b and adds it to pv in FP64.  (On a GB300 each FP64 instruction
-// holds a warp for tens of cycles: none stays on the sweeps' dependency chain.)  One warp sweeps one tile at a
-// time (tiles from a ticket counter in tile-hyperplane order, reversed for the backward
-// sweep): it stages the tile's records in shared memory with one bulk copy per array
-// (cp.async.bulk, completion on an mbarrier), waits for the done flags of the (at most
-// three) tiles it depends on, reads the contributions they left at its faces, and then
-// walks the tile's hyperplanes: lane (lj, lk) holds cell (s - lj - lk, lj, lk) at step s.
-// Each cell forms its products A.dq for its three downstream neighbours (its outgoing
-// contributions) once its dq is known: the +i one stays in the lane for its next cell, the
-// +j and +k ones move to lanes +1 and +TILE_J by shuffles, and those leaving the tile go to
-// the downstream tile's entry block (tin).  So only FP32 arithmetic, shuffles and the done
-// flags between tiles lie on the sweep's dependency chain.  The waits are bounded as in the
-// FP64 form's dataflow sweep; `withhold` >= 0 names a tile whose flag is never raised (the
-// stall test).
+// holds a warp for tens of cycles: none stays on the sweeps' dependency chain.)  A CTA
+// sweeps one tile at a time (tiles from a ticket counter in tile-hyperplane order, reversed
+// for the backward sweep) with one warp: it stages the tile's records in shared memory with
+// two bulk copies (cp.async.bulk, completion on an mbarrier) and walks the tile's
+// hyperplanes: lane (lj, lk) holds cell (s - lj - lk, lj, lk) at step s.  Each cell forms
+// its products A.dq for its three downstream neighbours (its outgoing contributions) once
+// its dq is known: the +i one stays in the lane for its next cell, the +j and +k ones move
+// to lanes +1 and +TILE_J by shuffles, and those leaving the tile go to the downstream
+// tile's entry block (tin).
+// What bounds a sweep is the chain of these steps over the tiles, so a tile does not wait
+// for the ones before it to finish, only step by step for what it needs of them: the
+// entries are the signal themselves (tin starts as all ones, a NaN pattern that no
+// contribution keeps), and four more warps, a thread per entry, poll them into shared
+// memory and arrive at an mbarrier per step (tile_entry).  A tile then starts 8, 8 or 4
+// steps after the one before it in i, j or k, where with done flags it started 18 later
+// plus a fence and a round trip to L2.  Both sweeps of an iteration: 1.03 -> 0.49 ms at
+// 128x64x64 cells, 0.22 -> 0.12 ms at 16x12x10, 1.15 -> 0.94 ms on 24 uneven blocks of 3.0 M
+// cells, 4.0 -> 3.6 ms on 8 blocks of 14.2 M.  (Three warps with a product each, the solution
+// in all of them, took 1.7 ms where one warp took 1.03.)
+// The needed tiles always hold earlier tickets, so the waits end; they are bounded as in the
+// FP64 form's dataflow sweep; `withhold` >= 0 names a tile whose contributions are never
+// written (the stall test).
 constexpr unsigned TILE_B32 = TS_FIELDS * TILE_SLOTS * 4;   // the FP32 fields one sweep reads
 constexpr unsigned TILE_BIN = NPVM * TILE_IN * 4;           // the entering contributions
-constexpr unsigned TILE_SMEM = TILE_B32 + TILE_BIN + 16;
+constexpr int TILE_SIG = TILE_I + TILE_J - 1;               // steps that contributions enter at (k face: the most)
+constexpr unsigned TILE_SMEM = TILE_B32 + TILE_BIN + 8 * (1 + TILE_SIG);
+constexpr int TILE_T = 32 + TILE_IN;                        // the sweeping warp, and a thread per entry
+constexpr unsigned IN_UNSET = ~0u;
+static_assert(TILE_I == 8 && TILE_J == 8, "tile_entry takes an entry's face coordinates modulo 8");
 static_assert(TILE_B32 % 16 == 0 && (TR_COMMON * TILE_SLOTS * 4) % 16 == 0, "bulk copies move multiples of 16 bytes");
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" : : "r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_init(unsigned long long* bar, int arrivals) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" : : "r"(smem_u32(bar)), "r"(arrivals) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" : : : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" : : "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_expect(unsigned long long* bar, unsigned bytes) {
   asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }"
@@ -1497,31 +1489,119 @@ __device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned pari
                : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
+// (bounded: the guard of a wait that ends by itself)
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
+  for (long long it = 0; it < (1ll << 26); ++it)
+    if (mbar_test(bar, parity)) return true;
+  return false;
+}
+__device__ __forceinline__ unsigned ld_relaxed(const float* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_entry(float* p, float x) {
+  unsigned b = __float_as_uint(x);
+  if (b == IN_UNSET) b = 0x7fc00000u;   // (a NaN all the same)
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" : : "l"(p), "r"(b) : "memory");
+}
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                : : "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// One entry of a tile (a face cell's contribution): polls its values in the entry block until
+// the tile before has written them all, copies them to shared memory and arrives at the
+// barrier of the step that needs them.  Far from its turn a warp polls one value per entry
+// and sleeps between polls; once one of its entries has come it polls whole entries.
 template <bool FWD, int npv>
-__global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long spin, int withhold) {
+__device__ __forceinline__ void tile_entry(const DevPtr& d, const TileDesc& T, int tile, int h, float* SIN,
+                                           unsigned long long* sig, long long spin) {
+  // sweep-local coordinates of the entry's cell on its face, and its slot in the entry block
+  const int face = (h < TILE_IN_J) ? 0 : (h < TILE_IN_K) ? 1 : 2;
+  const int p = (h & 7), q = (face == 2) ? (h - TILE_IN_K) >> 3 : (h & 31) >> 3;
+  const int np = (face == 0) ? T.nj : T.ni, nq = (face == 2) ? T.nj : T.nk;
+  const int dep = FWD ? (face == 0 ? T.lo[0] : face == 1 ? T.lo[1] : T.lo[2])
+                      : (face == 0 ? T.hi[0] : face == 1 ? T.hi[1] : T.hi[2]);
+  const bool live = p < np && q < nq;
+  const int at = live ? h - (p + 8 * q) + (FWD ? p + 8 * q : np - 1 - p + 8 * (nq - 1 - q)) : h;
+  const float* in = d.tin + (long long)tile * NPVM * TILE_IN + at;
+  bool todo = live && dep >= 0, near = false;
+  if (!todo) {   // block faces bring no contribution
+    if (live)
+#pragma unroll
+      for (int v = 0; v < npv; ++v) SIN[v * TILE_IN + at] = 0.0f;
+    mbar_arrive(sig + p + q);
+  }
+  for (long long it = 0; __any_sync(0xffffffffu, todo); ++it) {
+    unsigned w[npv];
+    bool set = false;
+    if (todo) {
+      w[npv - 1] = ld_relaxed(in + (npv - 1) * TILE_IN);
+      set = w[npv - 1] != IN_UNSET;
+      if (near) {
+#pragma unroll
+        for (int v = 0; v < npv - 1; ++v) w[v] = ld_relaxed(in + v * TILE_IN);
+#pragma unroll
+        for (int v = 0; v < npv - 1; ++v) set = set && w[v] != IN_UNSET;
+      }
+    }
+    if (!near) {
+      near = __any_sync(0xffffffffu, set);
+      set = false;
+      if (!near) __nanosleep(it > 64 ? 200 : 20);
+    }
+    bool out = it >= spin;
+    if ((it & 63) == 63 && *(volatile int*)&d.sc->sweep_stall) out = true;
+    if (out && todo && !set) {
+      atomicExch(&d.sc->sweep_stall, 1);
+#pragma unroll
+      for (int v = 0; v < npv; ++v) w[v] = 0u;
+      set = true;
+    }
+    if (todo && set) {
+#pragma unroll
+      for (int v = 0; v < npv; ++v) SIN[v * TILE_IN + at] = __uint_as_float(w[v]);
+      mbar_arrive(sig + p + q);
+      todo = false;
+    }
+  }
+}
+
+template <bool FWD, int npv>
+__global__ void __launch_bounds__(TILE_T, 3) k_sweep_tile(DevPtr d, Par c, long long spin, int withhold) {
   extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ int s_q[2];
   float* S32 = reinterpret_cast<float*>(smem);
   float* SIN = reinterpret_cast<float*>(smem + TILE_B32);
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + TILE_B32 + TILE_BIN);
-  const int lane = threadIdx.x;
+  unsigned long long* sig = bar + 1;   // one per step that contributions enter at
+  const int lane = threadIdx.x;        // (of the sweeping warp)
   const int lj = lane % TILE_J, lk = lane / TILE_J;
   const float sgn = FWD ? 1.0f : -1.0f;
   unsigned* ticket = d.tickets + (FWD ? 0 : 1);
-  if (lane == 0) mbar_init(bar);
-  __syncwarp();
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  if (threadIdx.x < TILE_SIG) {
+    // the entries a step needs: face cells whose sweep-local coordinates add up to it
+    int m = 0;
+    for (int p = 0; p < 8; ++p) {
+      const int q = (int)threadIdx.x - p;
+      m += 2 * (q >= 0 && q < TILE_K) + (q >= 0 && q < TILE_J);
+    }
+    mbar_init(sig + threadIdx.x, m);
+  }
   unsigned parity = 0;
-  for (;;) {
-    int q = 0;
-    if (lane == 0) q = (int)atomicAdd(ticket, 1u);
-    q = __shfl_sync(0xffffffffu, q, 0);
+  for (;; parity ^= 1u) {
+    if (threadIdx.x == 0) s_q[parity] = (int)atomicAdd(ticket, 1u);
+    __syncthreads();
+    const int q = s_q[parity];
     if (q >= d.ntile) break;
     const int tile = FWD ? q : d.ntile - 1 - q;
     const TileDesc T = d.tiles[tile];
+    if (threadIdx.x >= 32) {
+      tile_entry<FWD, npv>(d, T, tile, threadIdx.x - 32, SIN, sig, spin);
+      continue;
+    }
     // ---- stage the tile's records (written by earlier launches): the common fields and
     // this sweep's faces and spectral radii
     if (lane == 0) {
@@ -1532,32 +1612,17 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
       bulk_load(S32, rf, TR_COMMON * TILE_SLOTS * 4, bar);
       bulk_load(S32 + TR_COMMON * TILE_SLOTS, rf + (FWD ? TR_FACEP : TR_FACEM) * TILE_SLOTS, 12 * TILE_SLOTS * 4, bar);
     }
-    // ---- the tiles this one depends on, then the contributions they left at its faces
-    // (the tiles before and after, as scalars: no indexing into the descriptor)
-    const int dep0 = FWD ? T.lo[0] : T.hi[0], dep1 = FWD ? T.lo[1] : T.hi[1], dep2 = FWD ? T.lo[2] : T.hi[2];
-    const int nxt0 = FWD ? T.hi[0] : T.lo[0], nxt1 = FWD ? T.hi[1] : T.lo[1], nxt2 = FWD ? T.hi[2] : T.lo[2];
-    {
-      const int mine = (lane == 0) ? dep0 : (lane == 1) ? dep1 : (lane == 2) ? dep2 : -1;
-      if (mine >= 0) wait_flag(d, d.done + mine, spin);
-    }
-    __syncwarp();
-    {
-      const float* in = d.tin + (long long)tile * NPVM * TILE_IN;
-      for (int e = lane; e < NPVM * TILE_IN; e += 32) SIN[e] = __ldcg(in + e);
-    }
+    // the tiles after this one (as scalars: no indexing into the descriptor)
+    const bool silent = tile == withhold;
+    const int nxt0 = silent ? -1 : FWD ? T.hi[0] : T.lo[0], nxt1 = silent ? -1 : FWD ? T.hi[1] : T.lo[1],
+              nxt2 = silent ? -1 : FWD ? T.hi[2] : T.lo[2];
     // ---- the staged records (the copy completes by itself: the wait is bounded only as a
     // guard, and on a timeout the tile's cells are skipped)
-    bool staged = false;
-    for (long long it = 0; it < (1ll << 26); ++it)
-      if (mbar_test(bar, parity)) { staged = true; break; }
-    parity ^= 1u;
-    __syncwarp();
+    const bool staged = mbar_wait(bar, parity);
     if (!staged) atomicExch(&d.sc->sweep_stall, 1);
     // ---- the tile's hyperplanes
     const int ni = T.ni, nj = T.nj, nk = T.nk;
     const bool col = lj < nj && lk < nk && staged;
-    // faces with a tile beyond them: the others (block faces) bring no contribution
-    const bool hi_ = dep0 >= 0, hj_ = dep1 >= 0, hk_ = dep2 >= 0;
     // lane's sweep-local column coordinates (reversed in the backward sweep)
     const int pj = FWD ? lj : nj - 1 - lj, pk = FWD ? lk : nk - 1 - lk;
     float ci[NPVM], cj[NPVM], ck[NPVM];
@@ -1565,6 +1630,8 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
     for (int v = 0; v < NPVM; ++v) ci[v] = cj[v] = ck[v] = 0.0f;
     const int nsteps = ni + nj + nk - 2;
     for (int s = 0; s < nsteps; ++s) {
+      // the step's entering contributions (their waits are bounded, so this one ends)
+      if (s < TILE_SIG && !mbar_wait(sig + s, parity)) atomicExch(&d.sc->sweep_stall, 1);
       // the +j / +k contributions of the previous step from the neighbouring columns
       float rj[NPVM], rk[NPVM];
 #pragma unroll
@@ -1581,9 +1648,12 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
         const bool fi = pi == 0, fj = pj == 0, fk = pk == 0;
 #pragma unroll
         for (int v = 0; v < NPVM; ++v) {
-          const float a0 = fi ? (hi_ ? SIN[v * TILE_IN + lj + TILE_J * lk] : 0.0f) : ci[v];
-          const float a1 = fj ? (hj_ ? SIN[v * TILE_IN + TILE_IN_J + TILE_I * lk + li] : 0.0f) : rj[v];
-          const float a2 = fk ? (hk_ ? SIN[v * TILE_IN + TILE_IN_K + TILE_I * lj + li] : 0.0f) : rk[v];
+          float a0 = ci[v], a1 = rj[v], a2 = rk[v];
+          if (v < npv) {
+            if (fi) a0 = SIN[v * TILE_IN + lj + TILE_J * lk];
+            if (fj) a1 = SIN[v * TILE_IN + TILE_IN_J + TILE_I * lk + li];
+            if (fk) a2 = SIN[v * TILE_IN + TILE_IN_K + TILE_I * lj + li];
+          }
           acc[v] = (a0 + a1) + a2;
         }
         // the cell's state and diagonal block (FP32), D^-1 acc, dq = own part + it
@@ -1641,28 +1711,18 @@ __global__ void __launch_bounds__(32) k_sweep_tile(DevPtr d, Par c, long long sp
         contribution(1, cj);
         contribution(2, ck);
         // contributions that leave the tile: into the entry block of the tile beyond
-        if (pi == ni - 1 && nxt0 >= 0) {
-          float* dst = d.tin + (long long)nxt0 * NPVM * TILE_IN + lj + TILE_J * lk;
-          for (int v = 0; v < NPVM; ++v) dst[v * TILE_IN] = ci[v];
-        }
-        if (pj == nj - 1 && nxt1 >= 0) {
-          float* dst = d.tin + (long long)nxt1 * NPVM * TILE_IN + TILE_IN_J + TILE_I * lk + li;
-          for (int v = 0; v < NPVM; ++v) dst[v * TILE_IN] = cj[v];
-        }
-        if (pk == nk - 1 && nxt2 >= 0) {
-          float* dst = d.tin + (long long)nxt2 * NPVM * TILE_IN + TILE_IN_K + TILE_I * lj + li;
-          for (int v = 0; v < NPVM; ++v) dst[v * TILE_IN] = ck[v];
-        }
+        auto leave = [&](int to, int at, const float* o) {
+          float* dst = d.tin + (long long)to * NPVM * TILE_IN + at;
+#pragma unroll
+          for (int v = 0; v < npv; ++v) st_entry(dst + v * TILE_IN, o[v]);
+        };
+        if (pi == ni - 1 && nxt0 >= 0) leave(nxt0, lj + TILE_J * lk, ci);
+        if (pj == nj - 1 && nxt1 >= 0) leave(nxt1, TILE_IN_J + TILE_I * lk + li, cj);
+        if (pk == nk - 1 && nxt2 >= 0) leave(nxt2, TILE_IN_K + TILE_I * lj + li, ck);
       } else {
 #pragma unroll
         for (int v = 0; v < NPVM; ++v) cj[v] = ck[v] = 0.0f;
       }
-    }
-    // ---- publish the tile's contributions and dq
-    __syncwarp();
-    if (lane == 0 && tile != withhold) {
-      __threadfence();
-      st_release(d.done + tile, 1);
     }
   }
 }
@@ -1673,7 +1733,7 @@ static SweepTile sweep_tile_kernel(bool fwd, int npv) {
                  : (fwd ? k_sweep_tile<true, 7> : k_sweep_tile<false, 7>);
 }
 static void launch_sweep_tile(const Engine& E, bool fwd, int grid, cudaStream_t s, long long spin, int withhold) {
-  sweep_tile_kernel(fwd, E.par.npv)<<<grid, 32, TILE_SMEM, s>>>(E.d, E.par, spin, withhold);
+  sweep_tile_kernel(fwd, E.par.npv)<<<grid, TILE_T, TILE_SMEM, s>>>(E.d, E.par, spin, withhold);
 }
 
 // ------------------------------------------------------------------ update + residual
@@ -2010,9 +2070,8 @@ int ensure_copy_stream(cfd3d_handle* h) {
   return CFD3D_OK;
 }
 
-// polls of a tile's done flag, and of a neighbour's dq in the FP64 form, before a sweep gives
-// up (some tenths of a second)
-constexpr long long SWEEP_SPIN = 1ll << 22, SWEEP_SPIN_DQ = 1ll << 19;
+// polls of a neighbour's values before a sweep gives up (some tenths of a second)
+constexpr long long SWEEP_SPIN = 1ll << 19;
 
 // k_rhs in the instantiation of the form (mixed / FP64), the time integrator (sweep records
 // for LU-SGS) and the extended sources (DES length scale, gravity)
@@ -2100,9 +2159,11 @@ int launch_boundary(const Engine& E, cudaStream_t s) {
   return n;
 }
 
-// dqs as the FP64 form's dataflow sweeps expect it at their start
+// dqs (the FP64 form) and the tiles' entry blocks (the mixed form) as the dataflow sweeps
+// expect them at their start
 void unset_dq(const Engine& E, cudaStream_t s) {
-  cudaMemsetAsync(E.d.dqs, 0xff, (size_t)E.par.npv * E.nint * sizeof(double), s);
+  if (E.par.mixed) cudaMemsetAsync(E.d.tin, 0xff, (size_t)E.d.ntile * NPVM * TILE_IN * sizeof(float), s);
+  else cudaMemsetAsync(E.d.dqs, 0xff, (size_t)E.par.npv * E.nint * sizeof(double), s);
 }
 
 // the launch sequence of one iteration (captured into the graph); `mark` (optional)
@@ -2170,22 +2231,22 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
     return;
   }
   if (c.mixed) {
-    // tile sweeps: flags and tickets cleared, one persistent launch per sweep
+    // tile sweeps: entries unset and tickets cleared, one persistent launch per sweep
     cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), s);
-    cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), s);
+    unset_dq(E, s);
     launch_sweep_tile(E, true, E.sweep_grid, s, SWEEP_SPIN, -1);
     stage(5);
-    cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), s);
+    unset_dq(E, s);
     launch_sweep_tile(E, false, E.sweep_grid, s, SWEEP_SPIN, -1);
     n += 2;
   } else if (!E.sweep_planes) {
     // dataflow sweeps: tickets cleared and dq unset, one persistent launch per sweep
     cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), s);
     unset_dq(E, s);
-    k_sweep_df<true><<<E.sweep_grid, 4 * SW_CH, 0, s>>>(d, c, SWEEP_SPIN_DQ, -1);
+    k_sweep_df<true><<<E.sweep_grid, 4 * SW_CH, 0, s>>>(d, c, SWEEP_SPIN, -1);
     stage(5);
     unset_dq(E, s);
-    k_sweep_df<false><<<E.sweep_grid, 4 * SW_CH, 0, s>>>(d, c, SWEEP_SPIN_DQ, -1);
+    k_sweep_df<false><<<E.sweep_grid, 4 * SW_CH, 0, s>>>(d, c, SWEEP_SPIN, -1);
     n += 2;
   } else {
     const int np = (int)E.plane_off.size() - 1;
@@ -2676,7 +2737,7 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
     // the largest shared-memory carveout: three tiles' records per SM
     for (bool fwd : {true, false})
       CFD_CUDA(cudaFuncSetAttribute(sweep_tile_kernel(fwd, c.npv), cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), 32, TILE_SMEM);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), TILE_T, TILE_SMEM);
     E.sweep_grid = std::max(1, std::min(std::max(per, 1) * nsm, E.d.ntile));
     CFD_CUDA(cudaDeviceSynchronize());
     return CFD3D_OK;
@@ -2726,7 +2787,6 @@ void cfd3d_destroy(cfd3d_handle* h) {
   cudaFree(E.d_tp_ent);
   cudaFree(E.d_tp_x);
   cudaFree(E.d.rec);
-  cudaFree(E.d.done);
   cudaFree(E.d.tickets);
   cudaFree(E.d_chunk_t0);
   cudaFree(E.d_tiles);
@@ -3427,7 +3487,7 @@ int cfd3d_autotune(cfd3d_handle* h, int reps, int* choice) {
   int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), 32, TILE_SMEM);
+  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), TILE_T, TILE_SMEM);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
   const int nwork = c.mixed ? d.ntile : d.nchunk;
   int bestg = E.sweep_grid;
@@ -3439,14 +3499,12 @@ int cfd3d_autotune(cfd3d_handle* h, int reps, int* choice) {
     // rewrites the right-hand side it reads, which changes the values but not the work)
     const float t = time_calls(E, reps, [&] {
       cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), E.st);
-      if (c.mixed) cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
-      else unset_dq(E, E.st);
+      unset_dq(E, E.st);
       if (c.mixed) launch_sweep_tile(E, true, grid, E.st, SWEEP_SPIN, -1);
-      else k_sweep_df<true><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN_DQ, -1);
-      if (c.mixed) cudaMemsetAsync(d.done, 0, (size_t)nwork * sizeof(int), E.st);
-      else unset_dq(E, E.st);
+      else k_sweep_df<true><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN, -1);
+      unset_dq(E, E.st);
       if (c.mixed) launch_sweep_tile(E, false, grid, E.st, SWEEP_SPIN, -1);
-      else k_sweep_df<false><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN_DQ, -1);
+      else k_sweep_df<false><<<grid, 4 * SW_CH, 0, E.st>>>(d, c, SWEEP_SPIN, -1);
     });
     if (t < tbest) { tbest = t; bestg = grid; }
   }
@@ -3478,8 +3536,7 @@ int cfd3d_sweep_stall_test(cfd3d_handle* h) {
   // raises its flags, with a short poll limit
   launch_iteration(E, false);
   CFD_CUDA(cudaMemsetAsync(d.tickets, 0, 2 * sizeof(unsigned), E.st));
-  if (c.mixed) CFD_CUDA(cudaMemsetAsync(d.done, 0, (size_t)d.ntile * sizeof(int), E.st));
-  else unset_dq(E, E.st);
+  unset_dq(E, E.st);
   if (c.mixed) launch_sweep_tile(E, true, E.sweep_grid, E.st, 1 << 12, 0);
   else k_sweep_df<true><<<E.sweep_grid, 4 * SW_CH, 0, E.st>>>(d, c, 1 << 12, 0);
   CFD_CUDA(cudaStreamSynchronize(E.st));
@@ -3607,7 +3664,7 @@ int cfd3d_set_launch_shapes(cfd3d_handle* h, const int* shapes) {
   int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), 32, TILE_SMEM);
+  if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), TILE_T, TILE_SMEM);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
   if (shapes[2] < 1 || shapes[2] > std::max(per, 1)) { E.err = "sweep CTAs per SM outside 1 .. the occupancy limit"; return CFD3D_ERR_ARG; }
   const int nb = (int)E.blk.size();

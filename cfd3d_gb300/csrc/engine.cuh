@@ -175,16 +175,15 @@ struct DevPtr {
   double* rec;
   const int *cells, *pos, *nbf, *nbb;
   // dataflow sweeps: chunk starts in t (chunks of at most SW_CH cells, never across a
-  // plane; nchunk + 1 entries), the two sweeps' chunk tickets; the tile sweeps' done flags
+  // plane; nchunk + 1 entries), the two sweeps' tickets
   const int* chunk_t0;
   int nchunk;
-  int* done;
   unsigned* tickets;
   // mixed form: the tile sweeps (setup_tiles).  tiles in forward ticket order; trf the FP32
   // tile records; tq the own part D^-1 res per slot (k_rhs, an FP32 solve); tyf / tyb the
   // FP32 corrections of the forward / backward sweep, so that dq = tq + tyf + tyb (k_update);
   // tin the contributions entering each tile (written by the neighbouring tiles during a
-  // sweep); done flags per tile
+  // sweep, all ones until then)
   int ntile;
   long long nslot;
   // mixed form: index lists of the states that need further IF97 sums, by kind (MX_*), mxcap

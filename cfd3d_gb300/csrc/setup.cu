@@ -1000,7 +1000,6 @@ bool setup_tiles(Engine& E) {
       cudaMalloc(&E.d.tyf, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&E.d.tyb, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&E.d.tin, (size_t)ntile * NPVM * TILE_IN * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&E.d.done, (size_t)ntile * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&E.d.tickets, 2 * sizeof(unsigned)) != cudaSuccess) {
     E.err = "device allocation failed (tile sweeps)";
     return false;
@@ -1014,7 +1013,6 @@ bool setup_tiles(Engine& E) {
   cudaMemsetAsync(E.d.tyb, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
   cudaMemsetAsync(E.d.trf, 0, (size_t)ntile * NTR * TILE_SLOTS * sizeof(float), E.st);
   cudaMemsetAsync(E.d.tin, 0, (size_t)ntile * NPVM * TILE_IN * sizeof(float), E.st);
-  cudaMemsetAsync(E.d.done, 0, (size_t)ntile * sizeof(int), E.st);
   cudaMemsetAsync(E.d.tickets, 0, 2 * sizeof(unsigned), E.st);
   E.d.tiles = E.d_tiles;
   E.d.pos = E.d_pos;
