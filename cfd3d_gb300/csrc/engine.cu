@@ -24,6 +24,7 @@
 #include <cstring>
 #include <cuda.h>
 #include <fcntl.h>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <type_traits>
@@ -2407,51 +2408,10 @@ float time_calls(Engine& E, int reps, F fn) {
 }
 }  // namespace
 
+// ---- pointwise EOS: its static device buffer, for few points
 namespace {
-template <bool TERMS>
-int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
-               const double* y2, double* dv, double* tv) {
-  if (n <= 0 || !p || !t || !y1 || !y2 || !dv || (fluid != 1 && fluid != 2) || ngas != 1) return CFD3D_ERR_ARG;
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return CFD3D_ERR_NODEVICE;
-  double *dp = nullptr, *dt = nullptr, *dy1 = nullptr, *dy2 = nullptr, *ddv = nullptr, *dtv = nullptr;
-  unsigned long long* fb = nullptr;
-  size_t b = (size_t)n * 8;
-  int rc = CFD3D_OK;
-  if (cudaMalloc(&dp, b) || cudaMalloc(&dt, b) || cudaMalloc(&dy1, b) || cudaMalloc(&dy2, b) ||
-      cudaMalloc(&ddv, b * NDV) || cudaMalloc(&dtv, b * 2) || cudaMalloc(&fb, 8)) {
-    rc = CFD3D_ERR_NOMEM;
-  } else {
-    cudaMemcpy(dp, p, b, cudaMemcpyHostToDevice);
-    cudaMemcpy(dt, t, b, cudaMemcpyHostToDevice);
-    cudaMemcpy(dy1, y1, b, cudaMemcpyHostToDevice);
-    cudaMemcpy(dy2, y2, b, cudaMemcpyHostToDevice);
-    cudaMemset(fb, 0, 8);
-    k_eos_points<TERMS><<<(unsigned)((n + 127) / 128), 128>>>(fluid, with_prop, n, dp, dt, dy1, dy2, ddv, dtv, fb);
-    if (cudaMemcpy(dv, ddv, b * NDV, cudaMemcpyDeviceToHost) != cudaSuccess) rc = CFD3D_ERR_CUDA;
-    if (tv && with_prop && cudaMemcpy(tv, dtv, b * 2, cudaMemcpyDeviceToHost) != cudaSuccess) rc = CFD3D_ERR_CUDA;
-  }
-  cudaFree(dp); cudaFree(dt); cudaFree(dy1); cudaFree(dy2); cudaFree(ddv); cudaFree(dtv); cudaFree(fb);
-  return rc;
-}
-}  // namespace
-
-extern "C" {
-
-const char* cfd3d_last_error(const cfd3d_handle* h) { return h ? h->E.err.c_str() : "null handle"; }
-
-int cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
-                   const double* y2, double* dv, double* tv) {
-  return eos_points<false>(fluid, ngas, with_prop, n, p, t, y1, y2, dv, tv);
-}
-
-// ---- pointwise EOS through a static device buffer (no allocation)
-namespace {
-struct EosScratch {
-  double p[CFD3D_EOS_NOALLOC_MAX], t[CFD3D_EOS_NOALLOC_MAX], y1[CFD3D_EOS_NOALLOC_MAX], y2[CFD3D_EOS_NOALLOC_MAX];
-  double dv[NDV * CFD3D_EOS_NOALLOC_MAX], tv[2 * CFD3D_EOS_NOALLOC_MAX];
-  unsigned long long fallbacks;   // must start at zero: the kernel counts into it
-};
+constexpr size_t EOS_PER_POINT = 4 + NDV + 2;   // p, t, y1, y2; dv; tv
+struct EosScratch { double x[1 + EOS_PER_POINT * CFD3D_EOS_NOALLOC_MAX]; };
 // The buffer's device address per CUDA context.  A context has its own copy of every
 // module's globals, and a context that ends (cudaDeviceReset, a primary context released
 // and made again) takes the copy with it, so the cache is keyed on the context's unique id
@@ -2485,6 +2445,94 @@ bool current_ctx_id(unsigned long long& id) {
 }  // namespace
 static __device__ __align__(256) EosScratch g_eos_scratch;
 
+namespace {
+// the buffer's address in the current context (set up on the first call there), or null;
+// g_eos_scratch_mu is held from here to the end of the call that uses the buffer
+double* eos_scratch() {
+  unsigned long long ctx = 0;
+  if (!current_ctx_id(ctx)) return nullptr;
+  for (const ScratchSlot& sl : g_eos_scratch_slots)
+    if (ctx && sl.ctx == ctx) return sl.ptr->x;
+  // (with no context current yet, the lookup makes the device's primary context current)
+  void* ptr = nullptr;
+  if (cudaGetSymbolAddress(&ptr, g_eos_scratch) != cudaSuccess || !ptr) return nullptr;
+  if (!ctx && (!current_ctx_id(ctx) || !ctx)) return nullptr;
+  g_eos_scratch_slots.push_back({ctx, static_cast<EosScratch*>(ptr)});
+  return static_cast<EosScratch*>(ptr)->x;
+}
+
+// n points through the device buffer x (1 + EOS_PER_POINT n doubles).  Few points are a
+// matter of calls, not of bytes: their arrays are packed on the host, one copy each way (up
+// to EOS_PACK doubles, 64 KB).
+constexpr size_t EOS_PACK = 8192;
+template <bool TERMS>
+int eos_run(int fluid, int with_prop, int64_t n, const double* p, const double* t, const double* y1, const double* y2,
+            double* dv, double* tv, double* x) {
+  const size_t m = (size_t)n, b = m * 8, out = (NDV + (tv && with_prop ? 2 : 0)) * m;
+  double *in = x + 1, *ddv = in + 4 * m, *dtv = ddv + NDV * m;
+  unsigned long long* fb = reinterpret_cast<unsigned long long*>(x);   // starts at zero: the kernel counts into it
+  std::unique_ptr<double[]> hold(out <= EOS_PACK ? new (std::nothrow) double[out] : nullptr);
+  double* stage = hold.get();   // (out covers the 4 n + 1 values on the way in)
+  const bool packed = stage != nullptr;
+  const double* src[4] = {p, t, y1, y2};
+  if (packed) {
+    stage[0] = 0.0;
+    for (int q = 0; q < 4; ++q) std::memcpy(stage + 1 + q * m, src[q], b);
+    if (cudaMemcpy(x, stage, 8 + 4 * b, cudaMemcpyHostToDevice) != cudaSuccess) return CFD3D_ERR_CUDA;
+  } else {
+    for (int q = 0; q < 4; ++q)
+      if (cudaMemcpy(in + q * m, src[q], b, cudaMemcpyHostToDevice) != cudaSuccess) return CFD3D_ERR_CUDA;
+    if (cudaMemset(fb, 0, 8) != cudaSuccess) return CFD3D_ERR_CUDA;
+  }
+  // a warp's FP64 instructions follow one another at the pace of its SM's pipe: few points
+  // are spread over the SMs, a warp each
+  const int T = n <= 16384 ? 32 : 128;
+  k_eos_points<TERMS><<<(unsigned)((n + T - 1) / T), T>>>(fluid, with_prop, n, in, in + m, in + 2 * m, in + 3 * m, ddv,
+                                                          dtv, fb);
+  if (cudaGetLastError() != cudaSuccess) return CFD3D_ERR_CUDA;
+  if (packed) {
+    if (cudaMemcpy(stage, ddv, out * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
+    std::memcpy(dv, stage, b * NDV);
+    if (tv && with_prop) std::memcpy(tv, stage + NDV * m, b * 2);
+    return CFD3D_OK;
+  }
+  if (cudaMemcpy(dv, ddv, b * NDV, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
+  if (tv && with_prop && cudaMemcpy(tv, dtv, b * 2, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
+  return CFD3D_OK;
+}
+
+// As many points as the static buffer holds go through it; more through one allocation.
+// (200 points took 271 us with an allocation per array and 115 us through the buffer with a
+// copy per array; packed 77 us, 45 of them the kernel's.  4000 points 316 -> 133 us, 300000
+// points 2.88 -> 2.50 ms, of which the copy of the results to pageable memory is most.)
+template <bool TERMS>
+int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
+               const double* y2, double* dv, double* tv) {
+  if (n <= 0 || !p || !t || !y1 || !y2 || !dv || (fluid != 1 && fluid != 2) || ngas != 1) return CFD3D_ERR_ARG;
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return CFD3D_ERR_NODEVICE;
+  if (n <= CFD3D_EOS_NOALLOC_MAX) {
+    std::lock_guard<std::mutex> lock(g_eos_scratch_mu);
+    if (double* x = eos_scratch()) return eos_run<TERMS>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x);
+    cudaGetLastError();
+  }
+  double* x = nullptr;
+  if (cudaMalloc(&x, (1 + EOS_PER_POINT * (size_t)n) * 8) != cudaSuccess) return CFD3D_ERR_NOMEM;
+  const int rc = eos_run<TERMS>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x);
+  cudaFree(x);
+  return rc;
+}
+}  // namespace
+
+extern "C" {
+
+const char* cfd3d_last_error(const cfd3d_handle* h) { return h ? h->E.err.c_str() : "null handle"; }
+
+int cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
+                   const double* y2, double* dv, double* tv) {
+  return eos_points<false>(fluid, ngas, with_prop, n, p, t, y1, y2, dv, tv);
+}
+
 int cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t,
                            const double* y1, const double* y2, double* dv, double* tv) {
   if (n <= 0 || n > CFD3D_EOS_NOALLOC_MAX || !p || !t || !y1 || !y2 || !dv || (fluid != 1 && fluid != 2) ||
@@ -2492,36 +2540,9 @@ int cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const 
     return CFD3D_ERR_ARG;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return CFD3D_ERR_NODEVICE;
-  EosScratch* S = nullptr;
-  {
-    // set-up on the first call in a context: the buffer's device address there
-    std::lock_guard<std::mutex> lock(g_eos_scratch_mu);
-    unsigned long long ctx = 0;
-    if (!current_ctx_id(ctx)) return CFD3D_ERR_CUDA;
-    for (const ScratchSlot& sl : g_eos_scratch_slots)
-      if (ctx && sl.ctx == ctx) S = sl.ptr;
-    if (!S) {
-      // (with no context current yet, the lookup makes the device's primary context current)
-      void* ptr = nullptr;
-      if (cudaGetSymbolAddress(&ptr, g_eos_scratch) != cudaSuccess || !ptr) return CFD3D_ERR_CUDA;
-      if (!ctx && (!current_ctx_id(ctx) || !ctx)) return CFD3D_ERR_CUDA;
-      S = static_cast<EosScratch*>(ptr);
-      g_eos_scratch_slots.push_back({ctx, S});
-    }
-  }
-  const size_t b = (size_t)n * 8;
-  if (cudaMemcpy(S->p, p, b, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(S->t, t, b, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(S->y1, y1, b, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(S->y2, y2, b, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemset(&S->fallbacks, 0, sizeof(unsigned long long)) != cudaSuccess)
-    return CFD3D_ERR_CUDA;
-  k_eos_points<false><<<(unsigned)((n + 127) / 128), 128>>>(fluid, with_prop, n, S->p, S->t, S->y1, S->y2, S->dv, S->tv,
-                                                      &S->fallbacks);
-  if (cudaGetLastError() != cudaSuccess) return CFD3D_ERR_CUDA;
-  if (cudaMemcpy(dv, S->dv, b * NDV, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
-  if (tv && with_prop && cudaMemcpy(tv, S->tv, b * 2, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
-  return CFD3D_OK;
+  std::lock_guard<std::mutex> lock(g_eos_scratch_mu);
+  double* x = eos_scratch();
+  return x ? eos_run<false>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x) : CFD3D_ERR_CUDA;
 }
 
 int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {

@@ -141,7 +141,7 @@ EOS_NOALLOC_MAX = 4096   # CFD3D_EOS_NOALLOC_MAX
 
 def eos_eval_noalloc(p, t, y1, y2, fluid=2, prop=False):
     """eos_eval through the library's static device buffer (no device allocation);
-    at most EOS_NOALLOC_MAX points per call, calls on one device must not overlap."""
+    at most EOS_NOALLOC_MAX points per call."""
     p, t, y1, y2 = (np.ascontiguousarray(a, dtype=np.float64).ravel() for a in (p, t, y1, y2))
     n = p.size
     dv = np.zeros((n, 18))

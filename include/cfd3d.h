@@ -293,9 +293,10 @@ int  cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double 
                     const double *t, const double *y1, const double *y2, double *dv,
                     double *tv);
 
-/* cfd3d_eos_eval without any device allocation: the points pass through one static
- * device buffer of CFD3D_EOS_NOALLOC_MAX points (about 0.8 MB of each context that loads
- * the library's device code, held until the context ends) instead of cudaMalloc'd arrays.  No counterpart in the reference.  It serves
+/* cfd3d_eos_eval without any device allocation: the points pass through the static
+ * device buffer of CFD3D_EOS_NOALLOC_MAX points that cfd3d_eos_eval uses for as few (about
+ * 0.8 MB of each context that loads the library's device code, held until the context
+ * ends), never through an allocation.  No counterpart in the reference.  It serves
  * callers that cannot allocate device memory: a caller evaluating a few points while the
  * engine's iterations run on their own stream (cudaFree synchronises the whole device,
  * so cfd3d_eos_eval would wait for them), and a caller whose device memory is taken by
@@ -305,8 +306,7 @@ int  cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double 
  * one after cudaDeviceReset) looks up the buffer's device address, so make it before any
  * stream capture there.  Under lazy module loading (the CUDA default) that first call is
  * also when the buffer is reserved: make it while device memory is still free, or load
- * modules eagerly (CUDA_MODULE_LOADING=EAGER).  All calls on one device share the buffer:
- * calls must not overlap (serialise them across host threads). */
+ * modules eagerly (CUDA_MODULE_LOADING=EAGER).  Calls of several host threads take turns. */
 #define CFD3D_EOS_NOALLOC_MAX 4096
 int  cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const double *p,
                             const double *t, const double *y1, const double *y2, double *dv,
