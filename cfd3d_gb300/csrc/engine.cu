@@ -2600,6 +2600,8 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   CFD_CUDA(cudaStreamCreateWithFlags(&E.st, cudaStreamNonBlocking));
   CFD_CUDA(cudaStreamCreateWithFlags(&E.st2, cudaStreamNonBlocking));
   for (auto& e : E.pipe_ev) CFD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  for (auto& t : E.st_dir) CFD_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+  for (auto& e : E.dir_ev) CFD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   // device buffers
   const Par& c = E.par;
   const long long n = E.ncell;
@@ -2612,20 +2614,26 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   bool ok = alloc(E.d.pv, c.npv) && alloc(E.d.dv, NDV) && alloc(E.d.tv, std::max(c.ntv, 1)) &&
             alloc(E.d.gm, GM_GRD + c.ngrd) && alloc(E.d.res, c.npv) && alloc(E.d.icav, 4) && alloc(E.d.itt, 4) &&
             alloc(E.d.ocut, 1) && alloc(E.d.dt, 1) && alloc(E.d.rcav, 2) && alloc(E.d.qq, std::max(2 * c.npv * (c.nqq ? 1 : 0), 1)) &&
-            alloc(E.d.dqs, c.npv) && alloc(E.d.dcv, c.npv);
+            alloc(E.d.dqs, c.mixed && c.timemethod == 3 ? 0 : c.npv) && alloc(E.d.dcv, c.mixed ? 0 : c.npv);
   auto allocf = [&](float*& p, long long planes) -> bool {
     if (cudaMalloc(&p, (size_t)planes * n * 4) != cudaSuccess) return false;
     cudaMemset(p, 0, (size_t)planes * n * 4);
     return true;
   };
+  // The mixed form's face directions run beside one another up to 2 GB of face records: each
+  // kernel's start, end and last wave then overlap with another's.  Face stage in turn and
+  // beside: 0.192 and 0.074 ms at 16x12x10 cells, 0.80 and 0.65 at 128x64x64, 4.92 and 4.67
+  // on 24 blocks of 3.0 M cells, 15.4 and 15.1 at 14.2 M, where another 3 GB would be
+  // allocated and cleared for it.
+  if (c.mixed) E.face_slots = (3.0 * 2 * FREC_SIDE * 4.0 * (double)n <= 2e9) ? 3 : 1;
   if (c.mixed)
     ok = ok && allocf(E.d.pvf, c.npv) && allocf(E.d.fi32, 3 * c.npv) && allocf(E.d.fv32, (c.iturb == -3) ? 1 : 3 * c.npv) &&
-         allocf(E.d.frec, 2 * 12) && allocf(E.d.lqf, NLQ);
+         allocf(E.d.frec, E.face_slots * 2 * FREC_SIDE) && allocf(E.d.lqf, NLQ);
   if (c.mixed) {
     // lists of face states (two per face of a direction) and of cells
     const long long most = std::max({2 * E.nface[0], 2 * E.nface[1], 2 * E.nface[2], E.nint});
     E.d.mxcap = (int)std::min<long long>(most, 0x7fffffffll);
-    ok = ok && cudaMalloc(&E.d.mxl, (size_t)E.d.mxcap * MX_KINDS * sizeof(int)) == cudaSuccess &&
+    ok = ok && cudaMalloc(&E.d.mxl, (size_t)E.d.mxcap * MX_KINDS * E.face_slots * sizeof(int)) == cudaSuccess &&
          cudaMalloc(&E.d.mxn, MXN * sizeof(int)) == cudaSuccess;
   }
   else {
@@ -2824,6 +2832,8 @@ void cfd3d_destroy(cfd3d_handle* h) {
   for (auto e : h->ev) if (e) cudaEventDestroy(e);
   for (auto e : E.pipe_ev) if (e) cudaEventDestroy(e);
   if (E.st2) cudaStreamDestroy(E.st2);
+  for (auto e : E.dir_ev) if (e) cudaEventDestroy(e);
+  for (auto t : E.st_dir) if (t) cudaStreamDestroy(t);
   if (E.st) cudaStreamDestroy(E.st);
   delete h;
 }

@@ -265,6 +265,11 @@ struct Engine {
   static constexpr int MAX_PIPE = 16;
   cudaStream_t st = nullptr, st2 = nullptr;
   cudaEvent_t pipe_ev[MAX_PIPE + 2] = {};
+  // mixed form, small cases: the face stage's directions beside one another (the viscous
+  // fluxes on st2), each with its own scratch; 1 or 3
+  int face_slots = 1;
+  cudaStream_t st_dir[2] = {};
+  cudaEvent_t dir_ev[4] = {};
   cudaGraphExec_t graph = nullptr;
   int graph_ready = 0;
   int launches_per_iter = 0;

@@ -542,37 +542,52 @@ void launch_face_flux_mixed(const Engine& E, cudaStream_t s, int b0, int b1) {
   }
   const long long share = (long long)(b1 - b0) * std::max(nsm, 1) * 8 / std::max(nb, 1);
   k_shadow<<<(unsigned)std::max<long long>(share, 1), 256, 0, s>>>(E.d, E.par, g0, g1);
-  // the i faces from their 38-cell stencils, the j and k faces by columns (k_muscl_march)
-  // under MUSCL; then the clips and the face EOS
   const bool march = E.par.nmuscl > 0, visc = E.par.iturb != -3, sums = march && E.par.fluid != 1;
-  auto cols = [&](int q) { return (unsigned)(((c1[q] - c0[q]) * E.par.npv + 127) / 128); };
   // (the groups of the pipeline follow one another on s, so they can share lists and counters)
-  int* cnt = E.d.mxn;
-  if (sums) cudaMemsetAsync(cnt, 0, MXN_FACE * sizeof(int), s);
-  auto face_eos = [&](int q) {
-    if (!sums) return;
-    // grids that fill the GPU at most, and no more than every state listed needs
-    const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>((2 * (f1[q] - f0[q]) + 255) / 256, 4ll * nsm));
-    k_face_eos<MX_LIQ><<<g, 256, 0, s>>>(E.d, E.par, cnt + 3 * q);
-    k_face_eos<MX_META><<<g, 256, 0, s>>>(E.d, E.par, cnt + 3 * q);
-    k_face_eos<MX_STABLE><<<g, 256, 0, s>>>(E.d, E.par, cnt + 3 * q);
-  };
-  k_recon_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0], cnt);
-  face_eos(0);
-  k_flux_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0]);
-  if (visc) k_visc_mx<0><<<nblk(f1[0] - f0[0]), T, 0, s>>>(E.d, E.par, f0[0], f1[0]);
-  if (march) k_muscl_march<1><<<cols(1), 128, 0, s>>>(E.d, E.par, c0[1], c1[1]);
-  if (march) k_recon_mx<1, true><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1], cnt + 3);
-  else k_recon_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1], cnt + 3);
-  face_eos(1);
-  k_flux_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1]);
-  if (visc) k_visc_mx<1><<<nblk(f1[1] - f0[1]), T, 0, s>>>(E.d, E.par, f0[1], f1[1]);
-  if (march) k_muscl_march<2><<<cols(2), 128, 0, s>>>(E.d, E.par, c0[2], c1[2]);
-  if (march) k_recon_mx<2, true><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2], cnt + 6);
-  else k_recon_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2], cnt + 6);
-  face_eos(2);
-  k_flux_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2]);
-  if (visc) k_visc_mx<2><<<nblk(f1[2] - f0[2]), T, 0, s>>>(E.d, E.par, f0[2], f1[2]);
+  if (sums) cudaMemsetAsync(E.d.mxn, 0, MXN_FACE * sizeof(int), s);
+  // the directions beside one another where each has scratch of its own, otherwise in turn
+  const bool beside = E.face_slots == 3 && b0 == 0 && b1 == nb;
+  if (beside) {
+    cudaEventRecord(E.dir_ev[0], s);
+    for (cudaStream_t t : {E.st2, E.st_dir[0], E.st_dir[1]}) cudaStreamWaitEvent(t, E.dir_ev[0], 0);
+  }
+  // the i faces from their 38-cell stencils, the j and k faces by columns (k_muscl_march)
+  // under MUSCL; then the clips and the face EOS, and the fluxes
+  for (int q = 0; q < 3; ++q) {
+    cudaStream_t t = (beside && q > 0) ? E.st_dir[q - 1] : s;
+    DevPtr d = E.d;
+    int* cnt = d.mxn + MX_KINDS * q;
+    if (beside) {
+      d.frec += (long long)q * 2 * FREC_SIDE * E.ncell;
+      d.mxl += (long long)q * MX_KINDS * d.mxcap;
+    }
+    const unsigned nf = nblk(f1[q] - f0[q]), cols = (unsigned)(((c1[q] - c0[q]) * E.par.npv + 127) / 128);
+    if (march && q == 1) k_muscl_march<1><<<cols, 128, 0, t>>>(d, E.par, c0[q], c1[q]);
+    if (march && q == 2) k_muscl_march<2><<<cols, 128, 0, t>>>(d, E.par, c0[q], c1[q]);
+    using Recon = void (*)(DevPtr, Par, long long, long long, int*);
+    const Recon recon = (q == 0) ? k_recon_mx<0> : (q == 1) ? (march ? k_recon_mx<1, true> : k_recon_mx<1>)
+                                                            : (march ? k_recon_mx<2, true> : k_recon_mx<2>);
+    recon<<<nf, T, 0, t>>>(d, E.par, f0[q], f1[q], cnt);
+    if (sums) {
+      // grids that fill the GPU at most, and no more than every state listed needs
+      const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>((2 * (f1[q] - f0[q]) + 255) / 256, 4ll * nsm));
+      k_face_eos<MX_LIQ><<<g, 256, 0, t>>>(d, E.par, cnt);
+      k_face_eos<MX_META><<<g, 256, 0, t>>>(d, E.par, cnt);
+      k_face_eos<MX_STABLE><<<g, 256, 0, t>>>(d, E.par, cnt);
+    }
+    using Flux = void (*)(DevPtr, Par, long long, long long);
+    const Flux flux = (q == 0) ? k_flux_mx<0> : (q == 1) ? k_flux_mx<1> : k_flux_mx<2>;
+    const Flux vf = (q == 0) ? k_visc_mx<0> : (q == 1) ? k_visc_mx<1> : k_visc_mx<2>;
+    flux<<<nf, T, 0, t>>>(d, E.par, f0[q], f1[q]);
+    if (visc) vf<<<nf, T, 0, beside ? E.st2 : s>>>(d, E.par, f0[q], f1[q]);
+  }
+  if (beside) {
+    cudaStream_t t[3] = {E.st2, E.st_dir[0], E.st_dir[1]};
+    for (int q = 0; q < 3; ++q) {
+      cudaEventRecord(E.dir_ev[1 + q], t[q]);
+      cudaStreamWaitEvent(s, E.dir_ev[1 + q], 0);
+    }
+  }
 }
 
 }  // namespace cfd
