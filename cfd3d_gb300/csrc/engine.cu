@@ -1458,7 +1458,8 @@ __global__ void __launch_bounds__(4 * SW_CH) k_sweep_df(DevPtr d, Par c, long lo
 // steps after the one before it in i, j or k, where with done flags it started 18 later
 // plus a fence and a round trip to L2.  Both sweeps of an iteration: 1.03 -> 0.49 ms at
 // 128x64x64 cells, 0.22 -> 0.12 ms at 16x12x10, 1.15 -> 0.94 ms on 24 uneven blocks of 3.0 M
-// cells, 4.0 -> 3.6 ms on 8 blocks of 14.2 M.  (Three warps with a product each, the solution
+// cells, 4.0 -> 3.6 ms on 8 blocks of 14.2 M.  (Reading a step's records ahead of its wait
+// was slower, 3.77 ms there.)  (Three warps with a product each, the solution
 // in all of them, took 1.7 ms where one warp took 1.03.)
 // The needed tiles always hold earlier tickets, so the waits end; they are bounded as in the
 // FP64 form's dataflow sweep; `withhold` >= 0 names a tile whose contributions are never
@@ -1505,6 +1506,10 @@ __device__ __forceinline__ void st_entry(float* p, float x) {
   unsigned b = __float_as_uint(x);
   if (b == IN_UNSET) b = 0x7fc00000u;   // (a NaN all the same)
   asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" : : "l"(p), "r"(b) : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, unsigned bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+               : : "l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -1606,7 +1611,9 @@ __global__ void __launch_bounds__(TILE_T, 3) k_sweep_tile(DevPtr d, Par c, long 
     // ---- stage the tile's records (written by earlier launches): the common fields and
     // this sweep's faces and spectral radii
     if (lane == 0) {
-      // the previous tile's shared-memory reads (generic proxy) before the bulk writes
+      // the previous tile's shared-memory reads (of its stores, and generic ones) before the
+      // bulk writes
+      asm volatile("cp.async.bulk.wait_group.read 0;" : : : "memory");
       asm volatile("fence.proxy.async.shared::cta;" : : : "memory");
       mbar_expect(bar, TILE_B32);
       const float* rf = d.trf + (long long)tile * NTR * TILE_SLOTS;
@@ -1681,19 +1688,16 @@ __global__ void __launch_bounds__(TILE_T, 3) k_sweep_tile(DevPtr d, Par c, long 
         for (int v = 0; v < NPVM; ++v) y[v] = 0.0f;
         diag_solve_t<float>(npv, D, pv, dv, acc, y);
         // dq in FP32 for the products: own part + correction; the correction kept for the
-        // update, and (forward) dq* as the backward sweep's own part
+        // update (in the place of the cell's diagonal block) and (forward) dq* as the backward
+        // sweep's own part
         float dqf[NPVM];
-        const long long gq = (long long)tile * NPVM * TILE_SLOTS + sl;
-        float* ty = FWD ? d.tyf : d.tyb;
-        float* own = d.trf + ((long long)tile * NTR + TR_X) * TILE_SLOTS + sl;
 #pragma unroll
         for (int v = 0; v < NPVM; ++v) {
+          dqf[v] = 0.0f;
           if (v < npv) {
             dqf[v] = S32[(TR_X + v) * TILE_SLOTS + sl] + y[v];
-            ty[gq + (long long)v * TILE_SLOTS] = y[v];
-            if (FWD) own[v * TILE_SLOTS] = dqf[v];
-          } else {
-            dqf[v] = 0.0f;
+            S32[(TR_DIAG + v) * TILE_SLOTS + sl] = y[v];
+            if (FWD) S32[(TR_X + v) * TILE_SLOTS + sl] = dqf[v];
           }
         }
         // outgoing contributions: A+ dq through the cell's + faces (forward), -A- dq through
@@ -1725,7 +1729,18 @@ __global__ void __launch_bounds__(TILE_T, 3) k_sweep_tile(DevPtr d, Par c, long 
         for (int v = 0; v < NPVM; ++v) cj[v] = ck[v] = 0.0f;
       }
     }
+    // ---- the corrections and dq* out of shared memory, whole planes of the tile at once
+    // (stored cell by cell, each four bytes of a sector of its own, they were eight writes
+    // per sector in L2: both sweeps of 14.2 M cells 3.60 ms, so 3.40)
+    asm volatile("fence.proxy.async.shared::cta;" : : : "memory");
+    __syncwarp();
+    if (lane == 0 && staged) {
+      bulk_store((FWD ? d.tyf : d.tyb) + (long long)tile * NPVM * TILE_SLOTS, S32 + TR_DIAG * TILE_SLOTS, npv * TILE_SLOTS * 4);
+      if (FWD) bulk_store(d.trf + ((long long)tile * NTR + TR_X) * TILE_SLOTS, S32 + TR_X * TILE_SLOTS, npv * TILE_SLOTS * 4);
+      asm volatile("cp.async.bulk.commit_group;" : : : "memory");
+    }
   }
+  if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" : : : "memory");
 }
 
 using SweepTile = void (*)(DevPtr, Par, long long, int);
