@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) k_eos_liq(DevPtr d, Par c, const int* lis
 }
 
 template <bool META>
-__global__ void __launch_bounds__(256) k_eos_vap(DevPtr d, Par c, const int* cnt) {
+__device__ __forceinline__ void eos_vap(const DevPtr& d, const Par& c, const int* cnt) {
   const int* L;
   const int m = list_of(d, cnt, META ? MX_META : MX_STABLE, L);
   const long long n = d.ncell;
@@ -59,6 +59,11 @@ __global__ void __launch_bounds__(256) k_eos_vap(DevPtr d, Par c, const int* cnt
     S[ES_IV * n + g] = iv;
     S[ES_HV * n + g] = hv;
   }
+}
+
+__global__ void __launch_bounds__(256) k_eos_vap(DevPtr d, Par c, const int* cnt) {
+  if (blockIdx.y == 0) eos_vap<true>(d, c, cnt);
+  else eos_vap<false>(d, c, cnt);
 }
 
 __global__ void __launch_bounds__(256) k_eos_mix(DevPtr d, Par c, const int* list, const int* count) {
@@ -103,12 +108,11 @@ void launch_eos_cells(const Engine& E, cudaStream_t s, const int* list, const in
     int* cnt = d.mxn + MXN_FACE;
     cudaMemsetAsync(cnt, 0, MX_KINDS * sizeof(int), s);
     k_eos_liq<<<grid(32), 256, 0, s>>>(d, c, list, count, cnt);
-    k_eos_vap<true><<<grid(4), 256, 0, s>>>(d, c, cnt);
-    k_eos_vap<false><<<grid(4), 256, 0, s>>>(d, c, cnt);
+    k_eos_vap<<<dim3(grid(4), 2), 256, 0, s>>>(d, c, cnt);
   }
   k_eos_mix<<<grid(32), 256, 0, s>>>(d, c, list, count);
 }
 
-int eos_cells_launches(const Engine& E) { return E.par.fluid != 1 ? 4 : 1; }
+int eos_cells_launches(const Engine& E) { return E.par.fluid != 1 ? 3 : 1; }
 
 }  // namespace cfd
