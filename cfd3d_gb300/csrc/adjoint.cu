@@ -15,7 +15,8 @@
 //                     residual saw;
 //   the face kernels  per face (adjoint_face.cu): the inviscid and viscous flux and the
 //                     reconstruction reversed, from the forward kernels' face states;
-//   k_adj_cell        per cell: cavitation, SST and dual-time sources;
+//   k_adj_cell_plain  per cell: cavitation, SST and dual-time sources (k_adj_cell by dual
+//                     numbers where a configuration needs it);
 //   k_adj_ghost x3    the boundary program in reverse phase order (corners, edges, faces and
 //                     halos): each ghost's gradient pushed to the cells it was made from;
 //   k_adj_eos         per interior cell: the gradient with respect to its dv / tv pushed

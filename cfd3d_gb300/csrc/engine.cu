@@ -5,12 +5,14 @@
 // handle's stream, captured once into a CUDA graph and replayed:
 //
 //   k_timestep            local time step + global minimum   (timestep_module.f90:127-212)
-//   k_ghost x3            boundary program: faces+halos, edges, corners (bc_module.f90:1235-1396)
+//   k_ghost, k_ghost_eos x3   boundary program: faces+halos, edges, corners (bc_module.f90:1235-1396)
 //   face kernels          inviscid + viscous face fluxes (flux.cu, flux_mixed.cu; rhs_module.f90:282-538)
 //   k_rhs                 flux differences + cavitation / SST / dual-time sources (:540-642)
-//   k_sweep (fwd) x S     forward LU-SGS sweep, one launch per hyperplane i+j+k = s
-//   k_sweep (bwd) x S     backward sweep                          (update_module.f90:486-670)
-//   k_update              pv += dq, clipping, EOS with transport, residual partial sums (:672-700)
+//   k_sweep_df / k_sweep_tile   forward and backward LU-SGS sweep, one persistent launch each
+//                         (FP64 / mixed form; update_module.f90:486-670)
+//   k_update              pv += dq, clipping, residual partial sums (:672-700), and in the FP64
+//                         form the EOS with transport; in the mixed form the EOS follows in
+//                         passes of its own (eos_mixed.cu)
 //   k_eddy                SST eddy viscosity                      (:701-732)
 //   k_finish              residual norms, max location, solution time
 //
@@ -41,16 +43,23 @@ struct Cell {
 
 __device__ __forceinline__ void load_cell(const DevPtr& d, const Par& c, long long g, Cell& x) {
   const long long n = d.ncell;
-  for (int v = 0; v < c.npv; ++v) x.pv[v] = d.pv[v * n + g];
+#pragma unroll
+  for (int v = 0; v < NPVM; ++v) x.pv[v] = (v < c.npv) ? d.pv[v * n + g] : 0.0;
+#pragma unroll
   for (int v = 0; v < NDV; ++v) x.dv[v] = d.dv[v * n + g];
-  x.tv[0] = x.tv[1] = x.tv[2] = 0.0;
-  for (int v = 0; v < c.ntv; ++v) x.tv[v] = d.tv[v * n + g];
+#pragma unroll
+  for (int v = 0; v < 3; ++v) x.tv[v] = (v < c.ntv) ? d.tv[v * n + g] : 0.0;
 }
 __device__ __forceinline__ void store_cell(const DevPtr& d, const Par& c, long long g, const Cell& x) {
   const long long n = d.ncell;
-  for (int v = 0; v < c.npv; ++v) d.pv[v * n + g] = x.pv[v];
+#pragma unroll
+  for (int v = 0; v < NPVM; ++v)
+    if (v < c.npv) d.pv[v * n + g] = x.pv[v];
+#pragma unroll
   for (int v = 0; v < NDV; ++v) d.dv[v * n + g] = x.dv[v];
-  for (int v = 0; v < c.ntv; ++v) d.tv[v * n + g] = x.tv[v];
+#pragma unroll
+  for (int v = 0; v < 3; ++v)
+    if (v < c.ntv) d.tv[v * n + g] = x.tv[v];
 }
 
 // ------------------------------------------------------------------ pointwise EOS
@@ -435,34 +444,43 @@ __device__ __forceinline__ void ghost_eos(const DevPtr& d, const Par& c, double 
   else deteos(c.fluid, c.with_prop, p, t, y1, y2, dv, tv, &d.sc->snd2_fallbacks);
 }
 
-__global__ void k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int nops) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
+// A phase's copies and reflections: the ghost is its source cell with some primitives (and
+// tv(3)) changed.  What bounds it is the scattered planes' latency, so it is kept apart from
+// the ghosts that go through the EOS, whose code would leave it twelve warps per SM, and dv
+// passes through in two batches (at 6 or 12 CTAs per SM, or in batches of six, it was
+// slower).  The boundary stage in one kernel and so: 56 and 47 us at 16x12x10 cells, 85 and
+// 72 us at 128x64x64, 0.354 and 0.295 ms on 24 blocks of 3.0 M cells (halo runs of three
+// cells: partial sectors), 2.42 and 2.25 ms on 8 blocks of 14.2 M.
+__global__ void __launch_bounds__(128, 8) k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int nops) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nops) return;
-  const GhostOp op = ops[q];
+  const GhostOp& op = ops[q];
   const long long n = d.ncell;
-  Cell x;
+#pragma unroll
+  for (int b = 0; b < NDV; b += 9) {
+    double y[9];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) y[v] = d.dv[(b + v) * n + op.src];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) d.dv[(b + v) * n + op.dst] = y[v];
+  }
+  struct { double pv[NPVM], tv[3]; } x;
+#pragma unroll
+  for (int v = 0; v < NPVM; ++v) x.pv[v] = (v < c.npv) ? d.pv[v * n + op.src] : 0.0;
+#pragma unroll
+  for (int v = 0; v < 3; ++v) x.tv[v] = (v < c.ntv) ? d.tv[v * n + op.src] : 0.0;
   switch (op.kind) {
-    case G_COPY:
-    case G_EXTRAP:
-      load_cell(d, c, op.src, x);
-      store_cell(d, c, op.dst, x);
-      return;
     case G_WALL_VISCOUS:
-      load_cell(d, c, op.src, x);
       x.pv[1] = -x.pv[1]; x.pv[2] = -x.pv[2]; x.pv[3] = -x.pv[3];
-      store_cell(d, c, op.dst, x);
-      return;
+      break;
     case G_WALL_KW: {
-      load_cell(d, c, op.src, x);
       double vis_b = d.tv[op.bnd], rho_b = d.dv[op.bnd], y5 = d.gm[(GM_GRD + 4) * n + op.bnd];
       double om = 1600.0 * vis_b / rho_b / (y5 * y5) - x.pv[8];
       x.pv[1] = -x.pv[1]; x.pv[2] = -x.pv[2]; x.pv[3] = -x.pv[3]; x.pv[7] = -x.pv[7]; x.pv[8] = om;
       x.tv[2] = -x.tv[2];
-      store_cell(d, c, op.dst, x);
-      return;
+      break;
     }
     case G_SYMMETRY: {
-      load_cell(d, c, op.src, x);
       double nx[3];
       face_vec(d, op.fplane, op.fidx, nx);
       for (int v = 0; v < 3; ++v) nx[v] *= (double)op.fsign;
@@ -471,9 +489,96 @@ __global__ void k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int no
       x.pv[1] = 2.0 * (us - nx[0] * un) - x.pv[1];
       x.pv[2] = 2.0 * (vs - nx[1] * un) - x.pv[2];
       x.pv[3] = 2.0 * (ws - nx[2] * un) - x.pv[3];
-      store_cell(d, c, op.dst, x);
-      return;
+      break;
     }
+    case G_WALL_KE:
+      // bcwallviscouske (src/bc_module.f90:2324-2366): u, v, w, k, eps and mu_t reflected
+      x.pv[1] = -x.pv[1]; x.pv[2] = -x.pv[2]; x.pv[3] = -x.pv[3]; x.pv[7] = -x.pv[7]; x.pv[8] = -x.pv[8];
+      x.tv[2] = -x.tv[2];
+      break;
+    case G_CRWALL:
+    case G_CRWALL_KW: {
+      // bccounterrotatingwallviscous (src/bc_module.f90:3516-3580) and its k-omega variant
+      // (:3654-3731): u = -u_mirror - 2 gridvel; k-omega: k and mu_t reflected, omega the
+      // mirror's, the reference's wall value being computed and then discarded
+      double gv[3] = {0.0, 0.0, 0.0};
+      if (c.rot) face_gridvel(d, c, op.bnd, op.gcell, gv);
+      for (int q3 = 0; q3 < 3; ++q3) x.pv[1 + q3] = -x.pv[1 + q3] - 2.0 * gv[q3];
+      if (op.kind == G_CRWALL_KW) { x.pv[7] = -x.pv[7]; x.tv[2] = -x.tv[2]; }
+      break;
+    }
+    case G_CRWALL_INV: {
+      // bccounterrotatingwallinviscid (:3733-3810): the symmetry reflection of the boundary
+      // cell's velocity less the face's grid velocity
+      double nx[3];
+      face_vec(d, op.fplane, op.fidx, nx);
+      for (int v = 0; v < 3; ++v) nx[v] *= (double)op.fsign;
+      double gv[3] = {0.0, 0.0, 0.0};
+      if (c.rot) face_gridvel(d, c, op.bnd, op.gcell, gv);
+      const double us = d.pv[n + op.bnd], vs = d.pv[2 * n + op.bnd], ws = d.pv[3 * n + op.bnd];
+      const double un = (us * nx[0] + vs * nx[1] + ws * nx[2]) / (nx[0] * nx[0] + nx[1] * nx[1] + nx[2] * nx[2]);
+      x.pv[1] = 2.0 * (us - nx[0] * un - gv[0]) - x.pv[1];
+      x.pv[2] = 2.0 * (vs - nx[1] * un - gv[1]) - x.pv[2];
+      x.pv[3] = 2.0 * (ws - nx[2] * un - gv[2]) - x.pv[3];
+      break;
+    }
+    case G_HFWALL_KW: {
+      // bcheatfluxwallviscouskw (src/bc_module.f90:4184-4273): u, v, w, k reflected, the
+      // wall temperature from the heat flux through the boundary cell, the SST omega wall
+      // value.  The routine's EOS call takes the mirror's state, so the ghost keeps the
+      // mirror's dv and tv(1:2); tv(3) reflects.
+      const long long b = op.bnd;
+      const double hf = heatflux_at(d.hft + op.pad, bc_time(d, c));
+      const double yb = d.gm[(GM_GRD + 4) * n + b], mub = d.tv[b], kb = d.tv[n + b];
+      const double ub = d.pv[n + b], vb = d.pv[2 * n + b], wb = d.pv[3 * n + b];
+      x.pv[1] = -x.pv[1]; x.pv[2] = -x.pv[2]; x.pv[3] = -x.pv[3]; x.pv[7] = -x.pv[7];
+      x.pv[4] = 2.0 * ((hf * yb + 0.5 * mub * (ub * ub + vb * vb + wb * wb)) / kb + d.pv[4 * n + b]) - x.pv[4];
+      x.pv[8] = 1600.0 * mub / d.dv[b] / (yb * yb) - x.pv[8];
+      x.tv[2] = -x.tv[2];
+      break;
+    }
+    case G_WALLWALL:
+    case G_WALLWALL_KW4:
+    case G_WALLWALL_KW8: {
+      double ppv[NPVM];
+#pragma unroll
+      for (int v = 0; v < NPVM; ++v) ppv[v] = -x.pv[v];
+      for (int m = 0; m < 6; ++m) {
+        if (op.nb[m] < 0) break;
+#pragma unroll
+        for (int v = 0; v < NPVM; ++v)
+          if (v < c.npv) ppv[v] -= d.pv[v * n + op.nb[m]];
+      }
+      x.pv[1] = ppv[1]; x.pv[2] = ppv[2]; x.pv[3] = ppv[3];
+      if (op.kind == G_WALLWALL) {
+        if (c.npv > 7) { x.pv[7] = ppv[7]; x.pv[8] = ppv[8]; }
+      } else {
+        double y5 = d.gm[(GM_GRD + 4) * n + op.src];
+        double var = 800.0 * x.tv[0] / d.dv[op.src] / (y5 * y5);
+        x.pv[7] = ppv[7];
+        x.pv[8] = ((op.kind == G_WALLWALL_KW8) ? 8.0 : 4.0) * var + ppv[8];
+      }
+      break;
+    }
+    default:   // G_COPY, G_EXTRAP
+      break;
+  }
+#pragma unroll
+  for (int v = 0; v < NPVM; ++v)
+    if (v < c.npv) d.pv[v * n + op.dst] = x.pv[v];
+#pragma unroll
+  for (int v = 0; v < 3; ++v)
+    if (v < c.ntv) d.tv[v * n + op.dst] = x.tv[v];
+}
+
+// A phase's ghosts that go through the EOS
+__global__ void __launch_bounds__(64) k_ghost_eos(DevPtr d, Par c, const GhostOp* __restrict__ ops, int nops) {
+  int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nops) return;
+  const GhostOp op = ops[q];
+  const long long n = d.ncell;
+  Cell x;
+  switch (op.kind) {
     case G_FARFIELD:
     case G_INFLOW_SUB:
     case G_OUTFLOW_SUB:
@@ -496,13 +601,6 @@ __global__ void k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int no
       store_cell(d, c, op.dst, x);
       return;
     }
-    case G_WALL_KE:
-      // bcwallviscouske (src/bc_module.f90:2324-2366): u, v, w, k, eps and mu_t reflected
-      load_cell(d, c, op.src, x);
-      x.pv[1] = -x.pv[1]; x.pv[2] = -x.pv[2]; x.pv[3] = -x.pv[3]; x.pv[7] = -x.pv[7]; x.pv[8] = -x.pv[8];
-      x.tv[2] = -x.tv[2];
-      store_cell(d, c, op.dst, x);
-      return;
     case G_TOTALP: {
       // bctotalpressurein's ghost (:3398-3505): p and T from the patch's Newton solve, the
       // normal inflow speed |u_avg|, y1, k, omega from the free stream -- and y2 reflected
@@ -529,53 +627,6 @@ __global__ void k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int no
       store_cell(d, c, op.dst, x);
       return;
     }
-    case G_CRWALL:
-    case G_CRWALL_KW: {
-      // bccounterrotatingwallviscous (src/bc_module.f90:3516-3580) and its k-omega variant
-      // (:3654-3731): u = -u_mirror - 2 gridvel; k-omega: k and mu_t reflected, omega the
-      // mirror's, the reference's wall value being computed and then discarded
-      load_cell(d, c, op.src, x);
-      double gv[3] = {0.0, 0.0, 0.0};
-      if (c.rot) face_gridvel(d, c, op.bnd, op.gcell, gv);
-      for (int q3 = 0; q3 < 3; ++q3) x.pv[1 + q3] = -x.pv[1 + q3] - 2.0 * gv[q3];
-      if (op.kind == G_CRWALL_KW) { x.pv[7] = -x.pv[7]; x.tv[2] = -x.tv[2]; }
-      store_cell(d, c, op.dst, x);
-      return;
-    }
-    case G_CRWALL_INV: {
-      // bccounterrotatingwallinviscid (:3733-3810): the symmetry reflection of the boundary
-      // cell's velocity less the face's grid velocity
-      load_cell(d, c, op.src, x);
-      double nx[3];
-      face_vec(d, op.fplane, op.fidx, nx);
-      for (int v = 0; v < 3; ++v) nx[v] *= (double)op.fsign;
-      double gv[3] = {0.0, 0.0, 0.0};
-      if (c.rot) face_gridvel(d, c, op.bnd, op.gcell, gv);
-      const double us = d.pv[n + op.bnd], vs = d.pv[2 * n + op.bnd], ws = d.pv[3 * n + op.bnd];
-      const double un = (us * nx[0] + vs * nx[1] + ws * nx[2]) / (nx[0] * nx[0] + nx[1] * nx[1] + nx[2] * nx[2]);
-      x.pv[1] = 2.0 * (us - nx[0] * un - gv[0]) - x.pv[1];
-      x.pv[2] = 2.0 * (vs - nx[1] * un - gv[1]) - x.pv[2];
-      x.pv[3] = 2.0 * (ws - nx[2] * un - gv[2]) - x.pv[3];
-      store_cell(d, c, op.dst, x);
-      return;
-    }
-    case G_HFWALL_KW: {
-      // bcheatfluxwallviscouskw (src/bc_module.f90:4184-4273): u, v, w, k reflected, the
-      // wall temperature from the heat flux through the boundary cell, the SST omega wall
-      // value.  The routine's EOS call takes the mirror's state, so the ghost keeps the
-      // mirror's dv and tv(1:2); tv(3) reflects.
-      load_cell(d, c, op.src, x);
-      const long long b = op.bnd;
-      const double hf = heatflux_at(d.hft + op.pad, bc_time(d, c));
-      const double yb = d.gm[(GM_GRD + 4) * n + b], mub = d.tv[b], kb = d.tv[n + b];
-      const double ub = d.pv[n + b], vb = d.pv[2 * n + b], wb = d.pv[3 * n + b];
-      x.pv[1] = -x.pv[1]; x.pv[2] = -x.pv[2]; x.pv[3] = -x.pv[3]; x.pv[7] = -x.pv[7];
-      x.pv[4] = 2.0 * ((hf * yb + 0.5 * mub * (ub * ub + vb * vb + wb * wb)) / kb + d.pv[4 * n + b]) - x.pv[4];
-      x.pv[8] = 1600.0 * mub / d.dv[b] / (yb * yb) - x.pv[8];
-      x.tv[2] = -x.tv[2];
-      store_cell(d, c, op.dst, x);
-      return;
-    }
     case G_MASSFLOW_IN: {
       // bcmassflowratein (:3812-4012) with the rate 0 its construct sets: the inflow speed
       // m / (rho A) is 0, so u = 2 (0 - gridvel) - u_mirror; T, y1, y2, k, omega from the
@@ -591,28 +642,6 @@ __global__ void k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int no
       pv[5] = fmin(fmax(pv[5], 0.0), 1.0);
       pv[6] = fmin(fmax(pv[6], 0.0), 1.0);
       ghost_eos(d, c, pv[0] + bp[0], pv[4], pv[5], pv[6], x.dv, x.tv);
-      store_cell(d, c, op.dst, x);
-      return;
-    }
-    case G_WALLWALL:
-    case G_WALLWALL_KW4:
-    case G_WALLWALL_KW8: {
-      load_cell(d, c, op.src, x);
-      double ppv[NPVM];
-      for (int v = 0; v < c.npv; ++v) ppv[v] = -x.pv[v];
-      for (int m = 0; m < 6; ++m) {
-        if (op.nb[m] < 0) break;
-        for (int v = 0; v < c.npv; ++v) ppv[v] -= d.pv[v * n + op.nb[m]];
-      }
-      x.pv[1] = ppv[1]; x.pv[2] = ppv[2]; x.pv[3] = ppv[3];
-      if (op.kind == G_WALLWALL) {
-        if (c.npv > 7) { x.pv[7] = ppv[7]; x.pv[8] = ppv[8]; }
-      } else {
-        double y5 = d.gm[(GM_GRD + 4) * n + op.src];
-        double var = 800.0 * x.tv[0] / x.dv[0] / (y5 * y5);
-        x.pv[7] = ppv[7];
-        x.pv[8] = ((op.kind == G_WALLWALL_KW8) ? 8.0 : 4.0) * var + ppv[8];
-      }
       store_cell(d, c, op.dst, x);
       return;
     }
@@ -2156,6 +2185,19 @@ int face_rhs_launches(const Engine& E) {
   return ng * (8 + (c.nmuscl > 0 ? 2 : 0) + (c.nmuscl > 0 && c.fluid != 1 ? 9 : 0) + (c.iturb != -3 ? 3 : 0));
 }
 
+// one phase of the boundary program: its copies and reflections, and beside them on st2 the
+// ghosts that go through the EOS
+int launch_ghosts(const Engine& E, cudaStream_t s, int p) {
+  const int ne = E.nops_eos[p], n0 = E.nops[p] - ne;
+  const bool both = ne && n0;
+  cudaStream_t t = both ? E.st2 : s;
+  if (both) { cudaEventRecord(E.dir_ev[0], s); cudaStreamWaitEvent(t, E.dir_ev[0], 0); }
+  if (ne) k_ghost_eos<<<nblk_of(ne, 64), 64, 0, t>>>(E.d, E.par, E.d_ops[p] + n0, ne);
+  if (n0) k_ghost<<<nblk_of(n0, 128), 128, 0, s>>>(E.d, E.par, E.d_ops[p], n0);
+  if (both) { cudaEventRecord(E.dir_ev[1], t); cudaStreamWaitEvent(s, E.dir_ev[1], 0); }
+  return (ne > 0) + (n0 > 0);
+}
+
 // The boundary program -- the total-pressure pools, then faces + halos, edges, corners -- and,
 // with the surface-tension source, calvfg and setbc_vfg after it, as timeinteg calls them
 // (src/update_module.f90:240-243, 359-362, 479-482).  Returns the number of launches.
@@ -2165,7 +2207,7 @@ int launch_boundary(const Engine& E, cudaStream_t s) {
   int n = 0;
   if (d.ntp) { k_totalp<<<d.ntp, 128, 0, s>>>(d, c); ++n; }
   for (int p = 0; p < 3; ++p)
-    if (E.nops[p]) { k_ghost<<<nblk_of(E.nops[p], 128), 128, 0, s>>>(d, c, E.d_ops[p], E.nops[p]); ++n; }
+    n += launch_ghosts(E, s, p);
   if (c.csf) {
     k_vf<<<nblk_of(E.ncell, 256), 256, 0, s>>>(d);
     k_vfg<<<nblk_of(E.ncell, 256), 256, 0, s>>>(d);
@@ -3465,7 +3507,7 @@ int cfd3d_residual_vjp(cfd3d_handle* h, const double* cot, double* g_state, doub
   }
   // the forward boundary program: the ghost values the residual sees
   for (int p = 0; p < 3; ++p)
-    if (E.nops[p]) k_ghost<<<nblk_of(E.nops[p], 128), 128, 0, E.st>>>(E.d, c, E.d_ops[p], E.nops[p]);
+    launch_ghosts(E, E.st, p);
   if ((rc = adjoint_launch(E))) return rc;
   CFD_CUDA(cudaStreamSynchronize(E.st));
   CFD_CUDA(cudaGetLastError());

@@ -43,6 +43,12 @@ __host__ __device__ inline int ghost_ff_mode(int kind) {
   return kind == G_INFLOW_SUB ? 3 : kind == G_OUTFLOW_SUB ? 1 : kind == G_INFLOW_SUP ? 2 : 0;
 }
 
+// the kinds whose ghost state goes through the EOS
+inline bool ghost_needs_eos(int kind) {
+  return kind == G_FARFIELD || ghost_ff_mode(kind) || kind == G_TOTALP || kind == G_MASSFLOW_IN ||
+         kind == G_NOWALL3 || kind == G_NOWALL7;
+}
+
 // one ghost cell write of the compiled boundary program
 struct GhostOp {
   int kind;
@@ -239,7 +245,7 @@ struct Engine {
   DevPtr d{};
   // ghost program: phase 0 faces + halos, 1 edges, 2 corners
   GhostOp* d_ops[3] = {nullptr, nullptr, nullptr};
-  int nops[3] = {0, 0, 0};
+  int nops[3] = {0, 0, 0}, nops_eos[3] = {0, 0, 0};   // (the last nops_eos of a phase's go through the EOS)
   double* d_hft = nullptr;   // heat-flux histories (d.hft), null without heat-flux walls
   double* d_grav = nullptr;  // gravity history (d.grav), null without gravity
   int* d_tp_off = nullptr;

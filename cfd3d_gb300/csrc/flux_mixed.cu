@@ -2,10 +2,12 @@
 //
 //   k_shadow          FP32 gauge shadow pvf of every padded cell, after the boundary program,
 //                     and the cell's EOS state as the base of face-state expansions (lqf)
-//   k_recon_mx<DIR>   per face: MUSCL / MLP on pvf, clips, face-state rho and h (FP64
-//                     mixture of phases from df64 IF97 sums, or for a vapour-free state
-//                     near its cell the liquid by first-order expansion), written to the
-//                     face record frec
+//   k_recon_mx<DIR>   per face: MUSCL / MLP on pvf (the j and k faces' by columns,
+//                     k_muscl_march), clips, for a vapour-free state near its cell the
+//                     liquid's rho and h by first-order expansion, written to the face record
+//                     frec; other states listed for
+//   k_face_eos<KIND>  rho and h of the listed states (FP64 mixture of phases from df64 IF97
+//                     sums)
 //   k_flux_mx<DIR>    per face: FP32 Roe-average sound speed, inviscid flux with FP64
 //                     leading-order terms; stores F - Phi.n dl in FP32
 //   k_visc_mx<DIR>    per face: the FP32 viscous flux

@@ -535,7 +535,7 @@ int wall_kind(const Par& c) {
 
 bool setup_ghost_program(Engine& E, const cfd3d_block_desc* blocks, int nblocks) {
   const Par& c = E.par;
-  std::vector<GhostOp> ops[3];
+  std::vector<GhostOp> ops[3], eos_ops[3];
   std::vector<double> hft;   // heat-flux histories
   // total-pressure inlets: per pool 4 ints per face cell.  The reference reduces each inlet's
   // averages over the communicator of every rank carrying one (bc_comm_world, icolor 12,
@@ -697,7 +697,7 @@ bool setup_ghost_program(Engine& E, const cfd3d_block_desc* blocks, int nblocks)
               if (skip_zero_nb && nb[0] == 0 && nb[1] == 0 && nb[2] == 0) continue;
               op.nb[q2++] = gi(nb[0] + bi.dir[0] * i, nb[1] + bi.dir[1] * j, nb[2] + bi.dir[2] * k);
             }
-            ops[phase].push_back(op);
+            (ghost_needs_eos(op.kind) ? eos_ops : ops)[phase].push_back(op);
           }
     };
     for (auto& bi : bcs) emit(bi, 0, 0, false);
@@ -836,7 +836,9 @@ bool setup_ghost_program(Engine& E, const cfd3d_block_desc* blocks, int nblocks)
     }
   }
   for (int p = 0; p < 3; ++p) {
+    ops[p].insert(ops[p].end(), eos_ops[p].begin(), eos_ops[p].end());
     E.nops[p] = (int)ops[p].size();
+    E.nops_eos[p] = (int)eos_ops[p].size();
     if (E.nops[p] == 0) continue;
     if (cudaMalloc(&E.d_ops[p], ops[p].size() * sizeof(GhostOp)) != cudaSuccess) { E.err = "cudaMalloc ghost ops"; return false; }
     cudaMemcpy(E.d_ops[p], ops[p].data(), ops[p].size() * sizeof(GhostOp), cudaMemcpyHostToDevice);
