@@ -50,9 +50,9 @@ UNIT = "Mcell-iter/s"
 # DRAM bytes per cell of one k_rhs launch, dram__bytes_read.sum + dram__bytes_write.sum
 # of a one-pass ncu capture of the mixed form on the large case itself (14155776 cells, the
 # launch list of one pseudo-iteration), divided by the cells
-RHS_TRAFFIC_PER_CELL = (19.984210e9 + 11.177800e9) / 14155776
-# the same for the whole pseudo-iteration: dram read + write summed over its 22 launches
-ITER_TRAFFIC_PER_CELL = (72.270140e9 + 33.714040e9) / 14155776
+RHS_TRAFFIC_PER_CELL = (15.147836e9 + 8.649704e9) / 14155776
+# the same for the whole pseudo-iteration: dram read + write summed over its 35 launches
+ITER_TRAFFIC_PER_CELL = (66.336343e9 + 29.794348e9) / 14155776
 
 
 def algorithmic_bytes(cfg):
@@ -68,11 +68,11 @@ def rhs_bytes(cfg, mixed):
     """Algorithmic bytes per cell of the residual kernel k_rhs in the LU-SGS iteration (each
     datum once per cell).  FP64 form -- reads: the cell's + face fluxes (inviscid and
     viscous), pv, dv, tv, its + face vectors, volume and wall distance, the BDF history, dt;
-    writes: the residual, icav, itt, the omega bound, rcav and the 66-value FP64 sweep
+    writes: the residual, icav, itt, the omega bound, rcav and the 61-value FP64 sweep
     record.  Mixed form -- reads: the FP32 fluxes, pv, dv, tv, the volume, the BDF history,
     dt, the free-stream closure, the FP32 shadow of the SST variables and the FP32 metrics
-    (+ face vectors, volume, wall distance); writes: the omega bound, rcav, the 74-value FP32
-    tile record and the FP32 own part x0 (the residual, icav and itt stay in registers)."""
+    (+ face vectors, volume, wall distance); writes: the omega bound, rcav, 56 of the FP32
+    tile record's values and the FP32 own part x0 (the residual, icav and itt stay in registers)."""
     from cfd3d_gb300.abi import sizes
     npv, ntv, nqq, ngrd = sizes(cfg)
     vis = cfg.get("iturb", 0) != -3
@@ -81,11 +81,11 @@ def rhs_bytes(cfg, mixed):
     ndv = 18
     if not mixed:
         rd = 3 * (2 if vis else 1) * npv * 8 + 8 * npv + 8 * ndv + 8 * ntv + 8 * (9 + 2) + 8 * nqq * npv + 8
-        wr = 8 * npv + 8 * (4 + 4 + 1 + 2) + 8 * 66
+        wr = 8 * npv + 8 * (4 + 4 + 1 + 2) + 8 * 61
         return rd + wr
     rd = (3 * (2 if vis else 1) * npv * 4 + 8 * npv + 8 * ndv + 8 * ntv + 8 + 8 * nqq * npv + 8 + 8 * npv
           + (4 * 5 if sst else 0) + 4 * (9 + 2))
-    wr = (8 if sst else 0) + (16 if cav else 0) + 4 * 74 + 4 * npv
+    wr = (8 if sst else 0) + (16 if cav else 0) + 4 * 56 + 4 * npv
     return rd + wr
 
 
