@@ -63,20 +63,82 @@ __device__ __forceinline__ void store_cell(const DevPtr& d, const Par& c, long l
 }
 
 // ------------------------------------------------------------------ pointwise EOS
-// TERMS: the Gibbs sums term by term (deteos_t, the adjoint's), for the free-stream constants:
-// the mixed form's stored flux deviations are taken from them, so they keep the bits that
+// The Gibbs sums term by term (deteos_t, the adjoint's), for the free-stream constants: the
+// mixed form's stored flux deviations are taken from them, so they keep the bits that
 // checkpoints and earlier runs had
-template <bool TERMS>
-__global__ void k_eos_points(int fluid, int with_prop, long long n, const double* __restrict__ p,
-                             const double* __restrict__ t, const double* __restrict__ y1,
-                             const double* __restrict__ y2, double* __restrict__ dv, double* __restrict__ tv,
-                             unsigned long long* fb) {
+__global__ void k_eos_terms(int fluid, int with_prop, long long n, const double* __restrict__ p,
+                            const double* __restrict__ t, const double* __restrict__ y1,
+                            const double* __restrict__ y2, double* __restrict__ dv, double* __restrict__ tv) {
   long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n) return;
   double d[NDV], tt[2] = {0.0, 0.0};
-  if constexpr (TERMS) deteos_t<double>(fluid, with_prop, p[q], t[q], y1[q], y2[q], d, tt);
-  else deteos(fluid, with_prop, p[q], t[q], y1[q], y2[q], d, tt, fb);
+  deteos_t<double>(fluid, with_prop, p[q], t[q], y1[q], y2[q], d, tt);
   for (int v = 0; v < NDV; ++v) dv[NDV * q + v] = d[v];
+  if (tv) { tv[2 * q] = tt[0]; tv[2 * q + 1] = tt[1]; }
+}
+
+// deteos at n points.  What bounds it for few points is one warp's FP64 instructions, one per
+// 64 clocks: two warps share 32 points, the liquid with its transport properties on one, the
+// vapour on the other, the mixture on the first.  (A call of 200 points with one warp's chain
+// and so: 77 and 64 us; 4000 points 133 and 114 us; 300000 points the same.)
+__global__ void __launch_bounds__(64) k_eos_points(int fluid, int with_prop, long long n, const double* __restrict__ p,
+                                                   const double* __restrict__ t, const double* __restrict__ y1,
+                                                   const double* __restrict__ y2, double* __restrict__ dv,
+                                                   double* __restrict__ tv, unsigned long long* fb) {
+  __shared__ double s_v[9][32];
+  const int lane = threadIdx.x & 31;
+  const bool vapour = threadIdx.x >= 32;
+  const long long q = blockIdx.x * 32ll + lane;
+  const bool live = q < n;
+  Phase<double> l;
+  double ir[3], lv = 0.0, lc = 0.0, P = 0.0, T = 0.0, it = 0.0, pi1 = 0.0;
+  if (live) {
+    P = p[q];
+    T = t[q];
+    if (fluid != 1) { it = 1.0 / T; pi1 = 1.0e6 / P; }
+    if (!vapour) {
+      if (fluid == 1) {
+        stiffened(P, T, l);
+        ir[0] = 1.0 / l.rho;
+        if (with_prop) { lv = stiffened_vis(T); lc = 4598.0 * lv; }
+      } else {
+        if97_liquid<true>(P, T, it, l, ir[0]);
+        if (with_prop) iapws_transport(T, l.rho, lv, lc);
+      }
+    } else {
+      Phase<double> v;
+      double irv, vv = 0.0, vc = 0.0;
+      if (fluid == 1) {
+        ideal_gas(P, T, v);
+        irv = 1.0 / v.rho;
+        if (with_prop) { vv = ideal_vis(T); vc = 1395.333333 * vv; }
+      } else {
+        if97_vapour<true>(P, T, pi1, it, above_psat(P, T), v, irv);
+        if (with_prop) iapws_transport(T, v.rho, vv, vc);
+      }
+      const double x[9] = {v.rho, v.h, v.drdp, v.drdt, v.dhdp, v.dhdt, irv, vv, vc};
+#pragma unroll
+      for (int m = 0; m < 9; ++m) s_v[m][lane] = x[m];
+    }
+  }
+  __syncthreads();
+  if (vapour || !live) return;
+  Phase<double> v, g;
+  v.rho = s_v[0][lane]; v.h = s_v[1][lane]; v.drdp = s_v[2][lane];
+  v.drdt = s_v[3][lane]; v.dhdp = s_v[4][lane]; v.dhdt = s_v[5][lane];
+  ir[1] = s_v[6][lane];
+  if (fluid == 1) {
+    ideal_gas(P, T, g);
+    ir[2] = ir[1];
+  } else {
+    gas_phase(P, T, it, pi1, g, ir[2]);
+  }
+  double d[NDV];
+  const double a = y1[q], b = y2[q];
+  mixture<double>(l, v, g, a, b, d, fb, ir);
+  for (int m = 0; m < NDV; ++m) dv[NDV * q + m] = d[m];
+  double tt[2] = {0.0, 0.0};
+  if (with_prop) mixture_transport(T, a, b, lv, lc, s_v[7][lane], s_v[8][lane], ir, d[0], tt);
   if (tv) { tv[2 * q] = tt[0]; tv[2 * q + 1] = tt[1]; }
 }
 
@@ -2541,11 +2603,10 @@ int eos_run(int fluid, int with_prop, int64_t n, const double* p, const double* 
       if (cudaMemcpy(in + q * m, src[q], b, cudaMemcpyHostToDevice) != cudaSuccess) return CFD3D_ERR_CUDA;
     if (cudaMemset(fb, 0, 8) != cudaSuccess) return CFD3D_ERR_CUDA;
   }
-  // a warp's FP64 instructions follow one another at the pace of its SM's pipe: few points
-  // are spread over the SMs, a warp each
-  const int T = n <= 16384 ? 32 : 128;
-  k_eos_points<TERMS><<<(unsigned)((n + T - 1) / T), T>>>(fluid, with_prop, n, in, in + m, in + 2 * m, in + 3 * m, ddv,
-                                                          dtv, fb);
+  if (TERMS)
+    k_eos_terms<<<(unsigned)((n + 31) / 32), 32>>>(fluid, with_prop, n, in, in + m, in + 2 * m, in + 3 * m, ddv, dtv);
+  else
+    k_eos_points<<<(unsigned)((n + 31) / 32), 64>>>(fluid, with_prop, n, in, in + m, in + 2 * m, in + 3 * m, ddv, dtv, fb);
   if (cudaGetLastError() != cudaSuccess) return CFD3D_ERR_CUDA;
   if (packed) {
     if (cudaMemcpy(stage, ddv, out * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
@@ -2560,8 +2621,9 @@ int eos_run(int fluid, int with_prop, int64_t n, const double* p, const double* 
 
 // As many points as the static buffer holds go through it; more through one allocation.
 // (200 points took 271 us with an allocation per array and 115 us through the buffer with a
-// copy per array; packed 77 us, 45 of them the kernel's.  4000 points 316 -> 133 us, 300000
-// points 2.88 -> 2.50 ms, of which the copy of the results to pageable memory is most.)
+// copy per array; packed, and on two warps, 64 us, some 33 of them the kernel's.  4000 points
+// 316 -> 114 us, 300000 points 2.88 -> 2.49 ms, of which the copy of the results to pageable
+// memory is most.)
 template <bool TERMS>
 int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,
                const double* y2, double* dv, double* tv) {

@@ -260,6 +260,18 @@ static __device__ __noinline__ void vapour_inv_call(double p, double t, bool met
   vapour_inv_df64(df64(p), df64(t), meta, iv, hv);
 }
 
+// the gas with its reciprocal density, from 1/t and 1e6/p: rho = p r1 / t
+__device__ __forceinline__ void gas_phase(double p, double t, double it, double pi1, Phase<double>& g, double& ir) {
+  const double r1 = 0.00348383500557;
+  ir = t * pi1 * (1.0e-6 / r1);
+  g.h = 1004.64 * t;
+  g.rho = p * r1 * it;
+  g.drdp = r1 * it;
+  g.drdt = -(g.rho * it);
+  g.dhdp = 0.0;
+  g.dhdt = 1004.64;
+}
+
 // Phase properties of liquid, vapour and gas in FP64, with their reciprocal densities ir[3].
 // FULL = false evaluates only ir and h.  The metastable branch test p > p_sat(T) is taken as
 // the FP64 comparison in both forms so that they select the same term set.
@@ -279,15 +291,7 @@ __device__ __forceinline__ void phases(int fluid, double p, double t, Phase<doub
   }
   const double it = 1.0 / t, pi1 = 1.0e6 / p;
   if97_liquid<FULL>(p, t, it, l, ir[0]);
-  // the gas: rho = p r1 / t
-  const double r1 = 0.00348383500557;
-  ir[2] = t * pi1 * (1.0e-6 / r1);
-  g.h = 1004.64 * t;
-  g.rho = p * r1 * it;
-  g.drdp = r1 * it;
-  g.drdt = -(g.rho * it);
-  g.dhdp = 0.0;
-  g.dhdt = 1004.64;
+  gas_phase(p, t, it, pi1, g, ir[2]);
   if (!vap) {
     v.rho = 1.0; v.h = 0.0; v.drdp = 0.0; v.drdt = 0.0; v.dhdp = 0.0; v.dhdt = 1.0;
     ir[1] = 1.0;
@@ -439,6 +443,16 @@ __device__ __forceinline__ void eos_rho_h(int fluid, double p, double t, double 
   h = yl * l.h + y1 * v.h + y2 * g.h;
 }
 
+// the mixture's viscosity and conductivity from the liquid's and the vapour's
+__device__ __forceinline__ void mixture_transport(double t, double y1, double y2, double lv, double lc, double vv,
+                                                  double vc, const double* irh, double rho, double* tv) {
+  const double gv = ideal_vis(t), gc = 1395.333333 * gv;
+  const double yl = 1.0 - y1 - y2;
+  const double irhol = irh[0], irhov = irh[1], irhog = irh[2];
+  tv[0] = rho * (lv * yl * irhol + vv * y1 * irhov + gv * y2 * irhog);
+  tv[1] = rho * (lc * yl * irhol + vc * y1 * irhov + gc * y2 * irhog);
+}
+
 // eos%deteos: with transport properties when with_prop (tv(1:2) written), else simple
 __device__ __forceinline__ void deteos(int fluid, int with_prop, double p, double t, double y1, double y2,
                                        double* dv, double* tv, unsigned long long* fb) {
@@ -455,11 +469,7 @@ __device__ __forceinline__ void deteos(int fluid, int with_prop, double p, doubl
       iapws_transport(t, l.rho, lv, lc);
       iapws_transport(t, v.rho, vv, vc);
     }
-    double gv = ideal_vis(t), gc = 1395.333333 * gv;
-    double yl = 1.0 - y1 - y2;
-    const double irhol = irh[0], irhov = irh[1], irhog = irh[2];
-    tv[0] = dv[0] * (lv * yl * irhol + vv * y1 * irhov + gv * y2 * irhog);
-    tv[1] = dv[0] * (lc * yl * irhol + vc * y1 * irhov + gc * y2 * irhog);
+    mixture_transport(t, y1, y2, lv, lc, vv, vc, irh, dv[0], tv);
   }
 }
 
