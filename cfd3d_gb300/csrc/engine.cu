@@ -2331,7 +2331,7 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
       if (m == nstage) { stage(5); stage(6); }
       if (c.mixed) {
         k_update<true, true><<<E.red_grid, T, 0, s>>>(d, c, m);
-        launch_eos_cells(E, s, nullptr, nullptr, E.nint);
+        launch_eos_cells(E, s);
         n += eos_cells_launches(E);
       } else {
         k_update<false, true><<<E.red_grid, T, 0, s>>>(d, c, m);
@@ -2384,7 +2384,7 @@ void launch_iteration(Engine& E, bool full, cudaEvent_t* mark = nullptr) {
   stage(6);
   if (c.mixed) {
     k_update<true><<<E.red_grid, T, 0, s>>>(d, c, 0);
-    launch_eos_cells(E, s, nullptr, nullptr, E.nint);
+    launch_eos_cells(E, s);
     n += eos_cells_launches(E);
   } else {
     k_update<false><<<E.red_grid, T, 0, s>>>(d, c, 0);

@@ -169,7 +169,7 @@ struct DevPtr {
   float *pvf, *fi32, *fv32;
   float* gmf;        // mixed form: FP32 copy of gm (metrics of the FP32 viscous and SST terms)
   float* gmlo;       // mixed form: low parts of the face vectors, gm = gmf + gmlo (df64 terms)
-  float* frec;       // mixed form: reconstructed face states of one direction (2 x 12 planes)
+  float* frec;       // mixed form: reconstructed face states (2 x 12 planes), of face_slots directions
   // mixed form: per interior cell the free-stream part of its stored flux deviations,
   // (Phi + pref I).sum(n dl) over its faces, which depends on the metrics alone (npv planes)
   double* clo;
@@ -383,9 +383,8 @@ constexpr int SW_CH = 32;
 void launch_face_flux(const Engine& E, cudaStream_t s);
 int face_flux_launches(const Engine& E);
 void launch_face_flux_mixed(const Engine& E, cudaStream_t s, int b0, int b1);
-// the mixed form's cell EOS (eos_mixed.cu): dv and tv(1:2) of every interior cell, or of the
-// cells of a list, from pv
-void launch_eos_cells(const Engine& E, cudaStream_t s, const int* list, const int* count, long long most);
+// the mixed form's cell EOS (eos_mixed.cu): dv and tv(1:2) of every interior cell from pv
+void launch_eos_cells(const Engine& E, cudaStream_t s);
 int eos_cells_launches(const Engine& E);
 // discrete adjoint (adjoint.cu): buffers (allocated once, zeroed per call), the reverse
 // pass, and release

@@ -21,19 +21,18 @@ namespace cfd {
 enum { ES_IL = 0, ES_HL, ES_IG, ES_IV, ES_HV, NES };
 static_assert(NES * 2 <= 24, "the phase values fit the face records' planes");
 
-// the padded cell of item q
-__device__ __forceinline__ long long eos_cell(const DevPtr& d, const int* list, long long q) {
-  if (list) return list[q];
+// the padded cell of interior cell q
+__device__ __forceinline__ long long eos_cell(const DevPtr& d, long long q) {
   const int b = find_block_interior(d.blk, d.nblk, q);
   int i, j, k;
   return interior_cell(d.blk[b], q - d.blk[b].int_off, i, j, k);
 }
 
-__global__ void __launch_bounds__(256) k_eos_liq(DevPtr d, Par c, const int* list, const int* count, int* cnt) {
-  const long long n = d.ncell, m = count ? *count : d.nint;
+__global__ void __launch_bounds__(256) k_eos_liq(DevPtr d, Par c, int* cnt) {
+  const long long n = d.ncell;
   double* S = reinterpret_cast<double*>(d.frec);
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < m; q += (long long)gridDim.x * blockDim.x) {
-    const long long g = eos_cell(d, list, q);
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < d.nint; q += (long long)gridDim.x * blockDim.x) {
+    const long long g = eos_cell(d, q);
     const double p = d.pv[g] + c.pref, t = d.pv[4 * n + g], y1 = d.pv[5 * n + g];
     double il, hl, ig;
     liquid_inv_df64(df64(p), df64(t), &il, &hl, &ig);
@@ -66,12 +65,12 @@ __global__ void __launch_bounds__(256) k_eos_vap(DevPtr d, Par c, const int* cnt
   else eos_vap<false>(d, c, cnt);
 }
 
-__global__ void __launch_bounds__(256) k_eos_mix(DevPtr d, Par c, const int* list, const int* count) {
-  const long long n = d.ncell, m = count ? *count : d.nint;
+__global__ void __launch_bounds__(256) k_eos_mix(DevPtr d, Par c) {
+  const long long n = d.ncell;
   const double* S = reinterpret_cast<const double*>(d.frec);
   int bad = 0;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < m; q += (long long)gridDim.x * blockDim.x) {
-    const long long g = eos_cell(d, list, q);
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < d.nint; q += (long long)gridDim.x * blockDim.x) {
+    const long long g = eos_cell(d, q);
     const double p = d.pv[g] + c.pref, t = d.pv[4 * n + g], y1 = d.pv[5 * n + g], y2 = d.pv[6 * n + g];
     double dv[NDV], tv[2];
     if (c.fluid == 1) {
@@ -95,22 +94,22 @@ __global__ void __launch_bounds__(256) k_eos_mix(DevPtr d, Par c, const int* lis
   if (bad) atomicExch(&d.sc->nonfinite, 1);
 }
 
-void launch_eos_cells(const Engine& E, cudaStream_t s, const int* list, const int* count, long long most) {
+void launch_eos_cells(const Engine& E, cudaStream_t s) {
   const DevPtr& d = E.d;
   const Par& c = E.par;
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   auto grid = [&](int per) {
-    return (unsigned)std::max<long long>(1, std::min<long long>((most + 255) / 256, (long long)per * nsm));
+    return (unsigned)std::max<long long>(1, std::min<long long>((E.nint + 255) / 256, (long long)per * nsm));
   };
   if (c.fluid != 1) {
     int* cnt = d.mxn + MXN_FACE;
     cudaMemsetAsync(cnt, 0, MX_KINDS * sizeof(int), s);
-    k_eos_liq<<<grid(32), 256, 0, s>>>(d, c, list, count, cnt);
+    k_eos_liq<<<grid(32), 256, 0, s>>>(d, c, cnt);
     k_eos_vap<<<dim3(grid(4), 2), 256, 0, s>>>(d, c, cnt);
   }
-  k_eos_mix<<<grid(32), 256, 0, s>>>(d, c, list, count);
+  k_eos_mix<<<grid(32), 256, 0, s>>>(d, c);
 }
 
 int eos_cells_launches(const Engine& E) { return E.par.fluid != 1 ? 3 : 1; }
