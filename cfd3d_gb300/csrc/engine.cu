@@ -1476,7 +1476,9 @@ __global__ void __launch_bounds__(4 * SW_CH) k_sweep_df(DevPtr d, Par c, long lo
         }
         if (__all_sync(0xffffffffu, set)) break;
         ++it;
-        if ((it & 63) == 0 && *(volatile int*)&d.sc->sweep_stall) break;
+        // (the lanes leave together: another CTA may raise the flag between two lanes' reads,
+        // and a lane that left alone would leave the others waiting in the vote above)
+        if ((it & 63) == 0 && __any_sync(0xffffffffu, *(volatile int*)&d.sc->sweep_stall != 0)) break;
         if (it > spin) { atomicExch(&d.sc->sweep_stall, 1); break; }
         if (it > 2) __nanosleep(it > 64 ? 200 : 20);
       }
