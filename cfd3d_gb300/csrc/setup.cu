@@ -1006,10 +1006,15 @@ bool setup_tiles(Engine& E) {
     E.err = "device allocation failed (tile sweeps)";
     return false;
   }
-  cudaMemcpy(E.d_tiles, tiles.data(), ntile * sizeof(TileDesc), cudaMemcpyHostToDevice);
-  cudaMemcpy(E.d_pos, pos.data(), E.ncell * sizeof(int), cudaMemcpyHostToDevice);
-  // (on the engine's stream, which is not ordered after the default one: k_record_faces writes
-  // the records next)
+  // (on the engine's stream, which is not ordered after the default one, and waited for: a
+  // copy from pageable memory may return with the transfer to the device still to come, and
+  // k_record_faces scatters through pos next)
+  if (cudaMemcpyAsync(E.d_tiles, tiles.data(), ntile * sizeof(TileDesc), cudaMemcpyHostToDevice, E.st) != cudaSuccess ||
+      cudaMemcpyAsync(E.d_pos, pos.data(), E.ncell * sizeof(int), cudaMemcpyHostToDevice, E.st) != cudaSuccess ||
+      cudaStreamSynchronize(E.st) != cudaSuccess) {
+    E.err = "upload of the sweep tiles failed";
+    return false;
+  }
   cudaMemsetAsync(E.d.tq, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
   cudaMemsetAsync(E.d.tyf, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
   cudaMemsetAsync(E.d.tyb, 0, (size_t)ntile * NPVM * TILE_SLOTS * sizeof(float), E.st);
