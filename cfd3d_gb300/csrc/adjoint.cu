@@ -24,6 +24,7 @@
 // Gradients accumulate with atomics in padded SoA arrays: gpv (npv planes) and gdt (the dv
 // / tv entries that reach the residual, NGD planes).
 #include "adjoint.cuh"
+#include "alloc_group.h"
 
 namespace cfd {
 
@@ -266,21 +267,22 @@ inline unsigned adj_blocks(long long n, int T) { return (unsigned)((n + T - 1) /
 int adjoint_buffers(Engine& E) {
   const size_t n = (size_t)E.ncell;
   const int npv = E.par.npv;
-  if (!E.adj_lam) {
-    if (cudaMalloc(&E.adj_lam, n * npv * 8) != cudaSuccess || cudaMalloc(&E.adj_gpv, n * npv * 8) != cudaSuccess ||
-        cudaMalloc(&E.adj_gdt, n * NGD * 8) != cudaSuccess || cudaMalloc(&E.adj_gpar, 4 * 8) != cudaSuccess) {
-      E.err = "device allocation failed (adjoint buffers)";
-      return CFD3D_ERR_NOMEM;
-    }
-  }
+  // (out of memory: nothing half-made stays, and the error is this call's alone)
+  auto group = [&](std::initializer_list<GroupItem> items) {
+    if (alloc_group(items, [](void** p, size_t b) { return cudaMalloc(p, b) == cudaSuccess; }, [](void* p) { cudaFree(p); }))
+      return true;
+    cudaGetLastError();
+    E.err = "device allocation failed (adjoint buffers)";
+    return false;
+  };
+  if (!E.adj_lam && !group({{(void**)&E.adj_lam, n * npv * 8}, {(void**)&E.adj_gpv, n * npv * 8},
+                            {(void**)&E.adj_gdt, n * NGD * 8}, {(void**)&E.adj_gpar, 4 * 8}}))
+    return CFD3D_ERR_NOMEM;
   // the face kernels' states and scratch planes: the FP64 form's own, else one direction's
-  if (E.par.mixed && !E.adj_fi && E.par.nmuscl > 0) {
-    const size_t nfs = (E.par.nmuscl == 2) ? 5 : 1;
-    if (cudaMalloc(&E.adj_fi, n * npv * 3 * 8) != cudaSuccess || cudaMalloc(&E.adj_fsc, n * npv * nfs * 8) != cudaSuccess) {
-      E.err = "device allocation failed (adjoint buffers)";
-      return CFD3D_ERR_NOMEM;
-    }
-  }
+  const size_t nfs = (E.par.nmuscl == 2) ? 5 : 1;
+  if (E.par.mixed && !E.adj_fi && E.par.nmuscl > 0 &&
+      !group({{(void**)&E.adj_fi, n * npv * 3 * 8}, {(void**)&E.adj_fsc, n * npv * nfs * 8}}))
+    return CFD3D_ERR_NOMEM;
   cudaMemsetAsync(E.adj_lam, 0, n * npv * 8, E.st);
   cudaMemsetAsync(E.adj_gpv, 0, n * npv * 8, E.st);
   cudaMemsetAsync(E.adj_gdt, 0, n * NGD * 8, E.st);

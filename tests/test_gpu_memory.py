@@ -1,0 +1,45 @@
+"""Device memory: calls that find none left report it and leave the handle usable."""
+import numpy as np
+import pytest
+
+from cfd3d_gb300 import abi, native
+from cfd3d_gb300.native import Cfd3dError
+from tests import test_gpu_adjoint as base
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def _fill(leave):
+    """all of the device's free memory but about `leave` bytes"""
+    torch = pytest.importorskip("torch")
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    return torch.empty((free - leave) // (2 * MB) * (2 * MB), dtype=torch.uint8, device="cuda")
+
+
+# 64^3 cells in 70^3: 25 MB for each of the cotangent and the gradient, 27 MB for dv and tv; a
+# mixed-form handle then needs the face states and 123 MB of reconstruction planes
+@pytest.mark.parametrize("precision,leave", [(abi.FP64, 40 * MB), (abi.MIXED, 40 * MB), (abi.MIXED, 190 * MB)])
+def test_adjoint_after_out_of_memory(precision, leave):
+    import torch
+    c = base._state(1)
+    lam = np.random.default_rng(9).normal(size=abi.interior_shape(c["blocks"][0], 9))
+    e = native.Engine(c, precision=precision)
+    e.initialize(c["pv0"])
+    hold = _fill(leave)
+    for _ in range(2):
+        with pytest.raises(Cfd3dError) as ei:
+            e.residual_vjp([lam])
+        assert ei.value.code == abi.ERR_NOMEM
+    del hold
+    torch.cuda.empty_cache()
+    g = e.residual_vjp([lam])[0][0]
+    e.close()
+    f = native.Engine(c, precision=precision)
+    f.initialize(c["pv0"])
+    want = f.residual_vjp([lam])[0][0]
+    f.close()
+    for v in range(9):   # (sums by atomics, in any order)
+        assert np.abs(g[..., v] - want[..., v]).max() <= 1e-10 * np.abs(want[..., v]).max()
