@@ -19,9 +19,6 @@ UNITS = ["adjoint_face.cu", "adjoint_duals.cu", "adjoint.cu", "engine.cu", "setu
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-I", os.path.join(ROOT, "include")]
-# the adjoint's dual-number routines are large and off the common path: the device compiler's
-# fast-compile mode keeps their build at seconds instead of minutes
-UNIT_FLAGS = {"adjoint_duals.cu": ["-Ofc", "mid"]}
 
 
 def nvcc():
@@ -44,7 +41,7 @@ def build(force=False, verbose=False, extra=()):
 
     def compile_one(u):
         obj = os.path.join(OUT, u.replace(".cu", ".o"))
-        cmd = [nv, *ARCH, *FLAGS, *UNIT_FLAGS.get(u, []), *extra, "-c", os.path.join(SRC, u), "-o", obj]
+        cmd = [nv, *ARCH, *FLAGS, *extra, "-c", os.path.join(SRC, u), "-o", obj]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed for {u}:\n{r.stderr}")

@@ -181,10 +181,14 @@ __global__ void k_adj_ghost(DevPtr d, Par c, AdjPtr a, const GhostOp* __restrict
             for (int m = 0; m < 4; ++m) pbd[m] = seed(pb[m], 9 + m, k0);
             const DD ur = seed(c.uref, 15, k0);
             for (int v = 0; v < NPVM; ++v) bp[v] = DD(bpv[v]);
-            if (c.uref != 0.0 && 15 >= k0 && 15 < k0 + DC)
-              for (int e = 0; e < 3; ++e) bp[1 + e].d[15 - k0] = c.uref_vec[e] / c.uref;
+            // the free-stream velocity is uref times a direction
+            for (int e = 0; e < 3; ++e) {
+              const DD u = seed(0.0, 15, k0);
+              if (c.uref != 0.0) bp[1 + e] = bp[1 + e] + (c.uref_vec[e] / c.uref) * u;
+            }
             farfield_pv<DD>(c, nx, dl, pbd, seed(rb, 13, k0), seed(c2b, 14, k0), bp, ur * ur, x, ffm);
-            for (int qq = 0; qq < DC && k0 + qq < 16; ++qq) {
+#pragma unroll
+            for (int qq = 0; qq < DC; ++qq) {   // (DC divides 16)
               double s = 0.0;
               for (int v = 0; v < npv; ++v) s += gp[v] * x[v].d[qq];
               w[k0 + qq] = s;

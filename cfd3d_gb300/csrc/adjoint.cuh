@@ -12,7 +12,6 @@ namespace cfd {
 // reference's 1-based numbering
 enum { GD_RHO = 0, GD_H, GD_C2, GD_CP, GD_RL, GD_RV, GD_RG, GD_VIS, GD_CON, GD_MUT, NGD };
 constexpr int NGD_DV = 7;   // the planes that are dv entries
-static __constant__ int kGdDv[NGD_DV] = {0, 1, 5, 11, 2, 3, 4};   // their dv slots
 
 struct AdjPtr {
   const double* lam;   // padded cotangent (npv x ncell), zero outside the interior
@@ -33,6 +32,7 @@ static __device__ __noinline__ EosJac eos_jac(int fluid, double p, double t, dou
   deteos_t<D4>(fluid, 0, D4::seed(p, 0), D4::seed(t, 1), D4::seed(y1, 2), D4::seed(y2, 3), dv, nullptr);
   EosJac j;
   j.rho = dv[0].v; j.h = dv[1].v; j.c2 = dv[5].v;
+#pragma unroll
   for (int m = 0; m < 4; ++m) { j.drho[m] = dv[0].d[m]; j.dh[m] = dv[1].d[m]; j.dc2[m] = dv[5].d[m]; }
   return j;
 }
@@ -43,9 +43,12 @@ static __device__ __noinline__ void eos_chain(const Par& c, double p, double t, 
   using D4 = Dual<4>;
   D4 dv[NDV], tv[3];
   deteos_t<D4>(c.fluid, c.with_prop, D4::seed(p, 0), D4::seed(t, 1), D4::seed(y1, 2), D4::seed(y2, 3), dv, tv);
+  constexpr int slot[NGD_DV] = {0, 1, 5, 11, 2, 3, 4};   // the planes' dv entries
+#pragma unroll
   for (int m = 0; m < 4; ++m) {
     double s = 0.0;
-    for (int q = 0; q < NGD_DV; ++q) s += gd[q] * dv[kGdDv[q]].d[m];
+#pragma unroll
+    for (int q = 0; q < NGD_DV; ++q) s += gd[q] * dv[slot[q]].d[m];
     if (c.with_prop) s += gd[GD_VIS] * tv[0].d[m] + gd[GD_CON] * tv[1].d[m];
     ge[m] = s;
   }
@@ -55,10 +58,12 @@ static __device__ __noinline__ void eos_chain(const Par& c, double p, double t, 
 // Local Jacobians are taken DC seed directions at a time (a few passes of the same code
 // on Dual<DC>), which keeps the per-thread dual arrays small.
 constexpr int DC = 8;
-using DD = Dual<DC, 1>;   // (rolled loops: these kernels hold dozens of duals)
+using DD = Dual<DC>;
 __device__ __forceinline__ DD seed(double v, int i, int k0) {
-  DD r(v);
-  if (i >= k0 && i < k0 + DC) r.d[i - k0] = 1.0;
+  DD r;
+  r.v = v;
+#pragma unroll
+  for (int q = 0; q < DC; ++q) r.d[q] = (i - k0 == q) ? 1.0 : 0.0;
   return r;
 }
 

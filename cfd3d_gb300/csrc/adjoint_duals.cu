@@ -1,9 +1,7 @@
 // adjoint_duals.cu -- the parts of the discrete adjoint that stay with duals of eight
 // directions: the flux of Roe-M and AUSMPW+, and the cell sources of the cavitation models
 // other than Merkle's and of the DES lengths.  The file comment of adjoint.cu describes the
-// whole reverse pass.  This unit is built in the device compiler's fast-compile mode: its
-// full optimisation takes minutes over these routines, and it got the rolled dual loops of
-// the two fluxes wrong (gradients of 1e40 that this mode and the unrolled loops do not give).
+// whole reverse pass.
 #include "adjoint_flux.cuh"
 
 namespace cfd {
@@ -26,14 +24,18 @@ static __device__ __noinline__ void flux_back_duals(const Par& c, const double* 
     roe_state<DD>(npv, Ld, Rd, ravg);
     const int am[4] = {0, 4, 5, 6};
     DD rc2(jc.c2);
+#pragma unroll
     for (int m = 0; m < 4; ++m)
+#pragma unroll
       for (int q = 0; q < DC; ++q) rc2.d[q] += jc.dc2[m] * ravg[am[m]].d[q];
     const DD uref = seed(c.uref, S_UREF, k0);
     DD sdst[18];
     for (int l = 0; l < 18; ++l) sdst[l] = seed(sdv[l], S_SDST + l, k0);
     DD fx[NPVM];
     inviscid_flux_core<DD>(c, nx, Ld, Rd, sdst, ravg, rc2, uref * uref, fx);
-    for (int q = 0; q < DC && k0 + q < NS_INV; ++q) {
+#pragma unroll
+    for (int q = 0; q < DC; ++q) {
+      if (k0 + q >= NS_INV) break;
       double acc = 0.0;
       for (int v = 0; v < npv; ++v) acc += lam[v] * fx[v].d[q];
       w[k0 + q] = acc;
@@ -99,7 +101,9 @@ __global__ void __launch_bounds__(64) k_adj_cell(DevPtr d, Par c, AdjPtr a) {
         for (int m = 0; m < 4; ++m) dd[dvs[m]] = seed(dv[dvs[m]], 4 + m, k0);
         const CavOutT<DD> o = cavsource_t<DD>(c, p2, dd, vol, seed(c.uref, 8, k0), seed(c.c_v, 9, k0),
                                               seed(c.c_c, 10, k0));
-        for (int q = 0; q < DC && k0 + q < 11; ++q) w[k0 + q] = lam[5] * (o.r_v.d[q] - o.r_c.d[q]);
+#pragma unroll
+        for (int q = 0; q < DC; ++q)
+          if (k0 + q < 11) w[k0 + q] = lam[5] * (o.r_v.d[q] - o.r_c.d[q]);
       }
       for (int m = 0; m < 4; ++m) gp[pvs[m]] += w[m];
       gd[GD_RHO] += w[4]; gd[GD_RL] += w[5]; gd[GD_RV] += w[6]; gd[GD_RG] += w[7];
@@ -135,7 +139,9 @@ __global__ void __launch_bounds__(64) k_adj_cell(DevPtr d, Par c, AdjPtr a) {
           for (int e = 0; e < 3; ++e) gr[q][e] = seed(grv[q][e], 3 * q + e, k0);
         const SstOut<DD> so = sst_source<DD>(gr, seed(pv2[7], 15, k0), seed(pv2[8], 16, k0), seed(dv[0], 17, k0),
                                              seed(mu, 18, k0), seed(mut, 19, k0), y5, vol, c.ides, hmax);
-        for (int q = 0; q < DC && k0 + q < 20; ++q) w[k0 + q] = lam[7] * so.r7.d[q] + lam[8] * so.r8.d[q];
+#pragma unroll
+        for (int q = 0; q < DC; ++q)
+          if (k0 + q < 20) w[k0 + q] = lam[7] * so.r7.d[q] + lam[8] * so.r8.d[q];
       }
       // the cell gradients are linear in the face averages 0.5 (P[nbr] + P[g])
       const double sgn[6] = {-1.0, 1.0, -1.0, 1.0, -1.0, 1.0};

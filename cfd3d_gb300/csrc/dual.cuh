@@ -8,136 +8,144 @@
 // taken on the values, as in the forward evaluation, so the derivative is that of the
 // branch the forward residual took.  Values are formed without FMA contraction, like the
 // reconstruction's uncontracted arithmetic, so that ties at clip bounds resolve the same way.
+//
+// The direction index of a derivative is always known at compile time (loops over the
+// directions unrolled, seeds by comparison).  With an index computed at run time the device
+// compiler's full optimisation returned wrong derivatives: cell sources whose first eight
+// directions were lost where only the seeds were indexed so, flux gradients of 1e40 where
+// every loop was rolled.  The source was not at fault: on the host it reads no uninitialised
+// value, stays in range and gives the same bits rolled or unrolled.
 #pragma once
 #include <cmath>
 #include "eos64.cuh"
 
 namespace cfd {
 
-// U: unrolling of the loops over the directions (N: the duals live in registers)
-template <int N, int U = N>
+template <int N>
 struct Dual {
   double v;
   double d[N];
   __device__ __forceinline__ Dual() {}
   __device__ __forceinline__ Dual(double x) : v(x) {
-#pragma unroll U
+#pragma unroll
     for (int i = 0; i < N; ++i) d[i] = 0.0;
   }
   __device__ __forceinline__ static Dual seed(double x, int i) {
-    Dual r(x);
-    r.d[i] = 1.0;
+    Dual r;
+    r.v = x;
+#pragma unroll
+    for (int q = 0; q < N; ++q) r.d[q] = (q == i) ? 1.0 : 0.0;
     return r;
   }
   __device__ __forceinline__ explicit operator double() const { return v; }
 };
 
-#define DUAL_LOOP _Pragma("unroll U") for (int i = 0; i < N; ++i)
+#define DUAL_LOOP _Pragma("unroll") for (int i = 0; i < N; ++i)
 
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator+(const Dual<N, U>& a, const Dual<N, U>& b) {
-  Dual<N, U> r; r.v = __dadd_rn(a.v, b.v); DUAL_LOOP r.d[i] = a.d[i] + b.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> operator+(const Dual<N>& a, const Dual<N>& b) {
+  Dual<N> r; r.v = __dadd_rn(a.v, b.v); DUAL_LOOP r.d[i] = a.d[i] + b.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator-(const Dual<N, U>& a, const Dual<N, U>& b) {
-  Dual<N, U> r; r.v = __dsub_rn(a.v, b.v); DUAL_LOOP r.d[i] = a.d[i] - b.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> operator-(const Dual<N>& a, const Dual<N>& b) {
+  Dual<N> r; r.v = __dsub_rn(a.v, b.v); DUAL_LOOP r.d[i] = a.d[i] - b.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator-(const Dual<N, U>& a) {
-  Dual<N, U> r; r.v = -a.v; DUAL_LOOP r.d[i] = -a.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> operator-(const Dual<N>& a) {
+  Dual<N> r; r.v = -a.v; DUAL_LOOP r.d[i] = -a.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator*(const Dual<N, U>& a, const Dual<N, U>& b) {
-  Dual<N, U> r; r.v = __dmul_rn(a.v, b.v); DUAL_LOOP r.d[i] = a.d[i] * b.v + a.v * b.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, const Dual<N>& b) {
+  Dual<N> r; r.v = __dmul_rn(a.v, b.v); DUAL_LOOP r.d[i] = a.d[i] * b.v + a.v * b.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator/(const Dual<N, U>& a, const Dual<N, U>& b) {
-  Dual<N, U> r; r.v = a.v / b.v;
+template <int N> __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, const Dual<N>& b) {
+  Dual<N> r; r.v = a.v / b.v;
   const double ib = 1.0 / b.v;
   DUAL_LOOP r.d[i] = (a.d[i] - r.v * b.d[i]) * ib;
   return r;
 }
 // mixed operands
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator+(const Dual<N, U>& a, double b) { Dual<N, U> r = a; r.v = __dadd_rn(r.v, b); return r; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator+(double a, const Dual<N, U>& b) { Dual<N, U> r = b; r.v = __dadd_rn(a, r.v); return r; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator-(const Dual<N, U>& a, double b) { Dual<N, U> r = a; r.v = __dsub_rn(r.v, b); return r; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator-(double a, const Dual<N, U>& b) {
-  Dual<N, U> r; r.v = __dsub_rn(a, b.v); DUAL_LOOP r.d[i] = -b.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> operator+(const Dual<N>& a, double b) { Dual<N> r = a; r.v = __dadd_rn(r.v, b); return r; }
+template <int N> __device__ __forceinline__ Dual<N> operator+(double a, const Dual<N>& b) { Dual<N> r = b; r.v = __dadd_rn(a, r.v); return r; }
+template <int N> __device__ __forceinline__ Dual<N> operator-(const Dual<N>& a, double b) { Dual<N> r = a; r.v = __dsub_rn(r.v, b); return r; }
+template <int N> __device__ __forceinline__ Dual<N> operator-(double a, const Dual<N>& b) {
+  Dual<N> r; r.v = __dsub_rn(a, b.v); DUAL_LOOP r.d[i] = -b.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator*(const Dual<N, U>& a, double b) {
-  Dual<N, U> r; r.v = __dmul_rn(a.v, b); DUAL_LOOP r.d[i] = a.d[i] * b; return r;
+template <int N> __device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, double b) {
+  Dual<N> r; r.v = __dmul_rn(a.v, b); DUAL_LOOP r.d[i] = a.d[i] * b; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator*(double a, const Dual<N, U>& b) { return b * a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator/(const Dual<N, U>& a, double b) {
-  Dual<N, U> r; r.v = a.v / b;
+template <int N> __device__ __forceinline__ Dual<N> operator*(double a, const Dual<N>& b) { return b * a; }
+template <int N> __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, double b) {
+  Dual<N> r; r.v = a.v / b;
   const double ib = 1.0 / b;
   DUAL_LOOP r.d[i] = a.d[i] * ib;
   return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> operator/(double a, const Dual<N, U>& b) {
-  Dual<N, U> r; r.v = a / b.v;
+template <int N> __device__ __forceinline__ Dual<N> operator/(double a, const Dual<N>& b) {
+  Dual<N> r; r.v = a / b.v;
   const double f = -r.v / b.v;
   DUAL_LOOP r.d[i] = f * b.d[i];
   return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U>& operator+=(Dual<N, U>& a, const Dual<N, U>& b) { a = a + b; return a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U>& operator-=(Dual<N, U>& a, const Dual<N, U>& b) { a = a - b; return a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U>& operator*=(Dual<N, U>& a, const Dual<N, U>& b) { a = a * b; return a; }
+template <int N> __device__ __forceinline__ Dual<N>& operator+=(Dual<N>& a, const Dual<N>& b) { a = a + b; return a; }
+template <int N> __device__ __forceinline__ Dual<N>& operator-=(Dual<N>& a, const Dual<N>& b) { a = a - b; return a; }
+template <int N> __device__ __forceinline__ Dual<N>& operator*=(Dual<N>& a, const Dual<N>& b) { a = a * b; return a; }
 
 // comparisons on values
-template <int N, int U> __device__ __forceinline__ bool operator<(const Dual<N, U>& a, const Dual<N, U>& b) { return a.v < b.v; }
-template <int N, int U> __device__ __forceinline__ bool operator>(const Dual<N, U>& a, const Dual<N, U>& b) { return a.v > b.v; }
-template <int N, int U> __device__ __forceinline__ bool operator<=(const Dual<N, U>& a, const Dual<N, U>& b) { return a.v <= b.v; }
-template <int N, int U> __device__ __forceinline__ bool operator>=(const Dual<N, U>& a, const Dual<N, U>& b) { return a.v >= b.v; }
-template <int N, int U> __device__ __forceinline__ bool operator<(const Dual<N, U>& a, double b) { return a.v < b; }
-template <int N, int U> __device__ __forceinline__ bool operator>(const Dual<N, U>& a, double b) { return a.v > b; }
-template <int N, int U> __device__ __forceinline__ bool operator<=(const Dual<N, U>& a, double b) { return a.v <= b; }
-template <int N, int U> __device__ __forceinline__ bool operator>=(const Dual<N, U>& a, double b) { return a.v >= b; }
-template <int N, int U> __device__ __forceinline__ bool operator!=(const Dual<N, U>& a, double b) { return a.v != b; }
-template <int N, int U> __device__ __forceinline__ bool operator!=(const Dual<N, U>& a, const Dual<N, U>& b) { return a.v != b.v; }
-template <int N, int U> __device__ __forceinline__ bool operator==(const Dual<N, U>& a, const Dual<N, U>& b) { return a.v == b.v; }
-template <int N, int U> __device__ __forceinline__ bool operator==(const Dual<N, U>& a, double b) { return a.v == b; }
+template <int N> __device__ __forceinline__ bool operator<(const Dual<N>& a, const Dual<N>& b) { return a.v < b.v; }
+template <int N> __device__ __forceinline__ bool operator>(const Dual<N>& a, const Dual<N>& b) { return a.v > b.v; }
+template <int N> __device__ __forceinline__ bool operator<=(const Dual<N>& a, const Dual<N>& b) { return a.v <= b.v; }
+template <int N> __device__ __forceinline__ bool operator>=(const Dual<N>& a, const Dual<N>& b) { return a.v >= b.v; }
+template <int N> __device__ __forceinline__ bool operator<(const Dual<N>& a, double b) { return a.v < b; }
+template <int N> __device__ __forceinline__ bool operator>(const Dual<N>& a, double b) { return a.v > b; }
+template <int N> __device__ __forceinline__ bool operator<=(const Dual<N>& a, double b) { return a.v <= b; }
+template <int N> __device__ __forceinline__ bool operator>=(const Dual<N>& a, double b) { return a.v >= b; }
+template <int N> __device__ __forceinline__ bool operator!=(const Dual<N>& a, double b) { return a.v != b; }
+template <int N> __device__ __forceinline__ bool operator!=(const Dual<N>& a, const Dual<N>& b) { return a.v != b.v; }
+template <int N> __device__ __forceinline__ bool operator==(const Dual<N>& a, const Dual<N>& b) { return a.v == b.v; }
+template <int N> __device__ __forceinline__ bool operator==(const Dual<N>& a, double b) { return a.v == b; }
 
 // elementary functions
-template <int N, int U> __device__ __forceinline__ Dual<N, U> sqrt(const Dual<N, U>& a) {
-  Dual<N, U> r; r.v = ::sqrt(a.v);
+template <int N> __device__ __forceinline__ Dual<N> sqrt(const Dual<N>& a) {
+  Dual<N> r; r.v = ::sqrt(a.v);
   const double f = (r.v > 0.0) ? 0.5 / r.v : 0.0;
   DUAL_LOOP r.d[i] = f * a.d[i];
   return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> exp(const Dual<N, U>& a) {
-  Dual<N, U> r; r.v = ::exp(a.v); DUAL_LOOP r.d[i] = r.v * a.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> exp(const Dual<N>& a) {
+  Dual<N> r; r.v = ::exp(a.v); DUAL_LOOP r.d[i] = r.v * a.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> log(const Dual<N, U>& a) {
-  Dual<N, U> r; r.v = ::log(a.v); const double f = 1.0 / a.v; DUAL_LOOP r.d[i] = f * a.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> log(const Dual<N>& a) {
+  Dual<N> r; r.v = ::log(a.v); const double f = 1.0 / a.v; DUAL_LOOP r.d[i] = f * a.d[i]; return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> tanh(const Dual<N, U>& a) {
-  Dual<N, U> r; r.v = ::tanh(a.v); const double f = 1.0 - r.v * r.v; DUAL_LOOP r.d[i] = f * a.d[i]; return r;
+template <int N> __device__ __forceinline__ Dual<N> tanh(const Dual<N>& a) {
+  Dual<N> r; r.v = ::tanh(a.v); const double f = 1.0 - r.v * r.v; DUAL_LOOP r.d[i] = f * a.d[i]; return r;
 }
 // x^y with a constant exponent
-template <int N, int U> __device__ __forceinline__ Dual<N, U> pow(const Dual<N, U>& a, double y) {
-  Dual<N, U> r; r.v = ::pow(a.v, y);
+template <int N> __device__ __forceinline__ Dual<N> pow(const Dual<N>& a, double y) {
+  Dual<N> r; r.v = ::pow(a.v, y);
   const double f = (a.v != 0.0) ? y * r.v / a.v : 0.0;
   DUAL_LOOP r.d[i] = f * a.d[i];
   return r;
 }
 // x^y with both varying: d = x^y (y' log x + y x'/x)
-template <int N, int U> __device__ __forceinline__ Dual<N, U> pow(const Dual<N, U>& a, const Dual<N, U>& y) {
-  Dual<N, U> r; r.v = ::pow(a.v, y.v);
+template <int N> __device__ __forceinline__ Dual<N> pow(const Dual<N>& a, const Dual<N>& y) {
+  Dual<N> r; r.v = ::pow(a.v, y.v);
   const double lx = (a.v > 0.0) ? ::log(a.v) : 0.0;
   const double f = (a.v != 0.0) ? y.v * r.v / a.v : 0.0;
   DUAL_LOOP r.d[i] = r.v * lx * y.d[i] + f * a.d[i];
   return r;
 }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fabs(const Dual<N, U>& a) { return (a.v < 0.0) ? -a : a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fmin(const Dual<N, U>& a, const Dual<N, U>& b) { return (b.v < a.v) ? b : a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fmax(const Dual<N, U>& a, const Dual<N, U>& b) { return (b.v > a.v) ? b : a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fmin(const Dual<N, U>& a, double b) { return (b < a.v) ? Dual<N, U>(b) : a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fmax(const Dual<N, U>& a, double b) { return (b > a.v) ? Dual<N, U>(b) : a; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fmin(double a, const Dual<N, U>& b) { return (b.v < a) ? b : Dual<N, U>(a); }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> fmax(double a, const Dual<N, U>& b) { return (b.v > a) ? b : Dual<N, U>(a); }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> copysign(double a, const Dual<N, U>& b) { return Dual<N, U>(::copysign(a, b.v)); }
-template <int N, int U> __device__ __forceinline__ bool isfinite(const Dual<N, U>& a) { return ::isfinite(a.v); }
+template <int N> __device__ __forceinline__ Dual<N> fabs(const Dual<N>& a) { return (a.v < 0.0) ? -a : a; }
+template <int N> __device__ __forceinline__ Dual<N> fmin(const Dual<N>& a, const Dual<N>& b) { return (b.v < a.v) ? b : a; }
+template <int N> __device__ __forceinline__ Dual<N> fmax(const Dual<N>& a, const Dual<N>& b) { return (b.v > a.v) ? b : a; }
+template <int N> __device__ __forceinline__ Dual<N> fmin(const Dual<N>& a, double b) { return (b < a.v) ? Dual<N>(b) : a; }
+template <int N> __device__ __forceinline__ Dual<N> fmax(const Dual<N>& a, double b) { return (b > a.v) ? Dual<N>(b) : a; }
+template <int N> __device__ __forceinline__ Dual<N> fmin(double a, const Dual<N>& b) { return (b.v < a) ? b : Dual<N>(a); }
+template <int N> __device__ __forceinline__ Dual<N> fmax(double a, const Dual<N>& b) { return (b.v > a) ? b : Dual<N>(a); }
+template <int N> __device__ __forceinline__ Dual<N> copysign(double a, const Dual<N>& b) { return Dual<N>(::copysign(a, b.v)); }
+template <int N> __device__ __forceinline__ bool isfinite(const Dual<N>& a) { return ::isfinite(a.v); }
 
 // uncontracted arithmetic of the reconstruction: duals have no FMA ambiguity
-template <int N, int U> __device__ __forceinline__ Dual<N, U> nmul(const Dual<N, U>& a, const Dual<N, U>& b) { return a * b; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> nadd(const Dual<N, U>& a, const Dual<N, U>& b) { return a + b; }
-template <int N, int U> __device__ __forceinline__ Dual<N, U> nsub(const Dual<N, U>& a, const Dual<N, U>& b) { return a - b; }
+template <int N> __device__ __forceinline__ Dual<N> nmul(const Dual<N>& a, const Dual<N>& b) { return a * b; }
+template <int N> __device__ __forceinline__ Dual<N> nadd(const Dual<N>& a, const Dual<N>& b) { return a + b; }
+template <int N> __device__ __forceinline__ Dual<N> nsub(const Dual<N>& a, const Dual<N>& b) { return a - b; }
 
 #undef DUAL_LOOP
 
@@ -188,12 +196,12 @@ __device__ __forceinline__ void g64_groups3(double x, double y, double yi, G64Th
        x, y, yi, a, std::make_index_sequence<IGroups<TAB, N>::start(G + 1) - IGroups<TAB, N>::start(G)>{}), ...);
 }
 
-template <int N, int U>
-struct GibbsByParts<Dual<N, U>> {
+template <int N>
+struct GibbsByParts<Dual<N>> {
   static constexpr bool value = true;
   template <const IJN* TAB, size_t... K>
-  static __device__ __forceinline__ void sum(const Dual<N, U>& X, const Dual<N, U>&, const Dual<N, U>& Y,
-                                             const Dual<N, U>& YI, GAcc<Dual<N, U>>& a) {
+  static __device__ __forceinline__ void sum(const Dual<N>& X, const Dual<N>&, const Dual<N>& Y,
+                                             const Dual<N>& YI, GAcc<Dual<N>>& a) {
     constexpr size_t M = sizeof...(K);
     const double x = X.v, yi = YI.v, yi2 = yi * yi;
     G64Third g;
@@ -210,11 +218,11 @@ struct GibbsByParts<Dual<N, U>> {
     S[7] = fma(x, fma(x, g.c1, 2.0 * g.t2), g.o2) * yi2;
     S[8] = fma(x, fma(x, fma(x, g.d0, g.t3), g.o3), g.z3) * (yi2 * yi);
     const int from[5][3] = {{0, 2, 3}, {1, 3, 4}, {2, 5, 6}, {3, 6, 7}, {4, 7, 8}};
-    Dual<N, U>* out[5] = {&a.x, &a.y, &a.xx, &a.xy, &a.yy};
+    Dual<N>* out[5] = {&a.x, &a.y, &a.xx, &a.xy, &a.yy};
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-      Dual<N, U> r(S[from[q][0]]);
-#pragma unroll U
+      Dual<N> r(S[from[q][0]]);
+#pragma unroll
       for (int i = 0; i < N; ++i) r.d[i] = S[from[q][1]] * X.d[i] + S[from[q][2]] * Y.d[i];
       *out[q] = *out[q] + r;
     }
