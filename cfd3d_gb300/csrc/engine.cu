@@ -2605,11 +2605,16 @@ int eos_run(int fluid, int with_prop, int64_t n, const double* p, const double* 
       if (cudaMemcpy(in + q * m, src[q], b, cudaMemcpyHostToDevice) != cudaSuccess) return CFD3D_ERR_CUDA;
     if (cudaMemset(fb, 0, 8) != cudaSuccess) return CFD3D_ERR_CUDA;
   }
-  if (TERMS)
-    k_eos_terms<<<(unsigned)((n + 31) / 32), 32>>>(fluid, with_prop, n, in, in + m, in + 2 * m, in + 3 * m, ddv, dtv);
+  // (the launch's own status: an error that some earlier call left behind is not this call's)
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3((unsigned)((n + 31) / 32));
+  lc.blockDim = dim3(TERMS ? 32 : 64);
+  cudaError_t e;
+  if constexpr (TERMS)
+    e = cudaLaunchKernelEx(&lc, k_eos_terms, fluid, with_prop, (long long)n, in, in + m, in + 2 * m, in + 3 * m, ddv, dtv);
   else
-    k_eos_points<<<(unsigned)((n + 31) / 32), 64>>>(fluid, with_prop, n, in, in + m, in + 2 * m, in + 3 * m, ddv, dtv, fb);
-  if (cudaGetLastError() != cudaSuccess) return CFD3D_ERR_CUDA;
+    e = cudaLaunchKernelEx(&lc, k_eos_points, fluid, with_prop, (long long)n, in, in + m, in + 2 * m, in + 3 * m, ddv, dtv, fb);
+  if (e != cudaSuccess) return CFD3D_ERR_CUDA;
   if (packed) {
     if (cudaMemcpy(stage, ddv, out * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return CFD3D_ERR_CUDA;
     std::memcpy(dv, stage, b * NDV);
@@ -2638,7 +2643,10 @@ int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, c
     cudaGetLastError();
   }
   double* x = nullptr;
-  if (cudaMalloc(&x, (1 + EOS_PER_POINT * (size_t)n) * 8) != cudaSuccess) return CFD3D_ERR_NOMEM;
+  if (cudaMalloc(&x, (1 + EOS_PER_POINT * (size_t)n) * 8) != cudaSuccess) {
+    cudaGetLastError();
+    return CFD3D_ERR_NOMEM;
+  }
   const int rc = eos_run<TERMS>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x);
   cudaFree(x);
   return rc;
@@ -2666,7 +2674,7 @@ int cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const 
   return x ? eos_run<false>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x) : CFD3D_ERR_CUDA;
 }
 
-int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {
+static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {
   if (!out) return CFD3D_ERR_ARG;
   *out = nullptr;
   cfd3d_handle* h = new (std::nothrow) cfd3d_handle();
@@ -2911,6 +2919,13 @@ int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* b
   }
   CFD_CUDA(cudaDeviceSynchronize());
   return CFD3D_OK;
+}
+
+int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {
+  const int rc = create_handle(cfg, nblocks, blocks, out);
+  // a failed allocation's error is reported by rc: it does not stay for the next call
+  if (rc == CFD3D_ERR_NOMEM || rc == CFD3D_ERR_DESCRIPTOR) cudaGetLastError();
+  return rc;
 }
 
 void cfd3d_destroy(cfd3d_handle* h) {

@@ -399,10 +399,13 @@ void setup_planes(Engine& E);
 bool setup_vfg_halo(Engine& E, const cfd3d_block_desc* blocks, int nblocks);
 bool setup_tiles(Engine& E);
 
+// (the runtime keeps a failed call's error for the next cudaGetLastError: it is reported here,
+// so it is taken here)
 #define CFD_CUDA(call)                                                                 \
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
     if (e_ != cudaSuccess) {                                                           \
+      (void)cudaGetLastError();                                                        \
       E.err = std::string(#call) + ": " + cudaGetErrorString(e_);                      \
       return CFD3D_ERR_CUDA;                                                           \
     }                                                                                  \

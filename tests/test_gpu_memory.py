@@ -43,3 +43,30 @@ def test_adjoint_after_out_of_memory(precision, leave):
     f.close()
     for v in range(9):   # (sums by atomics, in any order)
         assert np.abs(g[..., v] - want[..., v]).max() <= 1e-10 * np.abs(want[..., v]).max()
+
+
+def test_a_failed_create_leaves_the_other_calls_alone():
+    import torch
+    c = base._state(1)
+    rng = np.random.default_rng(3)
+    p, t = rng.uniform(2e3, 3e5, 5000), rng.uniform(280.0, 320.0, 5000)
+    y1, y2 = rng.uniform(0.0, 0.5, 5000), np.full(5000, 1e-7)
+    want = native.eos_eval(p, t, y1, y2, prop=True)
+    for points in (5, 5000):   # through the static buffer, through an allocation
+        hold = _fill(40 * MB)
+        with pytest.raises(Cfd3dError) as ei:
+            native.Engine(c, precision=abi.FP64)
+        assert ei.value.code == abi.ERR_NOMEM
+        del hold
+        torch.cuda.empty_cache()
+        got = native.eos_eval(p[:points], t[:points], y1[:points], y2[:points], prop=True)
+        assert np.array_equal(got[0], want[0][:points]) and np.array_equal(got[1], want[1][:points])
+    hold = _fill(40 * MB)
+    with pytest.raises(Cfd3dError):
+        native.Engine(c, precision=abi.MIXED)
+    del hold
+    torch.cuda.empty_cache()
+    e = native.Engine(c, precision=abi.MIXED)
+    e.initialize(c["pv0"])
+    assert np.all(np.isfinite(e.iterate()[1]))
+    e.close()
