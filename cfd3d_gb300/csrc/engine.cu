@@ -32,6 +32,7 @@
 #include <type_traits>
 #include <unistd.h>
 #include <vector>
+#include "ctx_slots.h"
 #include "engine.cuh"
 #include "mixed.cuh"
 
@@ -2537,49 +2538,49 @@ struct EosScratch { double x[1 + EOS_PER_POINT * CFD3D_EOS_NOALLOC_MAX]; };
 // module's globals, and a context that ends (cudaDeviceReset, a primary context released
 // and made again) takes the copy with it, so the cache is keyed on the context's unique id
 // (cuCtxGetId; ids are never reused within a process), not on the device index.
-struct ScratchSlot { unsigned long long ctx; EosScratch* ptr; };
-std::mutex g_eos_scratch_mu;
-std::vector<ScratchSlot> g_eos_scratch_slots;
+using EosSlots = CtxSlots<double*>;
+EosSlots g_eos_slots;
 
 // the current context's id, through the runtime's driver entry points (no link against
 // the driver library); 0 when no context is current
 using FnCtxGetCurrent = CUresult (*)(CUcontext*);
 using FnCtxGetId = CUresult (*)(CUcontext, unsigned long long*);
-bool current_ctx_id(unsigned long long& id) {
-  static FnCtxGetCurrent get_cur = nullptr;
-  static FnCtxGetId get_id = nullptr;
-  if (!get_cur || !get_id) {
-    void* f1 = nullptr;
-    void* f2 = nullptr;
+struct CtxFns {
+  FnCtxGetCurrent cur = nullptr;
+  FnCtxGetId id = nullptr;
+  CtxFns() {
+    void *f1 = nullptr, *f2 = nullptr;
     if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f1, 12000, cudaEnableDefault, nullptr) != cudaSuccess ||
-        cudaGetDriverEntryPointByVersion("cuCtxGetId", &f2, 12000, cudaEnableDefault, nullptr) != cudaSuccess ||
-        !f1 || !f2)
-      return false;
-    get_cur = reinterpret_cast<FnCtxGetCurrent>(f1);
-    get_id = reinterpret_cast<FnCtxGetId>(f2);
+        cudaGetDriverEntryPointByVersion("cuCtxGetId", &f2, 12000, cudaEnableDefault, nullptr) != cudaSuccess)
+      return;
+    cur = reinterpret_cast<FnCtxGetCurrent>(f1);
+    id = reinterpret_cast<FnCtxGetId>(f2);
   }
+};
+bool current_ctx_id(unsigned long long& id) {
+  static const CtxFns f;   // (looked up once, by whichever thread comes first)
+  if (!f.cur || !f.id) return false;
   CUcontext ctx = nullptr;
-  if (get_cur(&ctx) != CUDA_SUCCESS) return false;
+  if (f.cur(&ctx) != CUDA_SUCCESS) return false;
   id = 0;
-  return !ctx || get_id(ctx, &id) == CUDA_SUCCESS;
+  return !ctx || f.id(ctx, &id) == CUDA_SUCCESS;
 }
 }  // namespace
 static __device__ __align__(256) EosScratch g_eos_scratch;
 
 namespace {
-// the buffer's address in the current context (set up on the first call there), or null;
-// g_eos_scratch_mu is held from here to the end of the call that uses the buffer
-double* eos_scratch() {
+// the buffer in the current context (looked up on the first call there), or null; the slot's
+// lock is held from here to the end of the call that uses the buffer
+EosSlots::Slot* eos_scratch() {
   unsigned long long ctx = 0;
   if (!current_ctx_id(ctx)) return nullptr;
-  for (const ScratchSlot& sl : g_eos_scratch_slots)
-    if (ctx && sl.ctx == ctx) return sl.ptr->x;
+  if (ctx)
+    if (EosSlots::Slot* s = g_eos_slots.find(ctx)) return s;
   // (with no context current yet, the lookup makes the device's primary context current)
   void* ptr = nullptr;
   if (cudaGetSymbolAddress(&ptr, g_eos_scratch) != cudaSuccess || !ptr) return nullptr;
   if (!ctx && (!current_ctx_id(ctx) || !ctx)) return nullptr;
-  g_eos_scratch_slots.push_back({ctx, static_cast<EosScratch*>(ptr)});
-  return static_cast<EosScratch*>(ptr)->x;
+  return g_eos_slots.put(ctx, static_cast<EosScratch*>(ptr)->x);
 }
 
 // n points through the device buffer x (1 + EOS_PER_POINT n doubles).  Few points are a
@@ -2638,8 +2639,10 @@ int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, c
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return CFD3D_ERR_NODEVICE;
   if (n <= CFD3D_EOS_NOALLOC_MAX) {
-    std::lock_guard<std::mutex> lock(g_eos_scratch_mu);
-    if (double* x = eos_scratch()) return eos_run<TERMS>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x);
+    if (EosSlots::Slot* sl = eos_scratch()) {
+      std::lock_guard<std::mutex> lock(sl->mu);
+      return eos_run<TERMS>(fluid, with_prop, n, p, t, y1, y2, dv, tv, sl->value);
+    }
     cudaGetLastError();
   }
   double* x = nullptr;
@@ -2669,9 +2672,13 @@ int cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const 
     return CFD3D_ERR_ARG;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return CFD3D_ERR_NODEVICE;
-  std::lock_guard<std::mutex> lock(g_eos_scratch_mu);
-  double* x = eos_scratch();
-  return x ? eos_run<false>(fluid, with_prop, n, p, t, y1, y2, dv, tv, x) : CFD3D_ERR_CUDA;
+  EosSlots::Slot* sl = eos_scratch();
+  if (!sl) {
+    cudaGetLastError();
+    return CFD3D_ERR_CUDA;
+  }
+  std::lock_guard<std::mutex> lock(sl->mu);
+  return eos_run<false>(fluid, with_prop, n, p, t, y1, y2, dv, tv, sl->value);
 }
 
 static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {

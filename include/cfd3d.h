@@ -306,7 +306,8 @@ int  cfd3d_eos_eval(int fluid, int ngas, int with_prop, int64_t n, const double 
  * one after cudaDeviceReset) looks up the buffer's device address, so make it before any
  * stream capture there.  Under lazy module loading (the CUDA default) that first call is
  * also when the buffer is reserved: make it while device memory is still free, or load
- * modules eagerly (CUDA_MODULE_LOADING=EAGER).  Calls of several host threads take turns. */
+ * modules eagerly (CUDA_MODULE_LOADING=EAGER).  Calls of several host threads take turns in
+ * one context, and do not wait for one another in different ones. */
 #define CFD3D_EOS_NOALLOC_MAX 4096
 int  cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const double *p,
                             const double *t, const double *y1, const double *y2, double *dv,
