@@ -2773,13 +2773,7 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
          cudaMalloc(&E.d.mxn, MXN * sizeof(int)) == cudaSuccess;
   }
   else {
-    // the face reconstruction's scratch: all three directions at once up to 128 MB of it.  A
-    // launch per direction leaves three partial last waves (the face stage of 128x64x64 cells
-    // 7.5 ms against 7.4), which is less than a larger allocation costs a short run.
-    E.d.nfs = (c.nmuscl == 2) ? 5 : (c.nmuscl > 0 ? 1 : 0);
-    E.d.fslots = (3.0 * E.d.nfs * c.npv * 8.0 * (double)n <= 1.28e8) ? 3 : 1;
-    ok = ok && alloc(E.d.fi, 3 * c.npv) && alloc(E.d.fv, (c.iturb == -3) ? 1 : 3 * c.npv) &&
-         alloc(E.d.fsc, (long long)E.d.fslots * E.d.nfs * c.npv);
+    ok = ok && alloc(E.d.fi, 3 * c.npv) && alloc(E.d.fv, (c.iturb == -3) ? 1 : 3 * c.npv);
   }
   if (c.csf) ok = ok && alloc(E.d.vf, 1) && alloc(E.d.vfg, 3) && alloc(E.d.csf, 3);
   if (!ok) { E.err = "device allocation failed"; return CFD3D_ERR_NOMEM; }
@@ -2916,6 +2910,26 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
     return CFD3D_ERR_NOMEM;
   }
   {
+    // The face reconstruction's scratch: all three directions at once up to 128 MB of it.  (A
+    // launch per direction leaves three partial last waves -- the face stage of 128x64x64 cells
+    // 7.5 ms against 7.4 -- which is less than a larger allocation costs a short run.)  Beyond, one
+    // direction's planes lie in the sweep records, which k_rhs writes when the face stage is
+    // over: 360 B a cell under MLP with nine unknowns, in 488.  Only blocks of so few interior
+    // cells that their padding outweighs the records take an allocation of their own.
+    E.d.nfs = (c.nmuscl == 2) ? 5 : (c.nmuscl > 0 ? 1 : 0);
+    const long long planes = (long long)E.d.nfs * c.npv;
+    E.d.fslots = (3.0 * planes * 8.0 * (double)n <= 1.28e8) ? 3 : 1;
+    if (E.d.fslots == 3 && !alloc(E.d.fsc, 3 * planes)) {
+      cudaGetLastError();
+      E.d.fsc = nullptr;
+      E.d.fslots = 1;
+    }
+    if (E.d.fslots == 1) {
+      if (planes * n <= NREC * E.nint) E.d.fsc = E.d.rec;
+      else if (!alloc(E.d.fsc, planes)) { E.err = "device allocation failed (face scratch)"; return CFD3D_ERR_NOMEM; }
+    }
+  }
+  {
     const char* mode = std::getenv("CFD3D_SWEEP");
     E.sweep_planes = (mode && std::strcmp(mode, "planes") == 0) ? 1 : 0;
     int dev = 0, nsm = 0, per = 0;
@@ -2940,8 +2954,9 @@ void cfd3d_destroy(cfd3d_handle* h) {
   Engine& E = h->E;
   if (E.graph) cudaGraphExecDestroy(E.graph);
   double* bufs[] = {E.d.pv, E.d.dv, E.d.tv, E.d.gm, E.d.res, E.d.icav, E.d.itt, E.d.ocut, E.d.dt, E.d.rcav,
-                    E.d.qq, E.d.dqs, E.d.dcv, E.d.fi, E.d.fv, E.d.fsc, E.d.partial, h->staging, E.d.clo,
+                    E.d.qq, E.d.dqs, E.d.dcv, E.d.fi, E.d.fv, E.d.partial, h->staging, E.d.clo,
                     E.d.vf, E.d.vfg, E.d.csf};
+  if (E.d.fsc != E.d.rec) cudaFree(E.d.fsc);
   for (double* p : bufs) cudaFree(p);
   float* fbufs[] = {E.d.pvf, E.d.fi32, E.d.fv32, E.d.frec, E.d.gmf, E.d.gmlo, E.d.lqf};
   for (float* p : fbufs) cudaFree(p);

@@ -141,7 +141,8 @@ __host__ __device__ __forceinline__ long long tq_at(long long s, int v) {
 struct DevPtr {
   double *pv, *dv, *tv, *gm, *res, *icav, *itt, *ocut, *dt, *rcav, *qq, *dqs, *dcv, *qold, *fi, *fv;
   // FP64 form: scratch planes of the face reconstruction (flux.cu), nfs per variable and
-  // direction slot; fslots directions at a time (3: all in one launch)
+  // direction slot; fslots directions at a time (3: all in one launch; 1: in rec's memory where
+  // that holds them)
   double* fsc;
   int nfs, fslots;
   const BlockGeom* blk;
