@@ -285,7 +285,7 @@ int adjoint_buffers(Engine& E) {
   // the face kernels' states and scratch planes: the FP64 form's own, else one direction's
   const size_t nfs = (E.par.nmuscl == 2) ? 5 : 1;
   if (E.par.mixed && !E.adj_fi && E.par.nmuscl > 0 &&
-      !group({{(void**)&E.adj_fi, n * npv * 3 * 8}, {(void**)&E.adj_fsc, n * npv * nfs * 8}}))
+      !group({{(void**)&E.adj_fi, n * npv * 8}, {(void**)&E.adj_fsc, n * npv * nfs * 8}}))
     return CFD3D_ERR_NOMEM;
   cudaMemsetAsync(E.adj_lam, 0, n * npv * 8, E.st);
   cudaMemsetAsync(E.adj_gpv, 0, n * npv * 8, E.st);
@@ -305,6 +305,7 @@ static DevPtr adj_dev(const Engine& E) {
   DevPtr d = E.d;
   if (E.par.mixed) {
     d.fi = E.adj_fi;
+    d.fi1 = 1;
     d.fsc = E.adj_fsc;
     d.nfs = (E.par.nmuscl == 2) ? 5 : (E.par.nmuscl > 0 ? 1 : 0);
     d.fslots = 1;

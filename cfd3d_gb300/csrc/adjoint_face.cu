@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(128) k_adj_recon(DevPtr d, Par c, AdjPtr a, in
   DirCell f;
   if (!dir_cell<0>(d, dir, blockIdx.x * (long long)blockDim.x + threadIdx.x, f)) return;
   const long long n = d.ncell, g = f.g, sn = f.sn, s1 = f.s1, s2 = f.s2;
-  const double gl = d.fi[((long long)dir * npv + v) * n + g], gr = fs_plane(d, slot, npv, v, FS_R)[g];
+  const double gl = fi_planes(d, dir, npv)[v * n + g], gr = fs_plane(d, slot, npv, v, FS_R)[g];
   if (gl == 0.0 && gr == 0.0) return;
   const double* P = d.pv + v * n + g;
   double* G = a.gpv + v * n + g;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(64) k_adj_flux(DevPtr d, Par c, AdjPtr a, int 
     const long long n = d.ncell, g = f.g, gr = f.g + f.sn;
     double lam[NPVM];
     const bool any = face_cotangent(a, npv, n, g, gr, lam);
-    double* fi = d.fi + (long long)dir * npv * n + g;
+    double* fi = fi_planes(d, dir, npv) + g;
     FaceGrad o{};
     if (any) {
       double nx[3], c9[NPVM], c10[NPVM];

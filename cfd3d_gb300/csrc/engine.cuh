@@ -145,6 +145,7 @@ struct DevPtr {
   // that holds them)
   double* fsc;
   int nfs, fslots;
+  int fi1;   // 1: fi holds one direction (the mixed form's adjoint), else three
   const BlockGeom* blk;
   int nblk;
   long long ncell;

@@ -38,6 +38,11 @@ __device__ __forceinline__ bool dir_cell(const DevPtr& d, int dir, long long t, 
 
 __device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 
+// the left face states, then the fluxes, of a direction (npv planes; fi1: one direction's at a time)
+__device__ __forceinline__ double* fi_planes(const DevPtr& d, int dir, int npv) {
+  return d.fi + (long long)(d.fi1 ? 0 : dir) * npv * d.ncell;
+}
+
 // scratch planes of one direction slot and variable
 enum { FS_MN = 0, FS_MX, FS_DEN, FS_IDQ, FS_R, NFS };
 __device__ __forceinline__ double* fs_plane(const DevPtr& d, int slot, int npv, int v, int q) {

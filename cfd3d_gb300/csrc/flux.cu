@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) k_recon64(DevPtr d, Par c, int dir0) {
   if (!dir_cell<0>(d, dir, blockIdx.x * (long long)blockDim.x + threadIdx.x, f)) return;
   const long long n = d.ncell, g = f.g, sn = f.sn;
   const double* P = d.pv + v * n + g;
-  double* outL = d.fi + ((long long)dir * npv + v) * n + g;
+  double* outL = fi_planes(d, dir, npv) + v * n + g;
   double* outR = fs_plane(d, slot, npv, v, FS_R) + g;
   const double cm2 = P[-2 * sn], cm1 = P[-sn], c0 = P[0], c1 = P[sn], c2 = P[2 * sn], c3 = P[3 * sn];
   const double eps = 1.0e-30;
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(3 * F64_FACES) k_flux64(DevPtr d, Par c, int d
   const bool live = dir_cell<0>(d, dir, blockIdx.x * (long long)F64_FACES + q, f);
   const long long n = d.ncell, g = f.g, gr = f.g + f.sn;
   const bool snd = c.nscheme == 2 || c.nscheme == 3;   // Roe-M and AUSMPW+ read the face sound speeds
-  double* fi = d.fi + (long long)dir * npv * n;
+  double* fi = fi_planes(d, dir, npv);
   if (live && role < 2 && c.nmuscl > 0) {
     const long long cell = role ? gr : g;
     double x[NPVM];

@@ -70,3 +70,23 @@ def test_a_failed_create_leaves_the_other_calls_alone():
     e.initialize(c["pv0"])
     assert np.all(np.isfinite(e.iterate()[1]))
     e.close()
+
+
+def test_memory_of_the_mixed_adjoint():
+    import torch
+    c = base._state(1)
+    lam = np.random.default_rng(9).normal(size=abi.interior_shape(c["blocks"][0], 9))
+    e = native.Engine(c, precision=abi.MIXED)
+    e.initialize(c["pv0"])
+    e.iterate()
+    small = native.Engine(base._state(4), precision=abi.MIXED)   # the kernels' modules and stacks
+    small.initialize(None)
+    small.residual_vjp([np.ones((16, 16, 16, 9))])
+    free = torch.cuda.mem_get_info()[0]
+    e.residual_vjp([lam])
+    held = free - torch.cuda.mem_get_info()[0]
+    e.close()
+    small.close()
+    # planes of 70^3 cells: cotangent and gradient 9 each, dv and tv 10, one direction's face states
+    # 9, five reconstruction planes a variable; seven allocations round up to 2 MB each
+    assert held <= 8 * 70 ** 3 * (9 + 9 + 10 + 9 + 45) + 7 * 2 * MB, held / MB
