@@ -2731,6 +2731,11 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
     E.blk.push_back(G);
   }
   if (off >= (1ll << 31)) { E.err = "case too large for 32-bit cell indices"; return CFD3D_ERR_ARG; }
+  // (the mixed form lists up to two states per face of a direction)
+  if (E.par.mixed && 2 * std::max({foff[0], foff[1], foff[2]}) > 0x7fffffffll) {
+    E.err = "case too large for 32-bit face state lists";
+    return CFD3D_ERR_ARG;
+  }
   E.ncell = off; E.nint = ioff;
   for (int q = 0; q < 3; ++q) { E.nface[q] = foff[q]; E.ncol[q] = coff[q]; E.nplane[q] = poff[q]; }
   CFD_CUDA(cudaStreamCreateWithFlags(&E.st, cudaStreamNonBlocking));
@@ -2766,9 +2771,9 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
     ok = ok && allocf(E.d.pvf, c.npv) && allocf(E.d.fi32, 3 * c.npv) && allocf(E.d.fv32, (c.iturb == -3) ? 1 : 3 * c.npv) &&
          allocf(E.d.frec, E.face_slots * 2 * FREC_SIDE) && allocf(E.d.lqf, NLQ);
   if (c.mixed) {
-    // lists of face states (two per face of a direction) and of cells
-    const long long most = std::max({2 * E.nface[0], 2 * E.nface[1], 2 * E.nface[2], E.nint});
-    E.d.mxcap = (int)std::min<long long>(most, 0x7fffffffll);
+    // lists of face states (two per face of a direction) and of cells: each is listed once at
+    // most, so that they all fit
+    E.d.mxcap = (int)std::max({2 * E.nface[0], 2 * E.nface[1], 2 * E.nface[2], E.nint});
     ok = ok && cudaMalloc(&E.d.mxl, (size_t)E.d.mxcap * MX_KINDS * E.face_slots * sizeof(int)) == cudaSuccess &&
          cudaMalloc(&E.d.mxn, MXN * sizeof(int)) == cudaSuccess;
   }

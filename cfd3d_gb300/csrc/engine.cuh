@@ -211,7 +211,8 @@ enum { MX_LIQ = 0, MX_META, MX_STABLE, MX_KINDS };
 constexpr int MXN_FACE = 3 * MX_KINDS, MXN = MXN_FACE + MX_KINDS;
 
 // item appended to the list of its kind: one atomic per kind of the lanes that call together.
-// (The order of a list is arbitrary; every entry's result goes to its own place.)
+// (The order of a list is arbitrary; every entry's result goes to its own place.  mxcap counts
+// every state there is, each appended once: the comparison with it never drops one.)
 __device__ __forceinline__ void list_add(const DevPtr& d, int* cnt, int kind, int item) {
   const unsigned same = __match_any_sync(__activemask(), kind);
   const int lane = threadIdx.x & 31, lead = __ffs(same) - 1;

@@ -249,7 +249,7 @@ __device__ __forceinline__ void face_eos_later(const DevPtr& d, const Par& c, in
     return;
   }
   const int kind = (x[5] == 0.0f) ? MX_LIQ : (above_psat(p, t) ? MX_META : MX_STABLE);
-  list_add(d, cnt, kind, 2 * g + side);
+  list_add(d, cnt, kind, (int)(2u * (unsigned)g + (unsigned)side));
 }
 
 // rho - rhoref and h - href of the listed face states by the df64 IF97 sums, one launch per
