@@ -2681,7 +2681,9 @@ int cfd3d_eos_eval_noalloc(int fluid, int ngas, int with_prop, int64_t n, const 
   return eos_run<false>(fluid, with_prop, n, p, t, y1, y2, dv, tv, sl->value);
 }
 
-static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {
+// lean: with the least scratch, the face directions in turn
+static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out,
+                         bool lean) {
   if (!out) return CFD3D_ERR_ARG;
   *out = nullptr;
   cfd3d_handle* h = new (std::nothrow) cfd3d_handle();
@@ -2766,7 +2768,7 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
   // beside: 0.192 and 0.074 ms at 16x12x10 cells, 0.80 and 0.65 at 128x64x64, 4.92 and 4.67
   // on 24 blocks of 3.0 M cells, 15.4 and 15.1 at 14.2 M, where another 3 GB would be
   // allocated and cleared for it.
-  if (c.mixed) E.face_slots = (3.0 * 2 * FREC_SIDE * 4.0 * (double)n <= 2e9) ? 3 : 1;
+  if (c.mixed) E.face_slots = (!lean && 3.0 * 2 * FREC_SIDE * 4.0 * (double)n <= 2e9) ? 3 : 1;
   if (c.mixed)
     ok = ok && allocf(E.d.pvf, c.npv) && allocf(E.d.fi32, 3 * c.npv) && allocf(E.d.fv32, (c.iturb == -3) ? 1 : 3 * c.npv) &&
          allocf(E.d.frec, E.face_slots * 2 * FREC_SIDE) && allocf(E.d.lqf, NLQ);
@@ -2923,15 +2925,12 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
     // cells that their padding outweighs the records take an allocation of their own.
     E.d.nfs = (c.nmuscl == 2) ? 5 : (c.nmuscl > 0 ? 1 : 0);
     const long long planes = (long long)E.d.nfs * c.npv;
-    E.d.fslots = (3.0 * planes * 8.0 * (double)n <= 1.28e8) ? 3 : 1;
-    if (E.d.fslots == 3 && !alloc(E.d.fsc, 3 * planes)) {
-      cudaGetLastError();
-      E.d.fsc = nullptr;
-      E.d.fslots = 1;
-    }
-    if (E.d.fslots == 1) {
-      if (planes * n <= NREC * E.nint) E.d.fsc = E.d.rec;
-      else if (!alloc(E.d.fsc, planes)) { E.err = "device allocation failed (face scratch)"; return CFD3D_ERR_NOMEM; }
+    E.d.fslots = (!lean && 3.0 * planes * 8.0 * (double)n <= 1.28e8) ? 3 : 1;
+    if (E.d.fslots == 1 && planes * n <= NREC * E.nint) {
+      E.d.fsc = E.d.rec;
+    } else if (!alloc(E.d.fsc, E.d.fslots * planes)) {
+      E.err = "device allocation failed (face scratch)";
+      return CFD3D_ERR_NOMEM;
     }
   }
   {
@@ -2948,9 +2947,15 @@ static int create_handle(const cfd3d_config* cfg, int nblocks, const cfd3d_block
 }
 
 int cfd3d_create(const cfd3d_config* cfg, int nblocks, const cfd3d_block_desc* blocks, cfd3d_handle** out) {
-  const int rc = create_handle(cfg, nblocks, blocks, out);
+  int rc = create_handle(cfg, nblocks, blocks, out, false);
   // a failed allocation's error is reported by rc: it does not stay for the next call
   if (rc == CFD3D_ERR_NOMEM || rc == CFD3D_ERR_DESCRIPTOR) cudaGetLastError();
+  // short of memory, a case whose face directions would run beside one another takes them in turn
+  if (rc == CFD3D_ERR_NOMEM && out && *out) {
+    cfd3d_destroy(*out);
+    rc = create_handle(cfg, nblocks, blocks, out, true);
+    if (rc == CFD3D_ERR_NOMEM) cudaGetLastError();
+  }
   return rc;
 }
 

@@ -90,3 +90,34 @@ def test_memory_of_the_mixed_adjoint():
     # planes of 70^3 cells: cotangent and gradient 9 each, dv and tv 10, one direction's face states
     # 9, five reconstruction planes a variable; seven allocations round up to 2 MB each
     assert held <= 8 * 70 ** 3 * (9 + 9 + 10 + 9 + 45) + 7 * 2 * MB, held / MB
+
+
+@pytest.mark.parametrize("precision,scale", [(abi.MIXED, 1), (abi.FP64, 2)])
+def test_create_with_little_memory_takes_the_directions_in_turn(precision, scale):
+    import torch
+    c = base._state(scale)
+
+    def run():
+        e = native.Engine(c, precision=precision)
+        e.initialize(c["pv0"])
+        for it in range(2):
+            e.iterate(1, it + 1, 0.0)
+        pv = e.download(0)["pv"]
+        e.close()
+        return pv
+
+    want = run()
+    free = torch.cuda.mem_get_info()[0]
+    e = native.Engine(c, precision=precision)
+    full = free - torch.cuda.mem_get_info()[0]
+    e.close()
+    # the other directions' scratch is 78 MB (64^3 cells, mixed) and 39 MB (32^3, FP64)
+    hold = _fill(full - 12 * MB)
+    e = native.Engine(c, precision=precision)
+    del hold
+    torch.cuda.empty_cache()
+    e.initialize(c["pv0"])
+    for it in range(2):
+        e.iterate(1, it + 1, 0.0)
+    assert np.array_equal(e.download(0)["pv"], want)
+    e.close()
