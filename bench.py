@@ -47,12 +47,13 @@ METRIC = "Mcell-iter/s per GB300, mixed vs FP64 form at stated error; % HBM peak
 UNIT = "Mcell-iter/s"
 
 
-# DRAM bytes per cell of one k_rhs launch, dram__bytes_read.sum + dram__bytes_write.sum
-# of a one-pass ncu capture of the mixed form on the large case itself (14155776 cells, the
-# launch list of one pseudo-iteration), divided by the cells
-RHS_TRAFFIC_PER_CELL = (15.147836e9 + 8.649704e9) / 14155776
-# the same for the whole pseudo-iteration: dram read + write summed over its 35 launches
-ITER_TRAFFIC_PER_CELL = (66.336343e9 + 29.794348e9) / 14155776
+# DRAM bytes per cell of one k_rhs launch, dram__bytes_read.sum + dram__bytes_write.sum of an
+# ncu capture of that kernel alone in the mixed form, on two of the large case's sixteen blocks
+# (1769472 cells: the same block shape, a few GB on the device), divided by the cells
+RHS_TRAFFIC_PER_CELL = (1.877308e9 + 1.037774e9) / 1769472
+# the same for the whole pseudo-iteration: summed over its kernels, each captured alone there,
+# the boundary program's scaled by its ghost counts in the large case
+ITER_TRAFFIC_PER_CELL = 4645.0 + 1790.9
 
 
 def algorithmic_bytes(cfg):

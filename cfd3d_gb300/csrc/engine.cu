@@ -513,7 +513,7 @@ __device__ __forceinline__ void ghost_eos(const DevPtr& d, const Par& c, double 
 // passes through in two batches (at 6 or 12 CTAs per SM, or in batches of six, it was
 // slower).  The boundary stage in one kernel and so: 56 and 47 us at 16x12x10 cells, 85 and
 // 72 us at 128x64x64, 0.354 and 0.295 ms on 24 blocks of 3.0 M cells (halo runs of three
-// cells: partial sectors), 2.42 and 2.25 ms on 8 blocks of 14.2 M.
+// cells: partial sectors), 2.42 and 2.25 ms on 16 blocks of 14.2 M.
 __global__ void __launch_bounds__(128, 8) k_ghost(DevPtr d, Par c, const GhostOp* __restrict__ ops, int nops) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nops) return;
@@ -1552,7 +1552,7 @@ __global__ void __launch_bounds__(4 * SW_CH) k_sweep_df(DevPtr d, Par c, long lo
 // steps after the one before it in i, j or k, where with done flags it started 18 later
 // plus a fence and a round trip to L2.  Both sweeps of an iteration: 1.03 -> 0.49 ms at
 // 128x64x64 cells, 0.22 -> 0.12 ms at 16x12x10, 1.15 -> 0.94 ms on 24 uneven blocks of 3.0 M
-// cells, 4.0 -> 3.6 ms on 8 blocks of 14.2 M.  (Reading a step's records ahead of its wait
+// cells, 4.0 -> 3.6 ms on 16 blocks of 14.2 M.  (Reading a step's records ahead of its wait
 // was slower, 3.77 ms there.)  (Three warps with a product each, the solution
 // in all of them, took 1.7 ms where one warp took 1.03.)
 // The needed tiles always hold earlier tickets, so the waits end; they are bounded as in the
@@ -2630,7 +2630,7 @@ int eos_run(int fluid, int with_prop, int64_t n, const double* p, const double* 
 // As many points as the static buffer holds go through it; more through one allocation.
 // (200 points took 271 us with an allocation per array and 115 us through the buffer with a
 // copy per array; packed, and on two warps, 64 us, some 33 of them the kernel's.  4000 points
-// 316 -> 114 us, 300000 points 2.88 -> 2.49 ms, of which the copy of the results to pageable
+// 316 -> 114 us, 300000 points 2.88 -> 2.07 ms, of which the copy of the results to pageable
 // memory is most.)
 template <bool TERMS>
 int eos_points(int fluid, int ngas, int with_prop, int64_t n, const double* p, const double* t, const double* y1,

@@ -10,7 +10,8 @@
 // 14.2 M-cell one), and a warp with some vapour ran the liquid's sums twice.  Now
 //   k_eos_liq         the liquid's df64 sums and the gas, every cell; cells with vapour are
 //                     listed by the vapour sums they need
-//   k_eos_vap<META>   the vapour's df64 sums of the listed cells, full warps
+//   k_eos_vap         the vapour's df64 sums of the listed cells, full warps, a grid row per
+//                     list
 //   k_eos_mix         FP32 derivatives and transport properties, the mixture
 // with the five phase values between them in the face records' planes (idle then).
 #include <algorithm>
