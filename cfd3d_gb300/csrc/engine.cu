@@ -3865,7 +3865,10 @@ int cfd3d_set_launch_shapes(cfd3d_handle* h, const int* shapes) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (c.mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_tile_kernel(true, c.npv), TILE_T, TILE_SMEM);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sweep_df<true>, 4 * SW_CH, 0);
-  if (shapes[2] < 1 || shapes[2] > std::max(per, 1)) { E.err = "sweep CTAs per SM outside 1 .. the occupancy limit"; return CFD3D_ERR_ARG; }
+  // (the FP64 form takes the shapes of tuning runs from when its sweep CTAs were one warp and
+  // eight fitted: a CTA that is not resident takes its ticket later, and none waits for it)
+  const int most = std::max(per, c.mixed ? 1 : 8);
+  if (shapes[2] < 1 || shapes[2] > most) { E.err = "sweep CTAs per SM outside 1 .. " + std::to_string(most); return CFD3D_ERR_ARG; }
   const int nb = (int)E.blk.size();
   if (shapes[3] < 1 || shapes[3] > std::min(nb, Engine::MAX_PIPE) || (!c.mixed && shapes[3] != 1)) {
     E.err = "pipeline groups outside 1 .. min(blocks, 16) (1 in the FP64 form)";

@@ -267,9 +267,10 @@ int  cfd3d_convert_selftest(long long n, unsigned long long seed, long long *mis
  * The autotuner chooses all four; results do not depend on them. */
 int  cfd3d_launch_shapes(const cfd3d_handle *h, int *shapes);
 /* Sets the four launch shapes of cfd3d_launch_shapes (for instance those a tuning run
- * found): threads per CTA 64, 128 or 256; sweep CTAs per SM from 1 to the occupancy limit;
- * pipeline groups from 1 to min(blocks, 16), 1 in the FP64 form.  CFD3D_ERR_ARG otherwise,
- * with nothing changed.  The iteration graph is re-captured at the next iteration. */
+ * found): threads per CTA 64, 128 or 256; sweep CTAs per SM from 1 to the occupancy limit, or
+ * to 8 in the FP64 form (those that are not resident start later); pipeline groups from 1 to
+ * min(blocks, 16), 1 in the FP64 form.  CFD3D_ERR_ARG otherwise, with nothing changed.  The
+ * iteration graph is re-captured at the next iteration. */
 int  cfd3d_set_launch_shapes(cfd3d_handle *h, const int *shapes);
 
 /* Test hook of the dataflow sweeps' bounded waits (no counterpart in the reference): one
